@@ -3,11 +3,11 @@
 // planar layout [candidates][rows][cols] and for batches of volumes in the chunked layout of
 // ssg_cells.cuh.
 //
-// Both layouts run the same kernels, templated on the cell width W (1 = planar, 8 = chunked):
 //   - downsampling: one thread per coarse pixel; its 3x3 range weights are computed once from the
 //     uint8 guides and shared by all candidates;
-//   - upsampling: one thread per fine pixel, with the coarse neighbourhood of a block staged in
-//     shared memory per chunk of candidates;
+//   - upsampling of chunked volumes: one thread per two fine pixels, with the coarse neighbourhood of
+//     a block staged in shared memory per chunk of candidates;
+//   - planar volumes of several candidates: ssg_isb_planar.cuh;
 //   - the last upsampling step can be fused with the selection, so that the filtered level-0
 //     volume is never written.
 // Guides, range weights and cost sums use the reference's arithmetic in its order
@@ -21,6 +21,7 @@
 
 #include "ssg_cells.cuh"
 #include "ssg_isb_common.cuh"
+#include "ssg_isb_planar.cuh"
 #include "ssg_tma.cuh"
 #include "ssg_uneven.cuh"
 
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kBatchBlock) isb_down_kernel(const uint8_t* __
 // neighbourhood, edge-clamped as the taps are, are staged per chunk of candidates in shared
 // memory with cp.async, double-buffered: each coarse cell is read from memory once per block,
 // and the next chunk streams in while this one is filtered.  Candidates are processed in parts
-// of 4 (W = 8) or 1 (W = 1) to bound the registers that hold the taps.
+// of 4 to bound the registers that hold the taps.
 // ---------------------------------------------------------------------------------------------
 constexpr int kUpTileX = kBatchBlock / 2;
 constexpr int kUpTileCols = kUpTileX + 2;
@@ -230,21 +231,15 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
 }
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
-{
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem));
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;\n" ::); }
 
-// A chunk's tile: [part][row 0..2][col 0..kUpTileCols-1][E floats], parts of E = 4 candidates
-// (W = 8, two parts) or of one candidate (W = 1).  A part starts on a 128-byte boundary (the
-// alignment of a TMA destination).
+// A chunk's tile: [part][row 0..2][col 0..kUpTileCols-1][E floats], two parts of E = 4 candidates.
+// A part starts on a 128-byte boundary (the alignment of a TMA destination).
 template <int W>
 struct UpTile {
-    static constexpr int parts = W == 8 ? 2 : 1;
-    static constexpr int E = W == 8 ? 4 : 1;
+    static constexpr int parts = 2;
+    static constexpr int E = 4;
     static constexpr int part_floats = (3 * kUpTileCols * E + 31) / 32 * 32;
     static constexpr int floats = parts * part_floats;
     static constexpr uint32_t part_bytes = 3 * kUpTileCols * E * sizeof(float);  // one TMA box
@@ -261,10 +256,7 @@ __device__ __forceinline__ void load_tile_async(float* __restrict__ buf, const f
         const int gx = min(max(x0 - 1 + col, 0), cols_in - 1), gy = min(max(y - 1 + row, 0), rows_in - 1);
         const float* src = chunk + ((int64_t)gy * cols_in + gx) * W + part * 4;
         float* dst = buf + part * UpTile<W>::part_floats + rc * UpTile<W>::E;
-        if constexpr (W == 8)
-            cp_async16(dst, src);
-        else
-            cp_async4(dst, src);
+        cp_async16(dst, src);
     }
 }
 
@@ -356,30 +348,6 @@ struct RawCell<8, float> {
         v[3] = p == 0 ? c[3] : c[7];
     }
 };
-template <>
-struct RawCell<1, float> {
-    float a;
-    __device__ __forceinline__ void load(const float* cell) { a = __ldg(cell); }
-    __device__ __forceinline__ void part(int, float v[1]) const { v[0] = a; }
-};
-
-template <int E>
-__device__ __forceinline__ void store_part(float* cell, int p, const float v[E])
-{
-    if constexpr (E == 4)
-        reinterpret_cast<float4*>(cell + 4 * p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    else
-        cell[0] = v[0];
-}
-
-template <int F>
-__device__ __forceinline__ constexpr bool uses_tap(int t)
-{
-    for (int i = 0; i < UpTaps<F>::n; ++i)
-        if (UpTaps<F>::tap(i) == t) return true;
-    return false;
-}
-
 template <int F, typename GL>
 __device__ __forceinline__ float fine_weights_padded(const typename GL::Pix (&gd)[9], const typename GL::Pix& up,
                                                      float weight_up, float weight_down, const LutRange& range,
@@ -487,12 +455,10 @@ __device__ __forceinline__ void up_part(const float (&tap)[9][UpTile<W>::E], con
             for (int e = 0; e < E; ++e)
                 if (k0 + e < ncand) s.push(k0 + e, acc[e]);
         }
-    } else if constexpr (W == 8) {
+    } else {
         // kept for the store of the whole cell after both parts
 #pragma unroll
         for (int e = 0; e < E; ++e) kept[part * E + e] = acc[e];
-    } else {
-        store_part<E>(reinterpret_cast<float*>(fine_chunk + (int64_t)px.index * W), part, acc);
     }
 }
 
@@ -514,12 +480,8 @@ __device__ __forceinline__ void up_chunk(const float* __restrict__ buf, int lx, 
             if (uses_tap<FA>(t) || uses_tap<FB>(t)) {
                 const int cell = (t / 3) * kUpTileCols + lx + t % 3;
                 const float* pb = buf + part * UpTile<W>::part_floats;
-                if constexpr (E == 4) {
-                    const float4 q = reinterpret_cast<const float4*>(pb)[cell];
-                    tap[t][0] = q.x; tap[t][1] = q.y; tap[t][2] = q.z; tap[t][3] = q.w;
-                } else {
-                    tap[t][0] = pb[cell];
-                }
+                const float4 q = reinterpret_cast<const float4*>(pb)[cell];
+                tap[t][0] = q.x; tap[t][1] = q.y; tap[t][2] = q.z; tap[t][3] = q.w;
             } else {
 #pragma unroll
                 for (int e = 0; e < E; ++e) tap[t][e] = 0.0f;
@@ -531,7 +493,7 @@ __device__ __forceinline__ void up_chunk(const float* __restrict__ buf, int lx, 
         if (kSelect || pb.active)
             up_part<FB, W, Tf, kSelect>(tap, pb, rb, part, k0, full, ncand, weight_up, fine_chunk, sb, kept_b);
     }
-    if constexpr (!kSelect && W == 8) {
+    if constexpr (!kSelect) {
         // one 256-bit store per fine cell (float32 levels, 32-byte aligned)
         if (pa.active) stg256(reinterpret_cast<float*>(fine_chunk + (int64_t)pa.index * W), kept_a);
         if (pb.active) stg256(reinterpret_cast<float*>(fine_chunk + (int64_t)pb.index * W), kept_b);
@@ -551,9 +513,8 @@ struct UpShared {
 // sh.lut is filled with the level's range weights and the block synchronised before the call.
 // kSelect = false: coarse float32 -> fine float32 in place (and the fine guides);
 // kSelect = true: the last step, fine level-0 costs of type Tf in, the selection out.
-// kWriteGuide: the filtered fine guide is formed and written (kGuideDefault: always except by
-// the chunked selecting step, whose guide nothing reads; the planar one writes it as the
-// reference's filter does).
+// kWriteGuide: the filtered fine guide is formed and written (not by the selecting step, whose guide
+// nothing reads).
 template <int W, typename Tf, bool kSelect, typename GL, bool kWriteGuide, bool kTma = false>
 __device__ __forceinline__ void isb_up_block(const uint8_t* __restrict__ guide_in, const float* __restrict__ cost_in,
                                              uint8_t* __restrict__ guide_io, Tf* __restrict__ cost_fine,
@@ -561,7 +522,7 @@ __device__ __forceinline__ void isb_up_block(const uint8_t* __restrict__ guide_i
                                              float weight_down, const SelectOut& so, int x0, int y, UpShared<W>& sh,
                                              const CUtensorMap* tmap = nullptr, int plane0 = 0, bool withhold = false)
 {
-    static_assert(!kTma || W == 8, "TMA tiles are for the chunked layout");
+    static_assert(W == 8, "the chunked layout");
     const int64_t pin = (int64_t)g.rows_in * g.cols_in, pio = (int64_t)g.rows_out * g.cols_out;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kind = warp >> 2;  // warp-uniform
@@ -956,15 +917,11 @@ static dim3 up1_grid(int cols_in, int rows_in, int instances)
                 (unsigned)instances);
 }
 
-template <int W, bool kSelect>
-constexpr bool kGuideDefault = !kSelect || W == 1;
-
 // blockIdx.z: instance of contiguous levels.  kBlocks: blocks per SM the registers are bounded
-// for (3 for the single-candidate filter; 2 or 3 for the chunked volumes, SSG_TUNE_ISB_UP_BLOCKS and
-// SSG_TUNE_ISB_SELECT_BLOCKS:
-// 3 spills a few of the taps' registers for more resident warps).
-template <int W, typename Tf, bool kSelect, typename GL, int kBlocks = (W == 1 ? 3 : 2),
-          bool kWriteGuide = kGuideDefault<W, kSelect>, bool kTma = false>
+// for (2 or 3, SSG_TUNE_ISB_UP_BLOCKS and SSG_TUNE_ISB_SELECT_BLOCKS: 3 spills a few of the taps'
+// registers for more resident warps).
+template <int W, typename Tf, bool kSelect, typename GL, int kBlocks = 2, bool kWriteGuide = !kSelect,
+          bool kTma = false>
 __global__ void __launch_bounds__(kBatchBlock, kBlocks) isb_up_kernel(const uint8_t* __restrict__ guide_in,
                                                             const float* __restrict__ cost_in,
                                                             uint8_t* __restrict__ guide_io,
@@ -1037,8 +994,7 @@ __global__ void __launch_bounds__(kBatchBlock) isb_down_uneven_kernel(const Leve
                                static_cast<float*>(d.cost_out), g, d.chunks, (int)o, lut);
 }
 
-template <int W, typename Tf, bool kSelect, int kBlocks = (W == 1 ? 3 : 2),
-          bool kWriteGuide = kGuideDefault<W, kSelect>>
+template <int W, typename Tf, bool kSelect, int kBlocks = 2, bool kWriteGuide = !kSelect>
 __global__ void __launch_bounds__(kBatchBlock, kBlocks) isb_up_uneven_kernel(const LevelDesc* __restrict__ descs)
 {
     const LevelDesc& d = descs[blockIdx.z];
@@ -1171,6 +1127,10 @@ static int launch_down(const uint8_t* gi, const Tin* ci, int ri, int cl_i, uint8
 {
     const LevelGeom g{ri, cl_i, ro, cl_o};
     const dim3 grid(grid_1d((int64_t)ro * cl_o, kBatchBlock), instances);
+    if constexpr (W == 1) {
+        if (chunks > 1)
+            return launch_down_planar<GL>(gi, ci, ri, cl_i, go, co, ro, cl_o, chunks, instances, var_inv_i, st);
+    }
     isb_down_kernel<W, Tin, GL><<<grid, kBatchBlock, 0, st>>>(gi, ci, go, co, g, chunks, var_inv_i,
                                                               range_table(var_inv_i, st));
     return launch_status("isb_down_kernel");
@@ -1184,17 +1144,21 @@ static int launch_up(const uint8_t* gi, const float* ci, int rc, int cc, uint8_t
 {
     const LevelGeom g{rc, cc, rf, cf_cols};
     const float* table = range_table(var_inv_i, st);
-    if constexpr (W == 1 && !kSelect) {
-        if (chunks == 1) {
-            if (guide)
-                isb_up1_kernel<GL, true><<<up1_grid(cc, rc, instances), kUp1X * kUp1Y, 0, st>>>(
-                    gi, ci, gio, cf, g, wu, wd, var_inv_i, table);
-            else
-                isb_up1_kernel<GL, false><<<up1_grid(cc, rc, instances), kUp1X * kUp1Y, 0, st>>>(
-                    gi, ci, gio, cf, g, wu, wd, var_inv_i, table);
-            return launch_status("isb_up1_kernel");
+    if constexpr (W == 1) {
+        if constexpr (!kSelect) {
+            if (chunks == 1) {
+                if (guide)
+                    isb_up1_kernel<GL, true><<<up1_grid(cc, rc, instances), kUp1X * kUp1Y, 0, st>>>(
+                        gi, ci, gio, cf, g, wu, wd, var_inv_i, table);
+                else
+                    isb_up1_kernel<GL, false><<<up1_grid(cc, rc, instances), kUp1X * kUp1Y, 0, st>>>(
+                        gi, ci, gio, cf, g, wu, wd, var_inv_i, table);
+                return launch_status("isb_up1_kernel");
+            }
         }
-    }
+        return launch_up_planar<kSelect, GL>(gi, ci, rc, cc, gio, cf, rf, cf_cols, ncand, instances, wu, wd,
+                                             var_inv_i, so, st);
+    } else {
     CUtensorMap map;
     std::memset(&map, 0, sizeof map);
     const dim3 grid = up_grid(cc, rc, instances);
@@ -1220,7 +1184,7 @@ static int launch_up(const uint8_t* gi, const float* ci, int rc, int cc, uint8_t
         const bool tma = tuning(SSG_TUNE_ISB_TILE_TMA) == 1 && encode_tensor_map(&map, ci, 4, dims, strides, box);
         const bool three = tuning(kSelect ? SSG_TUNE_ISB_SELECT_BLOCKS : SSG_TUNE_ISB_UP_BLOCKS) == 3;
         const bool withhold = tma && tuning(SSG_TUNE_TMA_WITHHOLD) == 1;
-        constexpr bool kG = kGuideDefault<W, kSelect>;
+        constexpr bool kG = !kSelect;
         if (tma) {
             const cudaError_t e = clear_tma_abort(st);
             if (e != cudaSuccess) return fail(SSG_ERR_CUDA, "clearing the TMA abort word: %s", cudaGetErrorString(e));
@@ -1237,11 +1201,9 @@ static int launch_up(const uint8_t* gi, const float* ci, int rc, int cc, uint8_t
         else
             isb_up_kernel<W, Tf, kSelect, GL><<<grid, kBatchBlock, 0, st>>>(gi, ci, gio, cf, g, chunks, ncand, wu, wd,
                                                                            var_inv_i, table, so, map, false);
-    } else {
-        isb_up_kernel<W, Tf, kSelect, GL><<<grid, kBatchBlock, 0, st>>>(gi, ci, gio, cf, g, chunks, ncand, wu, wd,
-                                                                       var_inv_i, table, so, map, false);
     }
     return launch_status(kSelect ? "isb_up_kernel<select>" : "isb_up_kernel");
+    }
 }
 
 // The first level of a pyramid's fused tail: the first level s >= 1 of at most `max_pixels`

@@ -220,6 +220,15 @@ struct UpTaps<3> {  // (1,1),(1,2),(2,1),(2,2)
     __device__ static constexpr float base(int) { return 1.0f; }
 };
 
+// whether fine pixel F reads tap t
+template <int F>
+__device__ __forceinline__ constexpr bool uses_tap(int t)
+{
+    for (int i = 0; i < UpTaps<F>::n; ++i)
+        if (UpTaps<F>::tap(i) == t) return true;
+    return false;
+}
+
 // Range weights of fine pixel F from the coarse guides `gd` and its own guide `up`; returns
 // 1 / (sum of weights) and the weighted guide sum `g` (isb_filter.cu:142-267).
 template <int F, typename RW, typename GL = G3>

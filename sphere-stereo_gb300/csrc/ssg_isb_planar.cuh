@@ -1,0 +1,429 @@
+// ISB filter steps on planar volumes of several candidates, [candidates][rows][cols] float32, the
+// reference's layout (python/isb_filter.cu:44-329): the fp32 path, ISB_Filter and the
+// differentiable sweep.
+//
+// A block takes consecutive pixels of the coarse level and all their candidates: each pixel's guide
+// weights are formed once per block, spread over the warps, and left in shared memory; then
+// kRanges groups of threads each take a range of the candidates, every thread keeping its pixel's
+// weights in registers, with no barrier between candidates.  Weights, sums and the reference's
+// operation order are those of ssg_isb_common.cuh, so the bits do not depend on how the candidates
+// are shared out.
+//
+// What bounds the steps: the latency of the loads in flight, against 34 + 134 MB (down) and 34 + 2 x
+// 134 MB (up) to move at 1024^2 x 32 candidates, 25 and 45 us at the measured copy rate.  One block
+// of a tile staged per candidate between two barriers, as the steps ran before, took 74 and 132 us
+// there, and 26 us on every small level, whose time is one thread's chain over all candidates;
+// now 48 and 95 us, and 5 to 8 us.
+#pragma once
+
+#include "ssg_isb_common.cuh"
+
+namespace ssg {
+
+constexpr int kPlanarBlock = 256;
+
+// The range weight of a colour distance from the table in global memory (through L1: a block of 32
+// pixels looks up 256 to 800 of the 766 entries, so a copy per block in shared memory would cost
+// more than the lookups), or evaluated when there is no table.
+struct TableRange {
+    const float* __restrict__ table;
+    float var_inv_i;
+    __device__ __forceinline__ float operator()(int d) const
+    {
+        return table ? __ldg(table + d) : range_weight((float)d, var_inv_i);
+    }
+};
+
+// Columns 2x and 2x + 1 of the three rows a coarse pixel reads, and column 2x - 1 where the previous
+// lane does not hold it.  kPairs: both columns in one 8-byte access (cols_in even, levels 8-byte
+// aligned).
+struct DownCells {
+    float a[3], b[3], l[3];
+};
+template <bool kPairs>
+__device__ __forceinline__ void load_down(const float* __restrict__ c, const int (&row)[3], int x2, int xp, bool left,
+                                          DownCells& d)
+{
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        if constexpr (kPairs) {
+            const float2 v = __ldg(reinterpret_cast<const float2*>(c + row[r] + x2));
+            d.a[r] = v.x;
+            d.b[r] = v.y;
+        } else {
+            d.a[r] = __ldg(c + row[r] + x2);
+            d.b[r] = __ldg(c + row[r] + xp);
+        }
+        if (left) d.l[r] = __ldg(c + row[r] + x2 - 1);
+    }
+}
+
+// Down step of a level pair.  blockIdx.x: group of kPx coarse pixels; blockIdx.y: instance of
+// contiguous volumes.  A lane loads columns 2x and 2x + 1 and takes column 2x - 1 from the lane
+// before it, kDownDepth candidates ahead of their use.
+constexpr int kDownDepth = 2;
+
+template <int kRanges, bool kPairs, typename GL>
+__global__ void __launch_bounds__(kPlanarBlock, 4) isb_down_planar_kernel(
+    const uint8_t* __restrict__ guide_in, const float* __restrict__ cost_in, uint8_t* __restrict__ guide_out,
+    float* __restrict__ cost_out, LevelGeom g, int ncand, float var_inv_i, const float* __restrict__ table)
+{
+    constexpr int kPx = kPlanarBlock / kRanges;
+    __shared__ float sw[8][kPx];
+    const int pin = g.rows_in * g.cols_in, pout = g.rows_out * g.cols_out;  // below 2^31 (check_levels)
+    const int64_t inst = blockIdx.y;
+    guide_in += inst * pin * GL::bytes;
+    guide_out += inst * pout * GL::bytes;
+    cost_in += inst * ncand * pin;
+    cost_out += inst * ncand * pout;
+    const int px = threadIdx.x % kPx, range = threadIdx.x / kPx;
+    const int o = blockIdx.x * kPx + px;
+    const bool in = o < pout;
+    const int oc = min(o, pout - 1);
+    const int y = oc / g.cols_out, x = oc - y * g.cols_out;
+    const int x2 = 2 * x, y2 = 2 * y;
+    const int xp = min(x2 + 1, g.cols_in - 1), xm = max(x2 - 1, 0);
+    const int row[3] = {max(y2 - 1, 0) * g.cols_in, y2 * g.cols_in, min(y2 + 1, g.rows_in - 1) * g.cols_in};
+    const int share = (ncand + kRanges - 1) / kRanges;
+    const int k0 = range * share, k1 = min(k0 + share, ncand);  // uniform over a warp: a range is whole warps
+    const bool left = (threadIdx.x & 31) == 0 && x > 0;
+    DownCells cell[kDownDepth];
+    const float* c = cost_in + (int64_t)k0 * pin;
+#pragma unroll
+    for (int j = 0; j < kDownDepth; ++j)
+        if (k0 + j < k1) load_down<kPairs>(c + (int64_t)j * pin, row, x2, xp, left, cell[j]);
+    // the eight neighbours in the reference's order (isb_filter.cu:75-104)
+    const int idx[8] = {row[0] + xm, row[1] + xm, row[2] + xm, row[2] + x2, row[2] + xp, row[1] + xp, row[0] + xp,
+                        row[0] + x2};
+    const TableRange rw{table, var_inv_i};
+    const typename GL::Pix cur = GL::load(guide_in, row[1] + x2);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        if (i % kRanges == range)
+            sw[i][px] = fmul(i % 2 ? 0.5f : 0.25f, rw(GL::dist(cur, GL::load(guide_in, idx[i]))));
+    __syncthreads();
+    float w[8], wsum = 1.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        w[i] = sw[i][px];
+        wsum = fadd(wsum, w[i]);
+    }
+    if (range == 0 && in) {
+        float gs[3] = {(float)GL::ch(cur, 0), (float)GL::ch(cur, 1), (float)GL::ch(cur, 2)};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const typename GL::Pix nb = GL::load(guide_in, idx[i]);
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) gs[ch] = fadd(gs[ch], fmul((float)GL::ch(nb, ch), w[i]));
+        }
+        const float den = fdiv(1.0f, wsum);
+        uint32_t v[3];
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) v[ch] = __float2uint_rz(fmul(gs[ch], den));
+        GL::store(guide_out, o, v);
+    }
+    __syncwarp();
+    const bool first = x == 0;
+    for (int k = k0; k < k1; k += kDownDepth) {
+#pragma unroll
+        for (int j = 0; j < kDownDepth; ++j) {
+            if (k + j >= k1) break;
+            const DownCells d = cell[j];
+            if (k + j + kDownDepth < k1)
+                load_down<kPairs>(c + (int64_t)kDownDepth * pin, row, x2, xp, left, cell[j]);
+            float m[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const float prev = __shfl_up_sync(0xffffffffu, d.b[r], 1);
+                m[r] = first ? d.a[r] : left ? d.l[r] : prev;
+            }
+            const float t[8] = {m[0], m[1], m[2], d.a[2], d.b[2], d.b[1], d.b[0], d.a[0]};
+            float acc = d.a[1];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc = fadd(acc, fmul(t[i], w[i]));
+            if (in) cost_out[(int64_t)(k + j) * pout + o] = fdiv(acc, wsum);
+            c += pin;
+        }
+    }
+}
+
+// Offsets of the fine pixels' weights and of the reciprocals of their sums in a pixel's 29 values
+template <int F>
+constexpr int up_weight_row()
+{
+    return F == 0 ? 0 : F == 1 ? 9 : F == 2 ? 15 : 21;
+}
+constexpr int kUpInvRow = 25, kUpRows = 29;
+constexpr int kUpDepth = 2;
+
+// Weights of fine pixel F of coarse pixel (x, y) into column `px` of sw, and its filtered guide
+template <int F, int kPx, typename GL>
+__device__ __forceinline__ void planar_fine_setup(const uint8_t* __restrict__ guide_in, uint8_t* __restrict__ guide_io,
+                                                  const LevelGeom& g, int x, int y, bool in_level, float weight_up,
+                                                  float weight_down, const TableRange& range, int px,
+                                                  float (&sw)[kUpRows][kPx])
+{
+    const int fx = 2 * x + (F >= 2 ? 1 : 0), fy = 2 * y + (F & 1);
+    if (!in_level || fx >= g.cols_out || fy >= g.rows_out) return;  // no such pixel: its weights are not read
+    int ci[9];
+    typename GL::Pix gd[9];
+    coarse_neighbourhood<int, GL>(guide_in, g.rows_in, g.cols_in, x, y, ci, gd);  // unused taps are not loaded
+    const int index = fy * g.cols_out + fx;
+    const typename GL::Pix up = GL::load(guide_io, index);
+    float w[UpTaps<F>::n], gs[3];
+    const float inv = fine_weights<F, TableRange, GL>(gd, up, weight_up, weight_down, range, w, gs);
+#pragma unroll
+    for (int i = 0; i < UpTaps<F>::n; ++i) sw[up_weight_row<F>() + i][px] = w[i];
+    sw[kUpInvRow + F][px] = inv;
+    uint32_t v[3];
+#pragma unroll
+    for (int ch = 0; ch < 3; ++ch) v[ch] = __float2uint_rz(fmul(gs[ch], inv));
+    GL::store(guide_io, index, v);
+}
+
+// What one range of consecutive candidates contributes to a pixel's selection: a Selector that saw
+// only its candidates, and its first and last cost for the neighbouring ranges
+struct RangeSelection {
+    float m, M, L, R, first, last;
+    int idx_need;  // 2 x index of the minimum + whether it is the range's last candidate
+};
+
+// The two fine pixels' costs of a row of one candidate.  kPairs: in one 8-byte access (cols_out even
+// and the levels 8-byte aligned, so every row of every plane is).
+template <bool kPairs>
+__device__ __forceinline__ float2 load_fine(const float* __restrict__ c, int at, bool second)
+{
+    if constexpr (kPairs) return *reinterpret_cast<const float2*>(c + at);
+    else return make_float2(c[at], second ? c[at + 1] : 0.0f);
+}
+
+// Candidates [k0, k1) of the two fine pixels FA, FB of one fine row of coarse pixel (x, y) in column
+// `px` of sw: filtered in place, or (kSelect) selected into sel_a, sel_b.
+template <int FA, int FB, bool kSelect, bool kPairs>
+__device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in, float* cost_io, const LevelGeom& g,
+                                              int x, int y, int k0, int k1, float weight_up,
+                                              const float (&sw)[kUpRows][32], int px, RangeSelection* sel_a,
+                                              RangeSelection* sel_b)
+{
+    const int fy = 2 * y + (FA & 1);
+    const bool second = 2 * x + 1 < g.cols_out;
+    const int pin = g.rows_in * g.cols_in, pio = g.rows_out * g.cols_out;
+    const int rr[3] = {max(y - 1, 0) * g.cols_in, y * g.cols_in, min(y + 1, g.rows_in - 1) * g.cols_in};
+    const int cc[3] = {max(x - 1, 0), x, min(x + 1, g.cols_in - 1)};
+    const int f0 = fy * g.cols_out + 2 * x;
+    // fine costs, which come from memory, are loaded kUpDepth candidates ahead of their use; the
+    // coarse taps, which neighbouring threads share in the caches, one ahead
+    float2 own[kUpDepth];
+    const float* c = cost_in + (int64_t)k0 * pin;
+    float* f = cost_io + (int64_t)k0 * pio;
+#pragma unroll
+    for (int j = 0; j < kUpDepth; ++j)
+        if (k0 + j < k1) own[j] = load_fine<kPairs>(f + (int64_t)j * pio, f0, second);
+    float cd[9];
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+        if (uses_tap<FA>(t) || uses_tap<FB>(t)) cd[t] = __ldg(c + rr[t / 3] + cc[t % 3]);
+    float wa[UpTaps<FA>::n], wb[UpTaps<FB>::n];
+#pragma unroll
+    for (int i = 0; i < UpTaps<FA>::n; ++i) wa[i] = sw[up_weight_row<FA>() + i][px];
+#pragma unroll
+    for (int i = 0; i < UpTaps<FB>::n; ++i) wb[i] = sw[up_weight_row<FB>() + i][px];
+    const float inv_a = sw[kUpInvRow + FA][px], inv_b = sw[kUpInvRow + FB][px];
+    Selector sa, sb;
+    float first_a = 0.0f, first_b = 0.0f;
+    for (int k = k0; k < k1; k += kUpDepth) {
+#pragma unroll
+        for (int j = 0; j < kUpDepth; ++j) {
+            if (k + j >= k1) break;
+            float nd[9];
+            if (k + j + 1 < k1) {
+                c += pin;
+#pragma unroll
+                for (int t = 0; t < 9; ++t)
+                    if (uses_tap<FA>(t) || uses_tap<FB>(t)) nd[t] = __ldg(c + rr[t / 3] + cc[t % 3]);
+            }
+            // isb_filter.cu:270-327
+            float va = fmul(weight_up, own[j].x), vb = fmul(weight_up, own[j].y);
+#pragma unroll
+            for (int i = 0; i < UpTaps<FA>::n; ++i) {
+                va = fadd(va, fmul(wa[i], cd[UpTaps<FA>::tap(i)]));
+                if (i < UpTaps<FB>::n) vb = fadd(vb, fmul(wb[i < UpTaps<FB>::n ? i : 0], cd[UpTaps<FB>::tap(i)]));
+            }
+            va = fmul(va, inv_a);
+            vb = fmul(vb, inv_b);
+            if (k + j + kUpDepth < k1) own[j] = load_fine<kPairs>(f + (int64_t)kUpDepth * pio, f0, second);
+            if constexpr (kSelect) {
+                if (k + j == k0) {
+                    first_a = va;
+                    first_b = vb;
+                }
+                sa.push(k + j, va);
+                sb.push(k + j, vb);
+            } else if constexpr (kPairs) {
+                *reinterpret_cast<float2*>(f + f0) = make_float2(va, vb);
+            } else {
+                f[f0] = va;
+                if (second) f[f0 + 1] = vb;
+            }
+            f += pio;
+#pragma unroll
+            for (int t = 0; t < 9; ++t)
+                if (uses_tap<FA>(t) || uses_tap<FB>(t)) cd[t] = nd[t];
+        }
+    }
+    if constexpr (kSelect) {
+        *sel_a = RangeSelection{sa.m, sa.M, sa.L, sa.R, first_a, sa.prev, 2 * sa.idx + (sa.need_right ? 1 : 0)};
+        *sel_b = RangeSelection{sb.m, sb.M, sb.L, sb.R, first_b, sb.prev, 2 * sb.idx + (sb.need_right ? 1 : 0)};
+    }
+}
+
+// Up step of a level pair: coarse filtered level -> fine level in place, or (kSelect) the last
+// step fused with the selection, its candidates shared out in consecutive ranges and combined in
+// candidate order.  A block takes 32 coarse pixels; a warp filters one of their two fine rows in
+// one of kRanges ranges of candidates.  blockIdx.x: group of coarse pixels; blockIdx.y: instance.
+template <int kRanges, bool kSelect, bool kPairs, typename GL>
+__global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges) isb_up_planar_kernel(
+    const uint8_t* __restrict__ guide_in, const float* __restrict__ cost_in, uint8_t* __restrict__ guide_io,
+    float* cost_io, LevelGeom g, int ncand, float weight_up, float weight_down, float var_inv_i,
+    const float* __restrict__ table, SelectOut so)
+{
+    constexpr int kPx = 32;
+    __shared__ float sw[kUpRows][kPx];
+    __shared__ RangeSelection part[kSelect ? kRanges : 1][kSelect ? 4 * kPx : 1];
+    const int pin = g.rows_in * g.cols_in, pio = g.rows_out * g.cols_out;  // below 2^31 (check_levels)
+    const int64_t inst = blockIdx.y;
+    guide_in += inst * pin * GL::bytes;
+    guide_io += inst * pio * GL::bytes;
+    cost_in += inst * ncand * pin;
+    cost_io += inst * ncand * pio;
+    const int px = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int o = blockIdx.x * kPx + px;
+    const bool in = o < pin;
+    const int y = o / g.cols_in, x = o - y * g.cols_in;
+    // weights: the four fine pixels go to four warps
+    const TableRange rw{table, var_inv_i};
+    for (int f = warp; f < 4; f += 2 * kRanges) {
+        switch (f) {
+        case 0: planar_fine_setup<0, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
+        case 1: planar_fine_setup<1, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
+        case 2: planar_fine_setup<2, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
+        default: planar_fine_setup<3, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
+        }
+    }
+    __syncthreads();
+    const int share = (ncand + kRanges - 1) / kRanges, range = warp >> 1;
+    const int k0 = range * share, k1 = min(k0 + share, ncand);
+    if (in && k0 < k1) {
+        if ((warp & 1) == 0)
+            planar_up_row<0, 2, kSelect, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px,
+                                                 &part[kSelect ? range : 0][kSelect ? px : 0],
+                                                 &part[kSelect ? range : 0][kSelect ? 2 * kPx + px : 0]);
+        else if (2 * y + 1 < g.rows_out)
+            planar_up_row<1, 3, kSelect, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px,
+                                                 &part[kSelect ? range : 0][kSelect ? kPx + px : 0],
+                                                 &part[kSelect ? range : 0][kSelect ? 3 * kPx + px : 0]);
+    }
+    if constexpr (kSelect) {
+        __syncthreads();
+        // one thread per fine pixel: the ranges in candidate order, as one Selector would have seen them
+        for (int q = warp; q < 4; q += 2 * kRanges) {
+            const int fx = 2 * x + (q >= 2 ? 1 : 0), fy = 2 * y + (q & 1);
+            if (!in || fx >= g.cols_out || fy >= g.rows_out) continue;
+            Selector s;
+            for (int r = 0; r * share < ncand; ++r) {
+                const RangeSelection p = part[r][q * kPx + px];
+                if (s.need_right) s.R = p.first;
+                s.need_right = false;
+                if (p.m < s.m) {
+                    s.m = p.m;
+                    s.idx = p.idx_need >> 1;
+                    s.L = s.idx == r * share ? s.prev : p.L;
+                    s.R = p.R;
+                    s.need_right = (p.idx_need & 1) != 0;
+                }
+                s.M = fmaxf(p.M, s.M);
+                s.prev = p.last;
+            }
+            const int64_t at = inst * pio + fy * g.cols_out + fx;
+            const float d = select_from(s, ncand, so.d0, so.dl, so.q);
+            so.distance[at] = d;
+            if (so.distance2) so.distance2[at] = d;
+            if (so.index) so.index[at] = s.idx;
+        }
+    }
+}
+
+// Into how many ranges a step's candidates are shared out: a power of two of at most `ncand`.  Every
+// range more repeats the set-up of the pixel's weights, which costs about as much as 10
+// candidates, and a level too small to fill the GPU needs the ranges to keep enough loads in
+// flight.  Measured at 32 candidates, in microseconds for 1, 2, 4 and 8 ranges: the down step to
+// 262144 pixels 54, 49, 48, 52, to 65536 27, 18, 16, 16, to 16384 24, 14, 9, 7; the up step from
+// 262144 pixels (selecting) 116, 128, 152, 192, from 65536 25, 31, 35, 42, from 16384 23, 15, 12, 15,
+// from 4096 22, 14, 10, 8.
+static int fit_ranges(int ranges, int ncand)
+{
+    while (ranges > ncand) ranges /= 2;
+    return ranges;
+}
+static int down_ranges(int64_t pixels, int ncand) { return fit_ranges(pixels >= 32768 ? 4 : 8, ncand); }
+static int up_ranges(int64_t pixels, int ncand)
+{
+    return fit_ranges(pixels >= 49152 ? 1 : pixels >= 24576 ? 2 : pixels >= 8192 ? 4 : 8, ncand);
+}
+
+template <typename GL>
+static int launch_down_planar(const uint8_t* gi, const float* ci, int ri, int cl_i, uint8_t* go, float* co, int ro,
+                              int cl_o, int ncand, int instances, float var_inv_i, cudaStream_t st)
+{
+    const LevelGeom g{ri, cl_i, ro, cl_o};
+    const float* table = range_table(var_inv_i, st);
+    const int64_t pout = (int64_t)ro * cl_o;
+    const int ranges = down_ranges(pout * instances, ncand);
+    const dim3 grid(grid_1d(pout, kPlanarBlock / ranges), instances);
+    const bool pairs = cl_i % 2 == 0 && ((uintptr_t)ci & 7) == 0;
+#define SSG_DOWN_PLANAR(R, P) \
+    isb_down_planar_kernel<R, P, GL><<<grid, kPlanarBlock, 0, st>>>(gi, ci, go, co, g, ncand, var_inv_i, table)
+#define SSG_DOWN_PLANAR2(R) \
+    if (pairs) SSG_DOWN_PLANAR(R, true); \
+    else SSG_DOWN_PLANAR(R, false);
+    if (ranges == 8) { SSG_DOWN_PLANAR2(8) }
+    else if (ranges == 4) { SSG_DOWN_PLANAR2(4) }
+    else if (ranges == 2) { SSG_DOWN_PLANAR2(2) }
+    else { SSG_DOWN_PLANAR2(1) }
+#undef SSG_DOWN_PLANAR2
+#undef SSG_DOWN_PLANAR
+    return launch_status("isb_down_planar_kernel");
+}
+
+template <bool kSelect, typename GL>
+static int launch_up_planar(const uint8_t* gi, const float* ci, int rc, int cc, uint8_t* gio, float* cf, int rf,
+                            int cf_cols, int ncand, int instances, float wu, float wd, float var_inv_i,
+                            const SelectOut& so, cudaStream_t st)
+{
+    const LevelGeom g{rc, cc, rf, cf_cols};
+    const float* table = range_table(var_inv_i, st);
+    const int64_t pin = (int64_t)rc * cc;
+    const bool pairs = cf_cols % 2 == 0 && ((uintptr_t)cf & 7) == 0;
+    const int ranges = up_ranges(pin * instances, ncand);
+    const dim3 grid(grid_1d(pin, 32), instances);
+#define SSG_UP_PLANAR(R, P) \
+    isb_up_planar_kernel<R, kSelect, P, GL><<<grid, 64 * R, 0, st>>>(gi, ci, gio, cf, g, ncand, wu, wd, var_inv_i, \
+                                                                           table, so)
+    if (ranges == 8) {
+        if (pairs) SSG_UP_PLANAR(8, true);
+        else SSG_UP_PLANAR(8, false);
+    } else if (ranges == 4) {
+        if (pairs) SSG_UP_PLANAR(4, true);
+        else SSG_UP_PLANAR(4, false);
+    } else if (ranges == 2) {
+        if (pairs) SSG_UP_PLANAR(2, true);
+        else SSG_UP_PLANAR(2, false);
+    } else {
+        if (pairs) SSG_UP_PLANAR(1, true);
+        else SSG_UP_PLANAR(1, false);
+    }
+#undef SSG_UP_PLANAR
+    return launch_status(kSelect ? "isb_up_planar_kernel<select>" : "isb_up_planar_kernel");
+}
+
+}  // namespace ssg

@@ -16,14 +16,16 @@
 //     float32 as numpy compares a float32 array with a Python float.
 // Sums are taken per block in a fixed order and reduced in a fixed order, so results do not
 // depend on scheduling.
+#include <algorithm>
+
 #include "ssg_common.cuh"
 
 namespace ssg {
 
 constexpr int kEvalBlocks = 304;  // blocks per frame: two per SM
 constexpr int kEvalThreads = 256;
-constexpr int kSsimTileX = 32, kSsimTileY = 8, kSsimWin = 7, kSsimHalf = 3;
-constexpr int kSsimInX = kSsimTileX + kSsimWin - 1, kSsimInY = kSsimTileY + kSsimWin - 1;
+constexpr int kEvalWarps = kEvalThreads / 32;
+constexpr int kSsimWin = 7, kSsimHalf = 3;
 
 struct EvalParams {
     int cols, rows, frames, thresholds;
@@ -51,8 +53,48 @@ __device__ __forceinline__ double block_sum(double v, double* sh)
 
 __device__ __forceinline__ float unit_value(uint8_t v) { return __fdiv_rn((float)v, 255.0f); }
 
+// FP64 runs at a sixty-fourth of the FP32 rate on this GPU (an FP64 operation per colour value of a
+// 2048x1024 panorama costs 11 us), so the sums are kept without it: colour errors as exact
+// integers, distance errors and SSIM values in two floats.
+
+// s.hi + s.lo += v (and + low), the rounding error of the sum kept in lo (Knuth's TwoSum, "The Art of
+// Computer Programming" vol. 2, 4.2.2).  An infinite or NaN v leaves hi as a plain sum would.
+struct TwoFloat {
+    float hi = 0.0f, lo = 0.0f;
+    __device__ __forceinline__ void add(float v, float low = 0.0f)
+    {
+        const float t = __fadd_rn(hi, v), b = __fsub_rn(t, hi);
+        lo += (__fsub_rn(hi, __fsub_rn(t, b)) + __fsub_rn(v, b)) + low;
+        hi = t;
+    }
+    __device__ __forceinline__ double value() const
+    {
+        return fabsf(hi) <= 3.402823466e38f ? (double)hi + (double)lo : (double)hi;
+    }
+};
+
+// Sum of float32 squares d2 in [0, 1] that are multiples of 2^-40, exact: every d2 is split into a
+// multiple of 2^-23 (the sum 1 + d2) and the rest (a multiple of 2^-40 below 2^-24), both read from
+// the bits of float sums.
+struct SquareSum {
+    uint32_t hi = 0, lo = 0;  // of at most 64 values, with the bits of the two biases
+    __device__ __forceinline__ void add(float d2)
+    {
+        const float r = __fadd_rn(d2, 1.0f);
+        hi += __float_as_uint(r) - 0x3F800000u;
+        const float rest = __fsub_rn(d2, __fsub_rn(r, 1.0f));
+        lo += __float_as_uint(__fmaf_rn(rest, 1099511627776.0f, 12582912.0f)) - 0x4B400000u;
+    }
+    __device__ __forceinline__ long long units() const  // multiples of 2^-40
+    {
+        return ((long long)hi << 17) + (long long)(int32_t)lo;
+    }
+};
+
 // Per-pixel sums: squared colour differences, inverse-distance errors and bad-pixel counts.
-// blockIdx.y: frame.
+// blockIdx.y: frame.  kVec: the frame's arrays are read 16 bytes at a time (all four 16-byte aligned
+// in every frame).  Bound by memory: 4 frames of 2048x1024 (117 MB) 450 -> 57 us.
+template <bool kVec>
 __global__ void __launch_bounds__(kEvalThreads) eval_pointwise_kernel(const __grid_constant__ EvalParams p,
                                                                       const uint8_t* __restrict__ rgb,
                                                                       const uint8_t* __restrict__ gt_rgb,
@@ -60,135 +102,249 @@ __global__ void __launch_bounds__(kEvalThreads) eval_pointwise_kernel(const __gr
                                                                       const float* __restrict__ gt_inv,
                                                                       double* __restrict__ partials)
 {
-    __shared__ double sh[kEvalThreads / 32];
-    const int64_t n = (int64_t)p.cols * p.rows;
+    __shared__ double sh[kEvalWarps];
+    __shared__ float unit[256];  // u8 / 255
+    unit[threadIdx.x] = unit_value((uint8_t)threadIdx.x);
+    __syncthreads();
+    const int64_t n = (int64_t)p.cols * p.rows, bytes = 3 * n;
     const int frame = blockIdx.y;
-    rgb += (int64_t)frame * n * 3;
-    gt_rgb += (int64_t)frame * n * 3;
-    inv += (int64_t)frame * n;
-    gt_inv += (int64_t)frame * n;
-    double sq = 0.0, err = 0.0, err2 = 0.0;
-    double bad[SSG_EVAL_MAX_THRESHOLDS];
+    rgb += frame * bytes;
+    gt_rgb += frame * bytes;
+    inv += frame * n;
+    gt_inv += frame * n;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    const auto square = [&](uint32_t g, uint32_t e) {
+        const float d = __fsub_rn(unit[g], unit[e]);
+        return __fmul_rn(d, d);
+    };
+    long long sq = 0;  // multiples of 2^-40
+    const int64_t groups = kVec ? bytes / 16 : 0;
+    for (int64_t i = first; i < groups; i += stride) {
+        const uint4 a = __ldg(reinterpret_cast<const uint4*>(gt_rgb) + i), b = __ldg(reinterpret_cast<const uint4*>(rgb) + i);
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+        SquareSum s;
 #pragma unroll
-    for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k) bad[k] = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        for (int w = 0; w < 4; ++w)
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch) {
-            const float d = __fsub_rn(unit_value(__ldg(gt_rgb + i * 3 + ch)), unit_value(__ldg(rgb + i * 3 + ch)));
-            sq += (double)__fmul_rn(d, d);
-        }
-        const float e = fabsf(__fsub_rn(__ldg(inv + i), __ldg(gt_inv + i)));
-        err += (double)e;
-        err2 += (double)__fmul_rn(e, e);
-#pragma unroll
-        for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k)
-            if (k < p.thresholds && e > p.threshold[k]) bad[k] += 1.0;
+            for (int k = 0; k < 4; ++k) s.add(square((aw[w] >> (8 * k)) & 255u, (bw[w] >> (8 * k)) & 255u));
+        sq += s.units();
     }
+    for (int64_t i = 16 * groups + first; i < bytes; i += stride) {
+        SquareSum s;
+        s.add(square(__ldg(gt_rgb + i), __ldg(rgb + i)));
+        sq += s.units();
+    }
+    TwoFloat err, err2;
+    int bad[SSG_EVAL_MAX_THRESHOLDS];
+#pragma unroll
+    for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k) bad[k] = 0;
+    const auto distance = [&](float a, float b) {
+        const float e = fabsf(__fsub_rn(a, b));
+        err.add(e);
+        err2.add(__fmul_rn(e, e));
+#pragma unroll
+        for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k) {
+            if (k >= p.thresholds) break;
+            bad[k] += e > p.threshold[k] ? 1 : 0;
+        }
+    };
+    const int64_t quads = kVec ? n / 4 : 0;
+    for (int64_t i = first; i < quads; i += stride) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(inv) + i), b = __ldg(reinterpret_cast<const float4*>(gt_inv) + i);
+        distance(a.x, b.x);
+        distance(a.y, b.y);
+        distance(a.z, b.z);
+        distance(a.w, b.w);
+    }
+    for (int64_t i = 4 * quads + first; i < n; i += stride) distance(__ldg(inv + i), __ldg(gt_inv + i));
     double* out = partials + ((int64_t)frame * gridDim.x + blockIdx.x) * eval_slots(p);
-    double s = block_sum(sq, sh);
+    double s = block_sum((double)sq * 0x1p-40, sh);
     if (threadIdx.x == 0) out[kSlotSq] = s;
-    s = block_sum(err, sh);
+    s = block_sum(err.value(), sh);
     if (threadIdx.x == 0) out[kSlotErr] = s;
-    s = block_sum(err2, sh);
+    s = block_sum(err2.value(), sh);
     if (threadIdx.x == 0) out[kSlotErr2] = s;
 #pragma unroll
     for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k) {
         if (k >= p.thresholds) break;
-        s = block_sum(bad[k], sh);
+        s = block_sum((double)bad[k], sh);
         if (threadIdx.x == 0) out[kSlotBad + k] = s;
     }
 }
 
-// SSIM map sums over the cropped region [3, rows - 3) x [3, cols - 3), all three channels:
-// tiles of kSsimTileX x kSsimTileY map pixels, each with its 6-pixel halo staged in shared memory
-// and the five window sums formed by rows, then by columns.  blockIdx.y: frame.
-__global__ void __launch_bounds__(kEvalThreads) eval_ssim_kernel(const __grid_constant__ EvalParams p,
-                                                                 const uint8_t* __restrict__ rgb,
-                                                                 const uint8_t* __restrict__ gt_rgb,
-                                                                 double* __restrict__ partials)
+// ---------------------------------------------------------------------------------------------
+// SSIM in integers.  A colour value is x = RN(u / 255) in float32: a multiple of 2^-31, so with
+// eps(u) = 255 * 2^31 x - 2^31 u, an integer of at most 16320, x = (u + eps(u) 2^-31) / 255 exactly.
+// The window sums of x, x^2 and xy are then integer sums of u and u^2, exact in 32 bits, plus
+// corrections linear in eps (below 2^-24 of them, so that float32 carries them to 2^-48; terms in
+// eps^2 are below 2^-48 and dropped).  With p = u + v and m = u - v, over the N = 49 pixels of a
+// window,
+//     (sum p)^2 -+ (sum m)^2                               are 4 UV and 2 (U^2 + V^2),
+//     N (sum p^2 -+ sum m^2) - ((sum p)^2 -+ (sum m)^2)    are N^2 times 4 cov and 2 (var + var),
+// so the four factors of the SSIM ratio are, up to a common scale, those integers plus a constant
+// each: the variances suffer no cancellation.  The ratio is formed in two floats (error 2^-43).
+//
+// Bound by instruction issue (about 130 per value).  FP64 sums per window took 7471 us for 4 frames
+// of 2048x1024, this form takes 167 us.
+// ---------------------------------------------------------------------------------------------
+constexpr int kSsimCols = 58;  // map columns of a warp: two per lane, the last three lanes are halo
+constexpr int kSums = 8;
+
+// the integer and the fractional part of the constants of the two kinds of factors
+constexpr double kSsimN = kSsimWin * kSsimWin, kSsimScale = 255.0 * 255.0 * kSsimN * kSsimN;
+constexpr double kSsimC1 = 2.0 * (0.01 * 2.0) * (0.01 * 2.0) * kSsimScale;
+constexpr double kSsimC2 = 2.0 * (0.03 * 2.0) * (0.03 * 2.0) * kSsimScale * (kSsimN - 1.0) / kSsimN;
+
+// i + frac + correction as two floats (|i| < 2^31)
+__device__ __forceinline__ void ssim_factor(int i, float rest, float& hi, float& lo)
 {
-    __shared__ double sx[kSsimInY][kSsimInX], sy[kSsimInY][kSsimInX];
-    __shared__ double hs[5][kSsimInY][kSsimTileX];  // row sums of x, y, xx, yy, xy
-    __shared__ double sh[kEvalThreads / 32];
+    hi = __int2float_rn(i);
+    // |i - hi| <= 64, read through the bits of a float
+    lo = __fsub_rn(__int_as_float(0x4B400000 + (i - __float2int_rn(hi))), 12582912.0f) + rest;
+}
+
+// SSIM of one window from its sums of p, m, p^2, m^2, eps_p, eps_m, p eps_p and m eps_m
+__device__ __forceinline__ void ssim_value(const int (&w)[kSums], float& value, float& low)
+{
+    constexpr int kI1 = (int)kSsimC1, kI2 = (int)kSsimC2, kN = kSsimWin * kSsimWin;
+    constexpr float kF1 = (float)(kSsimC1 - kI1), kF2 = (float)(kSsimC2 - kI2), kUnit = 0x1p-30f;  // 2 x 2^-31
+    const int pp = w[0] * w[0], mm = w[1] * w[1];
+    const float pe = (float)w[0] * (float)w[4], me = (float)w[1] * (float)w[5];
+    const float cp = fmaf((float)kN, (float)w[6], -pe), cm = fmaf((float)kN, (float)w[7], -me);
+    float a1, a1l, b1, b1l, a2, a2l, b2, b2l;
+    ssim_factor(pp - mm + kI1, fmaf(kUnit, pe - me, kF1), a1, a1l);
+    ssim_factor(pp + mm + kI1, fmaf(kUnit, pe + me, kF1), b1, b1l);
+    ssim_factor(kN * (w[2] - w[3]) - (pp - mm) + kI2, fmaf(kUnit, cp - cm, kF2), a2, a2l);
+    ssim_factor(kN * (w[2] + w[3]) - (pp + mm) + kI2, fmaf(kUnit, cp + cm, kF2), b2, b2l);
+    const float num = __fmul_rn(a1, a2), den = __fmul_rn(b1, b2);
+    const float num_l = fmaf(a1, a2l, fmaf(a1l, a2, __fmaf_rn(a1, a2, -num)));
+    const float den_l = fmaf(b1, b2l, fmaf(b1l, b2, __fmaf_rn(b1, b2, -den)));
+    const float r = rcp_approx(den);
+    value = __fmul_rn(num, r);
+    low = (__fmaf_rn(-value, den, num) + fmaf(-value, den_l, num_l)) * r;
+}
+
+// The products of one column of a row: (p, m) and their eps packed as 16-bit halves
+struct SsimPixel {
+    uint32_t pm, eps;
+    __device__ __forceinline__ void set(uint32_t u, uint32_t v, const int* __restrict__ table)
+    {
+        const int eu = table[u], ev = table[v];
+        pm = ((u + v) & 0xFFFFu) | ((u - v) << 16);
+        eps = ((uint32_t)(eu + ev) & 0xFFFFu) | ((uint32_t)(eu - ev) << 16);
+    }
+    // adds (kSign = 1) or subtracts its products
+    template <int kSign>
+    __device__ __forceinline__ void into(int (&s)[kSums]) const
+    {
+        const int p = (int16_t)pm, m = (int)pm >> 16, ep = (int16_t)eps, em = (int)eps >> 16;
+        s[0] += kSign * p;
+        s[1] += kSign * m;
+        s[2] += kSign * (p * p);
+        s[3] += kSign * (m * m);
+        s[4] += kSign * ep;
+        s[5] += kSign * em;
+        s[6] += kSign * (p * ep);
+        s[7] += kSign * (m * em);
+    }
+};
+
+// SSIM map sums over the cropped region [3, rows - 3) x [3, cols - 3), all three channels.  A warp takes
+// kSsimCols map columns of one channel and marches down `strip_rows` map rows: every lane keeps
+// the 7-row sums of its two image columns (the rows that leave the window are kept packed in
+// registers), and the 7-column sums come from the neighbouring lanes.  blockIdx.y: frame.
+__global__ void __launch_bounds__(kEvalThreads, 3) eval_ssim_kernel(const __grid_constant__ EvalParams p, int strips,
+                                                                    int strip_rows, const uint8_t* __restrict__ rgb,
+                                                                    const uint8_t* __restrict__ gt_rgb,
+                                                                    double* __restrict__ partials)
+{
+    __shared__ int table[256];
+    __shared__ double sh[kEvalWarps];
+    {
+        const int u = threadIdx.x;
+        const uint32_t x31 = (uint32_t)__fmul_rn(unit_value((uint8_t)u), 2147483648.0f);  // exact
+        table[u] = (int)(255u * x31 - ((uint32_t)u << 31));
+    }
+    __syncthreads();
     const int64_t n = (int64_t)p.cols * p.rows;
     const int frame = blockIdx.y;
     rgb += (int64_t)frame * n * 3;
     gt_rgb += (int64_t)frame * n * 3;
     const int out_cols = p.cols - 2 * kSsimHalf, out_rows = p.rows - 2 * kSsimHalf;
-    const int tiles_x = (out_cols + kSsimTileX - 1) / kSsimTileX;
-    const int tiles = tiles_x * ((out_rows + kSsimTileY - 1) / kSsimTileY);
-    constexpr double kNp = kSsimWin * kSsimWin, kCovNorm = kNp / (kNp - 1.0);
-    constexpr double kC1 = (0.01 * 2.0) * (0.01 * 2.0), kC2 = (0.03 * 2.0) * (0.03 * 2.0);
-    const int tx = threadIdx.x % kSsimTileX, ty = threadIdx.x / kSsimTileX;
-    double acc = 0.0;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int groups = (out_cols + kSsimCols - 1) / kSsimCols;
+    const int tasks = groups * strips * 3;
+    const int lane = threadIdx.x & 31;
+    TwoFloat acc;
+    for (int task = blockIdx.x * kEvalWarps + (threadIdx.x >> 5); task < tasks; task += gridDim.x * kEvalWarps) {
+        const int ch = task % 3, group = (task / 3) % groups, strip = task / 3 / groups;
         // map pixel (x, y) is image pixel (x + 3, y + 3); its window covers image x .. x + 6
-        const int x0 = (t % tiles_x) * kSsimTileX, y0 = (t / tiles_x) * kSsimTileY;
-        for (int ch = 0; ch < 3; ++ch) {
-            __syncthreads();  // the previous tile's sums are consumed
-            for (int q = threadIdx.x; q < kSsimInX * kSsimInY; q += blockDim.x) {
-                const int lx = q % kSsimInX, ly = q / kSsimInX;
-                const int x = min(x0 + lx, p.cols - 1), y = min(y0 + ly, p.rows - 1);
-                const int64_t o = ((int64_t)y * p.cols + x) * 3 + ch;
-                sx[ly][lx] = (double)unit_value(__ldg(gt_rgb + o));
-                sy[ly][lx] = (double)unit_value(__ldg(rgb + o));
-            }
-            __syncthreads();
-            for (int q = threadIdx.x; q < kSsimInY * kSsimTileX; q += blockDim.x) {
-                const int lx = q % kSsimTileX, ly = q / kSsimTileX;
-                double a = 0.0, b = 0.0, aa = 0.0, bb = 0.0, ab = 0.0;
+        const int x = group * kSsimCols + 2 * lane, y0 = strip * strip_rows;
+        const int rows_in = min(strip_rows, out_rows - y0) + kSsimWin - 1;
+        const bool on0 = 2 * lane < kSsimCols && x < out_cols, on1 = 2 * lane < kSsimCols && x + 1 < out_cols;
+        const int64_t c0 = 3 * (int64_t)min(x, p.cols - 1) + ch, c1 = 3 * (int64_t)min(x + 1, p.cols - 1) + ch;
+        const int64_t pitch = 3 * (int64_t)p.cols;
+        const uint8_t* g = gt_rgb + y0 * pitch;
+        const uint8_t* e = rgb + y0 * pitch;
+        SsimPixel ring[kSsimWin][2];
+        int s0[kSums], s1[kSums];
 #pragma unroll
-                for (int k = 0; k < kSsimWin; ++k) {
-                    const double u = sx[ly][lx + k], v = sy[ly][lx + k];
-                    a += u;
-                    b += v;
-                    aa += u * u;
-                    bb += v * v;
-                    ab += u * v;
+        for (int k = 0; k < kSums; ++k) s0[k] = s1[k] = 0;
+        uint32_t u0 = __ldg(g + c0), v0 = __ldg(e + c0), u1 = __ldg(g + c1), v1 = __ldg(e + c1);
+        for (int r = 0; r < rows_in; r += kSsimWin) {
+#pragma unroll
+            for (int i = 0; i < kSsimWin; ++i) {
+                if (r + i >= rows_in) break;
+                SsimPixel a, b;
+                a.set(u0, v0, table);
+                b.set(u1, v1, table);
+                if (r + i + 1 < rows_in) {  // the next row, while this one is summed
+                    g += pitch;
+                    e += pitch;
+                    u0 = __ldg(g + c0), v0 = __ldg(e + c0), u1 = __ldg(g + c1), v1 = __ldg(e + c1);
                 }
-                hs[0][ly][lx] = a;
-                hs[1][ly][lx] = b;
-                hs[2][ly][lx] = aa;
-                hs[3][ly][lx] = bb;
-                hs[4][ly][lx] = ab;
-            }
-            __syncthreads();
-            if (x0 + tx < out_cols && y0 + ty < out_rows) {
-                double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+                a.into<1>(s0);
+                b.into<1>(s1);
+                if (r > 0) {
+                    ring[i][0].into<-1>(s0);
+                    ring[i][1].into<-1>(s1);
+                }
+                ring[i][0] = a;
+                ring[i][1] = b;
+                if (r + i < kSsimWin - 1) continue;
+                int w0[kSums], w1[kSums];
 #pragma unroll
-                for (int k = 0; k < kSsimWin; ++k)
-#pragma unroll
-                    for (int j = 0; j < 5; ++j) m[j] += hs[j][ty + k][tx];
-#pragma unroll
-                for (int j = 0; j < 5; ++j) m[j] /= kNp;
-                const double ux = m[0], uy = m[1];
-                const double vx = kCovNorm * (m[2] - ux * ux), vy = kCovNorm * (m[3] - uy * uy);
-                const double vxy = kCovNorm * (m[4] - ux * uy);
-                const double a1 = 2.0 * ux * uy + kC1, a2 = 2.0 * vxy + kC2;
-                const double b1 = ux * ux + uy * uy + kC1, b2 = vx + vy + kC2;
-                acc += (a1 * a2) / (b1 * b2);
+                for (int k = 0; k < kSums; ++k) {
+                    const int pair = s0[k] + s1[k];
+                    const int mid = __shfl_down_sync(0xffffffffu, pair, 1) + __shfl_down_sync(0xffffffffu, pair, 2);
+                    w0[k] = pair + mid + __shfl_down_sync(0xffffffffu, s0[k], 3);
+                    w1[k] = s1[k] + mid + __shfl_down_sync(0xffffffffu, pair, 3);
+                }
+                float v, low;
+                ssim_value(w0, v, low);
+                if (on0) acc.add(v, low);
+                ssim_value(w1, v, low);
+                if (on1) acc.add(v, low);
             }
         }
     }
-    const double s = block_sum(acc, sh);
+    const double s = block_sum(acc.value(), sh);
     if (threadIdx.x == 0) partials[((int64_t)frame * gridDim.x + blockIdx.x) * eval_slots(p) + kSlotSsim] = s;
 }
 
-// One block per frame: the blocks' partial sums in block order, then the metrics.
+// One block per frame, a warp per slot: the blocks' partial sums in a fixed order, then the metrics.
 __global__ void __launch_bounds__(kEvalThreads) eval_finish_kernel(const __grid_constant__ EvalParams p, int blocks,
                                                                    const double* __restrict__ partials,
                                                                    double* __restrict__ out)
 {
-    __shared__ double sh[kEvalThreads / 32];
-    const int frame = blockIdx.x, slots = eval_slots(p);
+    const int frame = blockIdx.x, slots = eval_slots(p), lane = threadIdx.x & 31;
     const double n = (double)p.cols * p.rows;
     const double map_n = (double)(p.cols - 2 * kSsimHalf) * (p.rows - 2 * kSsimHalf);
     double* o = out + (int64_t)frame * (SSG_EVAL_FIXED_METRICS + p.thresholds);
-    for (int slot = 0; slot < slots; ++slot) {
-        double v = 0.0;
-        for (int b = threadIdx.x; b < blocks; b += blockDim.x) v += partials[((int64_t)frame * blocks + b) * slots + slot];
-        const double s = block_sum(v, sh);
-        if (threadIdx.x == 0) {
+    for (int slot = threadIdx.x >> 5; slot < slots; slot += kEvalWarps) {
+        double s = 0.0;
+        for (int b = lane; b < blocks; b += 32) s += partials[((int64_t)frame * blocks + b) * slots + slot];
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+        if (lane == 0) {
             if (slot == kSlotSq) o[0] = 10.0 * log10(1.0 / (s / (3.0 * n)));
             else if (slot == kSlotSsim) o[1] = s / (3.0 * map_n);
             else if (slot == kSlotErr) o[2] = s / n;
@@ -231,10 +387,23 @@ extern "C" int ssg_eval_panoramas(int cols, int rows, int frames, const uint8_t*
     cudaStream_t st = as_stream(stream);
     double* partials = static_cast<double*>(d_scratch);
     const dim3 grid(kEvalBlocks, frames);
-    eval_pointwise_kernel<<<grid, kEvalThreads, 0, st>>>(p, d_rgb, d_gt_rgb, d_inv_distance, d_gt_inv_distance,
-                                                         partials);
+    const int64_t n = (int64_t)cols * rows;
+    const bool vec = (((uintptr_t)d_rgb | (uintptr_t)d_gt_rgb | (uintptr_t)d_inv_distance | (uintptr_t)d_gt_inv_distance) & 15) == 0 &&
+                     (frames == 1 || n % 16 == 0);
+    if (vec)
+        eval_pointwise_kernel<true><<<grid, kEvalThreads, 0, st>>>(p, d_rgb, d_gt_rgb, d_inv_distance,
+                                                                   d_gt_inv_distance, partials);
+    else
+        eval_pointwise_kernel<false><<<grid, kEvalThreads, 0, st>>>(p, d_rgb, d_gt_rgb, d_inv_distance,
+                                                                    d_gt_inv_distance, partials);
     if (int e = launch_status("eval_pointwise_kernel")) return e;
-    eval_ssim_kernel<<<grid, kEvalThreads, 0, st>>>(p, d_rgb, d_gt_rgb, partials);
+    // one strip of rows per warp of the grid: every strip reads 6 rows more than it sums, so a strip
+    // is at least 8 rows high
+    const int out_rows = rows - 2 * kSsimHalf, groups = (cols - 2 * kSsimHalf + kSsimCols - 1) / kSsimCols;
+    int strips = std::max(1, std::min(kEvalBlocks * kEvalWarps / (3 * groups), (out_rows + 7) / 8));
+    const int strip_rows = (out_rows + strips - 1) / strips;
+    strips = (out_rows + strip_rows - 1) / strip_rows;
+    eval_ssim_kernel<<<grid, kEvalThreads, 0, st>>>(p, strips, strip_rows, d_rgb, d_gt_rgb, partials);
     if (int e = launch_status("eval_ssim_kernel")) return e;
     eval_finish_kernel<<<frames, kEvalThreads, 0, st>>>(p, kEvalBlocks, partials, d_metrics);
     return launch_status("eval_finish_kernel");

@@ -241,8 +241,9 @@ SSG_API int ssg_reproject_distance(const float* d_distance_in, float* d_distance
 
 /* Hole filling: `iterations` launches of inpaintKernel, python/stitcher.cu:283-323
  * (python/stitcher.py:195-200), each a Jacobi step (every pixel reads the map as it was before
- * the step).  Runs as tiled passes of up to 16 steps each in shared memory, alternating between
- * d_distance and d_scratch (rows x cols float32, caller-owned); the result ends in d_distance.
+ * the step).  Runs as tiled passes in shared memory, the first of up to 8 steps and the others of
+ * up to 24, alternating between d_distance and d_scratch (rows x cols float32, caller-owned); the
+ * result ends in d_distance (copied there after an odd number of passes).
  * Table entries whose offset field is 3 are ignored (the table kernel never writes one). */
 SSG_API int ssg_inpaint(float* d_distance, const uint8_t* d_table, float* d_scratch, int cols, int rows, double max_dist,
                 int iterations, void* stream);

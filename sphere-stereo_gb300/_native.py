@@ -43,6 +43,7 @@ TUNE_STAGE_COLUMNS = 15
 STATUS_TMA_TIMEOUT = 1
 STATUS_BARRIER_TIMEOUT = 2
 HOLE_SCRATCH_HEADER = 8
+MAX_FILL_STEPS = 254  # of a batch's hole filling
 ISB_SKIP_FINE_GUIDE = 1
 PIXEL_U8 = 0
 PIXEL_F32 = 1
@@ -255,8 +256,14 @@ def pointers(values) -> ctypes.Array:
     return (ctypes.c_void_p * len(values))(*[int(v) for v in values])
 
 
+def fill_launches(iterations: int) -> int:
+    """Kernels a tiled hole filling launches: one of up to 8 steps, then one per 24 (copies of whole
+    maps not counted)."""
+    return min(iterations, 1) if iterations <= 8 else 1 - (8 - iterations) // 24
+
+
 def hole_filling_launches(iterations: int) -> int:
-    """Kernels one batched hole filling of a uniform batch launches: the scan and step 1, then one
+    """Kernels ssg_inpaint_holes_batch launches: the scan and step 1, then one
     cooperative launch for the other steps (SSG_TUNE_HOLE_PERSISTENT), or a launch per step up to
     the tail (SSG_TUNE_HOLE_TAIL) and two for the tail."""
     if iterations <= 1:
@@ -314,11 +321,11 @@ def kernels_launched(name: str, args) -> int:
     if name in ("ssg_reproject_distance_batch", "ssg_reproject_distance_batch_approx"):
         return 2 if args[8] else 1
     if name == "ssg_inpaint":
-        return -(-int(args[6]) // 16)
+        return fill_launches(int(args[6]))
     if name == "ssg_inpaint_holes_batch":
         return hole_filling_launches(int(args[9]))
     if name == "ssg_inpaint_batch":
-        return -(-int(args[8]) // 16)
+        return fill_launches(int(args[8]))
     if name == "ssg_inpaint_noalloc":
-        return -(-int(args[5]) // 16)
+        return fill_launches(int(args[5]))
     return 1

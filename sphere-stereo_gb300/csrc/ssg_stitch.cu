@@ -6,11 +6,11 @@
 //    compare-and-store twice, stitcher.py:185-192) and targets outside the map are dropped (the
 //    reference's index is unchecked, stitcher.cu:198);
 //  * inpainting is a sequence of Jacobi steps (every pixel reads the map as it was before the
-//    step; the reference updates in place and its result depends on thread timing).  Up to 16
-//    steps run per launch on a shared-memory tile with a 16-pixel halo, ping-ponging between
-//    the map and a scratch map in global memory;
+//    step; the reference updates in place and its result depends on thread timing).  Up to 32
+//    steps run per launch on a shared-memory tile with a 32-pixel halo, from one map to another;
 //  * a table entry whose two best weights stay 0 (outside the model's valid area) encodes the
 //    offsets (0, 0); the reference leaves them uninitialised (stitcher.cu:231).
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -340,113 +340,331 @@ __global__ void __launch_bounds__(kStitchBlock) reproject_frames_kernel(const __
     }
 }
 
-// Tiled Jacobi inpainting: kTileW x kTileH outputs, a halo of kHalo >= steps pixels.
-constexpr int kTileW = 64, kTileH = 32, kHalo = 16;
-constexpr int kRegW = kTileW + 2 * kHalo, kRegH = kTileH + 2 * kHalo;
-constexpr int kInpaintBlock = 512;
-constexpr size_t kInpaintSmem =
-    sizeof(float) * 2 * kRegW * kRegH + sizeof(uchar2) * kRegW * kRegH + sizeof(uint16_t) * kRegW * kRegH;
+// ---------------------------------------------------------------------------------------------
+// Hole filling (inpaintKernel, stitcher.cu:283-323, as Jacobi steps), up to kHalo steps per launch from
+// one map to another.  A block takes kFillW x kFillH output pixels.  Where none of them is a hole
+// that can be filled it copies them; otherwise it holds their region with a halo of kHalo pixels in
+// shared memory and runs every step there:
+//   * only holes change, and a filled hole keeps its value, so each cell has a stamp: 0 not a hole,
+//     kUnfilled an open hole, s a hole filled at step s.  Step s reads a neighbour only when its
+//     stamp is below s, i.e. as it was before the step: one buffer, filled in place;
+//   * step 1 visits every fillable hole; a hole that it leaves open can only be filled at step s > 1
+//     through a neighbour filled at step s - 1 (one filled earlier would have filled it earlier), so
+//     step s visits the open holes that read a pixel filled at step s - 1, and the block stops at
+//     the first step that fills nothing.
+// A cell k pixels inside the region is exact through step k.
+//
+// The steps are a chain of dependent accesses: a step takes a fraction of a microsecond in shared
+// memory, and 4 us and more over lists in global memory (ssg_inpaint_holes_batch).  What is left is
+// bound by instruction issue (73 % in the first launch), so the halo follows the work: on rendered
+// frames 165 K of a 1024^2 map's pixels are fillable holes in 80 % of the tiles, 96 % of what is
+// ever filled is filled within 8 steps, and later steps fill something in 5 % of the tiles.  One
+// launch of 32 steps stages 6 cells per pixel; 8 steps stage 1.9 everywhere, and the other 24 stage
+// 4.4 only where a hole is still open.  Measured, 16 such maps: 465 us over lists, 560 us in one
+// launch, 158 + 104 us in two; two maps of noisy distances: 260 us (two launches of 16 steps over
+// every hole of a tile), 140 us in one, 38 + 48 us now.
+// ---------------------------------------------------------------------------------------------
+constexpr uint8_t kUnfilled = 255;
+constexpr int kFillW = 64, kFillH = 32;
+constexpr int kFillFirst = 8, kFillRest = 24;  // steps of the first launch and of each later one
 
-// One Jacobi step of inpaintKernel (stitcher.cu:283-323) at region cell j, reading `cur`.
-__device__ __forceinline__ float inpaint_cell(const float* cur, const uchar2* tab, int j, float hole_at_least,
-                                              float valid_at_most)
+template <int kHalo>
+struct FillShared {
+    static constexpr int width = kFillW + 2 * kHalo, height = kFillH + 2 * kHalo, cells = width * height;
+    static constexpr int threads = 512;
+    static constexpr int quads = (cells / 4 + threads - 1) / threads;  // groups of four cells per thread
+    float value[cells];
+    uint16_t table[cells];  // entries of the fillable holes, 0 elsewhere
+    uint16_t list[cells];   // cells in the order they were filled
+    uint8_t stamp[cells];
+    uint32_t claimed[cells / 32];
+    int filled[kHalo + 2];  // cells filled by each step
+    static_assert(kHalo % 4 == 0 && cells % 32 == 0 && 4 * quads <= 32 && (kFillW * kFillH) % (4 * threads) == 0,
+                  "rows of whole quads, a bit per cell of a thread");
+};
+
+// one of a table entry's two bytes (stitcher.cu:297-316): whether its neighbour counts (a weight above
+// 0, and no offset field of 3, a step of 2 that the table kernel never writes), and the neighbour's
+// offset in rows of `cols` cells
+__device__ __forceinline__ bool fill_weighted(uint32_t b)
 {
-    const float v = cur[j];
-    if (!(v >= hole_at_least)) return v;  // filled in an earlier step
-    const uchar2 t = tab[j];
-    const int n0 = j + ((t.x & 12) / 4 - 1) * kRegW + ((t.x & 3) - 1);
-    const int n1 = j + ((t.y & 12) / 4 - 1) * kRegW + ((t.y & 3) - 1);
-    // an offset field of 3 (a step of 2) never comes out of the table kernel; such a neighbour is
-    // ignored instead of read outside the 3x3 neighbourhood
-    const bool ok0 = (t.x & 3) != 3 && (t.x & 12) != 12, ok1 = (t.y & 3) != 3 && (t.y & 12) != 12;
-    const float w0 = ok0 ? (float)(t.x & 240) : 0.0f, w1 = ok1 ? (float)(t.y & 240) : 0.0f;
-    float val = 0.0f, ws = 0.0f;
-    if (w0 > 0.0f) {
-        const float sd = cur[n0];
-        if (sd <= valid_at_most) {
-            val = fadd(val, fmul(w0, sd));
-            ws = fadd(ws, w0);
-        }
-    }
-    if (w1 > 0.0f) {
-        const float sd = cur[n1];
-        if (sd <= valid_at_most) {
-            val = fadd(val, fmul(w1, sd));
-            ws = fadd(ws, w1);
-        }
-    }
-    return ws > 0.0f ? fdiv(val, ws) : v;
+    return (b & 240u) != 0u && (b & 3u) != 3u && (b & 12u) != 12u;
+}
+__device__ __forceinline__ int fill_offset(uint32_t b, int cols)
+{
+    return ((int)((b >> 2) & 3u) - 1) * cols + (int)(b & 3u) - 1;
 }
 
-// `steps` Jacobi steps on a 64 x 32 output tile from its region with a 16-pixel halo held in
-// shared memory.  Only hole pixels change, and a pixel that is not a hole never becomes one, so
-// the block lists the region's holes once and updates only those; a tile without holes copies
-// its input through.
-__global__ void __launch_bounds__(kInpaintBlock) inpaint_tile_kernel(const float* __restrict__ src,
-                                                                     float* __restrict__ dst,
-                                                                     const uchar2* __restrict__ table, int cols,
-                                                                     int rows, int references, int steps,
-                                                                     float hole_at_least, float valid_at_most)
+// fills open hole `cell` (table entry t) at step `step` if a usable neighbour exists, and lists it
+template <int kHalo>
+__device__ __forceinline__ void fill_cell(FillShared<kHalo>& sh, int cell, uint32_t t, int step, int list_begin,
+                                          float valid_at_most)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int hole_count;
-    // blockIdx.z: instance (frame * references + reference slot); tables are per slot
-    const int64_t P = (int64_t)cols * rows;
-    src += (int64_t)blockIdx.z * P;
-    dst += (int64_t)blockIdx.z * P;
-    table += (int64_t)(blockIdx.z % references) * P;
-    float* buf0 = reinterpret_cast<float*>(smem);
-    float* buf1 = buf0 + kRegW * kRegH;
-    uchar2* tab = reinterpret_cast<uchar2*>(buf1 + kRegW * kRegH);
-    uint16_t* holes = reinterpret_cast<uint16_t*>(tab + kRegW * kRegH);
-    const int ox = blockIdx.x * kTileW - kHalo, oy = blockIdx.y * kTileH - kHalo;
-    if (threadIdx.x == 0) hole_count = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    // kRegW * kRegH is a multiple of the block size: every warp runs whole iterations
-    for (int j = threadIdx.x; j < kRegW * kRegH; j += blockDim.x) {
-        const int lx = j % kRegW, ly = j / kRegW;
-        const int x = ox + lx, y = oy + ly;
-        const bool in = x >= 0 && x < cols && y >= 0 && y < rows;
-        const int64_t g = (int64_t)y * cols + x;
-        const float v = in ? src[g] : 0.0f;
-        buf0[j] = v;
-        buf1[j] = v;
-        tab[j] = in ? table[g] : make_uchar2(0, 0);
-        // hole test of stitcher.cu:287 and the interior test of :291; neighbours must lie inside
-        // the region (pixels whose neighbours do not are farther than `steps` from the outputs)
-        const bool hole = in && v >= hole_at_least && x >= 1 && y >= 1 && x < cols - 1 && y < rows - 1 && lx >= 1 &&
-                          ly >= 1 && lx < kRegW - 1 && ly < kRegH - 1;
-        const unsigned mask = __ballot_sync(0xffffffffu, hole);
-        int base = 0;
-        if (lane == 0 && mask) base = atomicAdd(&hole_count, __popc(mask));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (hole) holes[base + __popc(mask & ((1u << lane) - 1))] = (uint16_t)j;
-    }
-    __syncthreads();
-    const int n = hole_count;
-    float* cur = buf0;
-    float* nxt = buf1;
-    if (n > 0)
-        for (int s = 0; s < steps; ++s) {
-            for (int h = threadIdx.x; h < n; h += blockDim.x) {
-                const int j = holes[h];
-                nxt[j] = inpaint_cell(cur, tab, j, hole_at_least, valid_at_most);
+    float val = 0.0f, ws = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t b = i == 0 ? t & 255u : t >> 8;
+        const int n = cell + fill_offset(b, FillShared<kHalo>::width);
+        if (fill_weighted(b) && sh.stamp[n] < step) {
+            const float sd = sh.value[n], w = (float)(b & 240u);
+            if (sd <= valid_at_most) {
+                val = fadd(val, fmul(w, sd));
+                ws = fadd(ws, w);
             }
-            __syncthreads();
-            float* tmp = cur;
-            cur = nxt;
-            nxt = tmp;
         }
-    for (int j = threadIdx.x; j < kTileW * kTileH; j += blockDim.x) {
-        const int lx = kHalo + j % kTileW, ly = kHalo + j / kTileW;
-        const int x = ox + lx, y = oy + ly;
-        if (x < cols && y < rows) dst[(int64_t)y * cols + x] = cur[ly * kRegW + lx];
     }
+    if (!(ws > 0.0f)) return;
+    sh.value[cell] = fdiv(val, ws);
+    sh.stamp[cell] = (uint8_t)step;
+    // one atomic for the lanes that got here together
+    const unsigned mask = __activemask(), before = mask & ((1u << (threadIdx.x & 31)) - 1u);
+    int at = 0;
+    if (before == 0u) at = atomicAdd(&sh.filled[step], __popc(mask));
+    sh.list[list_begin + __shfl_sync(mask, at, __ffs(mask) - 1) + __popc(before)] = (uint16_t)cell;
+}
+
+// The maps of a launch: map z of blockIdx.z
+struct FillMap {
+    int cols, rows;
+    const float* src;
+    float* dst;
+    const uint16_t* table;
+};
+struct UniformFill {  // instances of one size, tables per reference slot
+    int cols, rows, references;
+    const float* src;
+    float* dst;
+    const uint8_t* tables;
+    __device__ __forceinline__ FillMap at(int z) const
+    {
+        const int64_t P = (int64_t)cols * rows;
+        return FillMap{cols, rows, src + z * P, dst + z * P,
+                       reinterpret_cast<const uint16_t*>(tables) + (z % references) * P};
+    }
+};
+
+template <int kHalo, typename Maps>
+__global__ void __launch_bounds__(FillShared<kHalo>::threads) fill_holes_kernel(const Maps maps, int steps,
+                                                                               float hole_at_least,
+                                                                               float valid_at_most)
+{
+    using Shared = FillShared<kHalo>;
+    constexpr int W = Shared::width, kThreads = Shared::threads;
+    extern __shared__ __align__(16) unsigned char fill_smem[];
+    Shared& sh = *reinterpret_cast<Shared*>(fill_smem);
+    const FillMap m = maps.at(blockIdx.z);
+    const int x0 = blockIdx.x * kFillW, y0 = blockIdx.y * kFillH;
+    if (x0 >= m.cols || y0 >= m.rows) return;  // no such map or tile (maps of several sizes)
+    // four cells of a row and their table entries: one access each where every row starts on a 16-byte
+    // (8-byte) boundary.  Both are loaded unconditionally, so that a block waits for memory once.
+    const bool vec = m.cols % 4 == 0 && (((uintptr_t)m.src | (uintptr_t)m.dst) & 15) == 0 && ((uintptr_t)m.table & 7) == 0;
+    const auto load4 = [&](int x, int y, float (&v)[4], uint2& t) {
+        v[0] = v[1] = v[2] = v[3] = 0.0f;
+        t = make_uint2(0u, 0u);
+        if (y < 0 || y >= m.rows) return;
+        const int64_t at = (int64_t)y * m.cols + x;
+        if (vec) {
+            if (x < 0 || x >= m.cols) return;
+            const float4 q = __ldg(reinterpret_cast<const float4*>(m.src + at));
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+            t = __ldg(reinterpret_cast<const uint2*>(m.table + at));
+        } else {
+            uint32_t e[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool in = x + i >= 0 && x + i < m.cols;
+                v[i] = in ? __ldg(m.src + at + i) : 0.0f;
+                e[i] = in ? __ldg(m.table + at + i) : 0u;
+            }
+            t = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+        }
+    };
+    const auto store4 = [&](int x, int y, const float (&v)[4]) {
+        if (y >= m.rows) return;
+        float* p = m.dst + (int64_t)y * m.cols + x;
+        if (vec) {
+            if (x < m.cols) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (x + i < m.cols) p[i] = v[i];
+        }
+    };
+    const auto any_hole = [&](const float (&v)[4]) {
+        return v[0] >= hole_at_least || v[1] >= hole_at_least || v[2] >= hole_at_least || v[3] >= hole_at_least;
+    };
+    // the table entry of cell i of a quad at (x, y) if it is a hole of the map's interior
+    // (stitcher.cu:287, :291) with a weighted neighbour, else 0
+    const auto hole_entry = [&](int x, int y, int i, const float (&v)[4], const uint2& q) -> uint32_t {
+        const uint32_t t = ((i < 2 ? q.x : q.y) >> (16 * (i & 1))) & 0xFFFFu;
+        const bool hole = v[i] >= hole_at_least && x + i >= 1 && y >= 1 && x + i < m.cols - 1 && y < m.rows - 1;
+        return hole && (fill_weighted(t & 255u) || fill_weighted(t >> 8)) ? t : 0u;
+    };
+    constexpr int kOwn = kFillW * kFillH / (4 * kThreads), kOwnRows = kThreads / (kFillW / 4);
+    const int tx = 4 * (threadIdx.x % (kFillW / 4)), ty = threadIdx.x / (kFillW / 4);  // of its first own quad
+    if constexpr (kHalo > kFillFirst) {
+        // after the first launch most tiles hold no hole that can still be filled
+        float v[kOwn][4];
+        uint2 t[kOwn];
+        bool any = false;
+#pragma unroll
+        for (int r = 0; r < kOwn; ++r) load4(x0 + tx, y0 + ty + r * kOwnRows, v[r], t[r]);
+#pragma unroll
+        for (int r = 0; r < kOwn; ++r)
+            if (any_hole(v[r]))
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    any = any || hole_entry(x0 + tx, y0 + ty + r * kOwnRows, i, v[r], t[r]) != 0u;
+        if (!__syncthreads_or(any)) {
+#pragma unroll
+            for (int r = 0; r < kOwn; ++r) store4(x0 + tx, y0 + ty + r * kOwnRows, v[r]);
+            return;
+        }
+    }
+    for (int i = threadIdx.x; i < Shared::cells / 32; i += kThreads) sh.claimed[i] = 0;
+    if (threadIdx.x < kHalo + 2) sh.filled[threadIdx.x] = 0;
+    uint32_t open = 0;  // bit 4 r + i: cell i of the thread's r-th quad is a fillable hole
+    {
+        float v[Shared::quads][4];
+        uint2 t[Shared::quads];
+#pragma unroll
+        for (int r = 0; r < Shared::quads; ++r) {
+            const int cell = 4 * (threadIdx.x + r * kThreads), ly = cell / W, lx = cell - ly * W;
+            if (cell < Shared::cells) load4(x0 - kHalo + lx, y0 - kHalo + ly, v[r], t[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < Shared::quads; ++r) {
+            const int cell = 4 * (threadIdx.x + r * kThreads), ly = cell / W, lx = cell - ly * W;
+            if (cell >= Shared::cells) break;
+            *reinterpret_cast<float4*>(sh.value + cell) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+            uint32_t stamps = 0;
+            uint2 entries = make_uint2(0u, 0u);
+            if (any_hole(v[r])) {
+                uint32_t e[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    // a hole on the region's border has neighbours outside: it is kHalo steps away
+                    const bool inside = lx + i >= 1 && lx + i < W - 1 && ly >= 1 && ly < Shared::height - 1;
+                    e[i] = inside ? hole_entry(x0 - kHalo + lx, y0 - kHalo + ly, i, v[r], t[r]) : 0u;
+                    if (e[i]) open |= 1u << (4 * r + i);
+                    if (v[r][i] >= hole_at_least) stamps |= (uint32_t)kUnfilled << (8 * i);
+                }
+                entries = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+            }
+            *reinterpret_cast<uint32_t*>(sh.stamp + cell) = stamps;
+            *reinterpret_cast<uint2*>(sh.table + cell) = entries;
+        }
+    }
+    __syncthreads();
+    while (open) {
+        const int bit = __ffs(open) - 1;
+        open &= open - 1;
+        const int cell = 4 * (threadIdx.x + (bit >> 2) * kThreads) + (bit & 3);
+        const uint32_t t = sh.table[cell], b0 = t & 255u, b1 = t >> 8;
+        // most holes lie among holes: their neighbours' stamps are all that is read
+        if ((fill_weighted(b0) && sh.stamp[cell + fill_offset(b0, W)] == 0) ||
+            (fill_weighted(b1) && sh.stamp[cell + fill_offset(b1, W)] == 0))
+            fill_cell(sh, cell, t, 1, 0, valid_at_most);
+    }
+    __syncthreads();
+    int begin = 0, count = sh.filled[1];
+    for (int step = 2; step <= steps && count > 0; ++step) {
+        // one thread per (cell filled at the last step, neighbour)
+        for (int h = threadIdx.x; h < 8 * count; h += kThreads) {
+            const int p = sh.list[begin + (h >> 3)], k = h & 7;
+            const int dx = k < 3 ? k - 1 : k == 3 ? -1 : k == 4 ? 1 : k - 6;
+            const int dy = k < 3 ? -1 : k < 5 ? 0 : 1;
+            const int q = p + dy * W + dx;  // p is not on the region's border
+            const uint32_t t = sh.table[q];
+            if (t == 0u || sh.stamp[q] != kUnfilled) continue;
+            const uint32_t b0 = t & 255u, b1 = t >> 8;
+            const bool reads = (fill_weighted(b0) && q + fill_offset(b0, W) == p) ||
+                               (fill_weighted(b1) && q + fill_offset(b1, W) == p);
+            // no other thread has taken q
+            if (reads && !(atomicOr(&sh.claimed[q >> 5], 1u << (q & 31)) & (1u << (q & 31))))
+                fill_cell(sh, q, t, step, begin + count, valid_at_most);
+        }
+        __syncthreads();
+        begin += count;
+        count = sh.filled[step];
+    }
+#pragma unroll
+    for (int r = 0; r < kOwn; ++r) {
+        const float4 q = *reinterpret_cast<const float4*>(sh.value + (kHalo + ty + r * kOwnRows) * W + kHalo + tx);
+        const float v[4] = {q.x, q.y, q.z, q.w};
+        store4(x0 + tx, y0 + ty + r * kOwnRows, v);
+    }
+}
+
+// one launch: up to kHalo steps of every map
+template <int kHalo, typename Maps>
+static int fill_pass(const Maps& maps, int max_cols, int max_rows, int count, int steps, double max_dist,
+                     cudaStream_t st)
+{
+    // more than 48 KB of shared memory: opted in once per device
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return launch_status("cudaGetDevice");
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(done.load() & bit)) {
+        const cudaError_t e = cudaFuncSetAttribute(fill_holes_kernel<kHalo, Maps>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)sizeof(FillShared<kHalo>));
+        if (e != cudaSuccess)
+            return fail(SSG_ERR_CUDA, "cudaFuncSetAttribute(fill_holes_kernel): %s", cudaGetErrorString(e));
+        done.fetch_or(bit);
+    }
+    // hole: distance >= MAX_DIST + 0.1 (double, stitcher.cu:287); usable neighbour:
+    // distance <= MAX_DIST + 0.1f (stitcher.cu:311)
+    const float hole = float_at_least(max_dist + 0.1), ok = float_at_most(max_dist + (double)0.1f);
+    const dim3 grid((max_cols + kFillW - 1) / kFillW, (max_rows + kFillH - 1) / kFillH, count);
+    fill_holes_kernel<kHalo, Maps><<<grid, FillShared<kHalo>::threads, sizeof(FillShared<kHalo>), st>>>(maps, steps,
+                                                                                                      hole, ok);
+    return launch_status("fill_holes_kernel");
+}
+
+// launches of `iterations` steps: the first of kFillFirst, the others of up to kFillRest
+int fill_passes(int iterations)
+{
+    return iterations <= kFillFirst ? (iterations > 0) : 1 + (iterations - kFillFirst + kFillRest - 1) / kFillRest;
+}
+
+// `iterations` steps, launch by launch; maps(pass) gives the maps that pass reads and writes
+template <typename Pass>
+static int fill_steps(const Pass& maps, int max_cols, int max_rows, int count, int iterations, double max_dist,
+                      cudaStream_t st)
+{
+    for (int pass = 0, done = 0; done < iterations; ++pass) {
+        const int left = iterations - done, steps = std::min(left, pass == 0 ? kFillFirst : kFillRest);
+        const int e = steps <= kFillFirst ? fill_pass<kFillFirst>(maps(pass), max_cols, max_rows, count, steps, max_dist, st)
+                                          : fill_pass<kFillRest>(maps(pass), max_cols, max_rows, count, steps, max_dist, st);
+        if (e) return e;
+        done += steps;
+    }
+    return SSG_OK;
+}
+
+static int copy_maps(float* to, const float* from, int64_t floats, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemcpyAsync(to, from, sizeof(float) * (size_t)floats, cudaMemcpyDeviceToDevice, st);
+    return e == cudaSuccess ? SSG_OK : fail(SSG_ERR_CUDA, "cudaMemcpyAsync: %s", cudaGetErrorString(e));
+}
+
+// in place on `map`, by way of `scratch`
+static int fill_uniform(float* map, float* scratch, const uint8_t* tables, int cols, int rows, int instances,
+                        int references, double max_dist, int iterations, cudaStream_t st)
+{
+    SSG_REQUIRE(((uintptr_t)tables & 1) == 0, "tables must be 2-byte aligned");
+    const auto maps = [&](int pass) {
+        return UniformFill{cols, rows, references, pass % 2 ? scratch : map, pass % 2 ? map : scratch, tables};
+    };
+    if (int e = fill_steps(maps, cols, rows, instances, iterations, max_dist, st)) return e;
+    return fill_passes(iterations) % 2 ? copy_maps(map, scratch, (int64_t)cols * rows * instances, st) : SSG_OK;
 }
 
 // ---------------------------------------------------------------------------------------------
-// Hole filling over lists of holes (the batched path), with the result of the Jacobi steps above.
+// Hole filling over lists of holes in global memory (ssg_inpaint_holes_batch), in place and with the
+// result of the steps above.
 // Only holes change, a filled hole keeps its value from then on, and a hole whose two table
 // weights are 0 (outside the model's valid area) never changes.  Every pixel gets a one-byte
 // stamp: 0 for a pixel that is not a hole, kUnfilled for a hole, s for a hole filled at step s.
@@ -459,7 +677,6 @@ __global__ void __launch_bounds__(kInpaintBlock) inpaint_tile_kernel(const float
 //     holes that read a pixel filled at step s - 1: the work of a step is its frontier.  A claim
 //     word per pixel (the last step that queued it) keeps a hole from being visited twice.
 // ---------------------------------------------------------------------------------------------
-constexpr uint8_t kUnfilled = 255;
 constexpr int kMaxListIterations = 254;
 
 struct HoleOffsets {
@@ -1250,21 +1467,6 @@ __global__ void __launch_bounds__(kStitchBlock) merge_frames_kernel(const __grid
     }
 }
 
-// The tile kernel needs more than 48 KB of dynamic shared memory: opt in once per device.
-static int enable_inpaint_smem()
-{
-    static std::atomic<uint64_t> done{0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return launch_status("cudaGetDevice");
-    const uint64_t bit = 1ull << (dev & 63);
-    if (done.load() & bit) return SSG_OK;
-    const cudaError_t e =
-        cudaFuncSetAttribute(inpaint_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInpaintSmem);
-    if (e != cudaSuccess) return fail(SSG_ERR_CUDA, "cudaFuncSetAttribute(inpaint_tile_kernel): %s", cudaGetErrorString(e));
-    done.fetch_or(bit);
-    return SSG_OK;
-}
-
 static int check_intrinsics(const ssg_intrinsics* k, int n)
 {
     SSG_REQUIRE(k, "intrinsics must not be NULL");
@@ -1435,35 +1637,12 @@ extern "C" int ssg_inpaint(float* d_distance, const uint8_t* d_table, float* d_s
 extern "C" int ssg_inpaint_batch(float* d_distance, const uint8_t* d_tables, float* d_scratch, int cols, int rows,
                                  int instances, int references, double max_dist, int iterations, void* stream)
 {
-    const uint8_t* d_table = d_tables;
-    SSG_REQUIRE(d_distance && d_table && d_scratch && d_distance != d_scratch, "null or aliased pointer");
+    SSG_REQUIRE(d_distance && d_tables && d_scratch && d_distance != d_scratch, "null or aliased pointer");
     SSG_REQUIRE(cols > 0 && rows > 0 && iterations >= 0, "invalid sizes");
     SSG_REQUIRE(references >= 1 && instances >= 1 && instances <= 65535 && instances % references == 0,
                 "instances must be a positive multiple of references");
-    if (int e = enable_inpaint_smem()) return e;
-    // hole: distance >= MAX_DIST + 0.1 (double, stitcher.cu:287); usable neighbour:
-    // distance <= MAX_DIST + 0.1f (stitcher.cu:311)
-    const float hole = float_at_least(max_dist + 0.1);
-    const float ok = float_at_most(max_dist + (double)0.1f);
-    dim3 grid((cols + kTileW - 1) / kTileW, (rows + kTileH - 1) / kTileH, instances);
-    float* a = d_distance;
-    float* b = d_scratch;
-    for (int done = 0; done < iterations;) {
-        const int steps = iterations - done < kHalo ? iterations - done : kHalo;
-        inpaint_tile_kernel<<<grid, kInpaintBlock, kInpaintSmem, as_stream(stream)>>>(
-            a, b, reinterpret_cast<const uchar2*>(d_table), cols, rows, references, steps, hole, ok);
-        if (int e = launch_status("inpaint_tile_kernel")) return e;
-        float* t = a;
-        a = b;
-        b = t;
-        done += steps;
-    }
-    if (a != d_distance) {
-        cudaError_t e = cudaMemcpyAsync(d_distance, a, sizeof(float) * (size_t)cols * rows * instances,
-                                        cudaMemcpyDeviceToDevice, as_stream(stream));
-        if (e != cudaSuccess) return fail(SSG_ERR_CUDA, "cudaMemcpyAsync: %s", cudaGetErrorString(e));
-    }
-    return SSG_OK;
+    return fill_uniform(d_distance, d_scratch, d_tables, cols, rows, instances, references, max_dist, iterations,
+                        as_stream(stream));
 }
 
 namespace ssg {
@@ -1472,27 +1651,26 @@ namespace ssg {
 // Stitch of an uneven batch: every job has its own rig, map and panorama sizes; its maps are
 // concatenated job by job (StitchJob::map_begin).
 // ---------------------------------------------------------------------------------------------
-struct JobMaps {
+// blockIdx.z of the hole filling: job * max_references + reference slot
+struct JobFill {
     const StitchJob* jobs;
-    int n;
-    __device__ __forceinline__ MapPixel at(int64_t g) const
+    int max_references;
+    bool to_raw;
+    __device__ __forceinline__ FillMap at(int z) const
     {
-        int lo = 0, hi = n - 1;  // the last job whose maps begin at or before g
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (jobs[mid].map_begin <= g) lo = mid;
-            else hi = mid - 1;
-        }
-        const StitchJob& J = jobs[lo];
-        const int64_t P = (int64_t)J.cols * J.rows, off = g - J.map_begin, slot = off / P, j = off - slot * P;
-        return MapPixel{J.cols, J.rows, (int)(j % J.cols), (int)(j / J.cols),
-                        reinterpret_cast<const uchar2*>(J.tables) + slot * P};
+        const StitchJob& J = jobs[z / max_references];
+        const int slot = z % max_references;
+        if (slot >= J.references) return FillMap{0, 0, nullptr, nullptr, nullptr};
+        const int64_t P = (int64_t)J.cols * J.rows;
+        float *raw = J.raw + slot * P, *filled = J.reprojected + slot * P;
+        return FillMap{J.cols, J.rows, to_raw ? filled : raw, to_raw ? raw : filled,
+                       reinterpret_cast<const uint16_t*>(J.tables) + slot * P};
     }
 };
 
 // blockIdx.y: job * max_references + reference slot
 __global__ void __launch_bounds__(kStitchBlock) reproject_uneven_kernel(const StitchJob* __restrict__ jobs,
-                                                                        int max_references)
+                                                                        int max_references, bool to_raw)
 {
     const StitchJob& J = jobs[blockIdx.y / max_references];
     const int slot = blockIdx.y % max_references;
@@ -1502,7 +1680,8 @@ __global__ void __launch_bounds__(kStitchBlock) reproject_uneven_kernel(const St
     // the uniform batch's arithmetic (reproject_frames_kernel<true>)
     float ray[3];
     pixel_ray(J.k[slot], J.cols, i, ray);
-    reproject_ray_fast(J.k[slot], J.t[slot], ray, J.distance + slot * P, J.reprojected + slot * P, J.cols, P, i);
+    reproject_ray_fast(J.k[slot], J.t[slot], ray, J.distance + slot * P,
+                       (to_raw ? J.raw : J.reprojected) + slot * P, J.cols, P, i);
 }
 
 // the approximate merge (merge_frames_kernel's arithmetic) of one job's panorama; blockIdx.y: job
@@ -1540,20 +1719,21 @@ __global__ void __launch_bounds__(kStitchBlock) merge_uneven_kernel(const Stitch
     for (int ch = 0; ch < 3; ++ch) J.rgb[3 * i + ch] = (uint8_t)__float2uint_rz(fminf(rgb[ch], 255.0f));
 }
 
-int launch_stitch_uneven(const StitchJob* d_jobs, int jobs, float* d_maps, int64_t total_map_pixels,
-                         int max_map_pixels, int max_pano_pixels, int max_references, double max_dist,
-                         int iterations, uint8_t* d_stamps, int32_t* d_holes, cudaStream_t st)
+int launch_stitch_uneven(const StitchJob* d_jobs, int jobs, float* d_maps, float* d_raw, int64_t total_map_pixels,
+                         int max_map_pixels, int max_map_cols, int max_map_rows, int max_pano_pixels,
+                         int max_references, double max_dist, int iterations, cudaStream_t st)
 {
     SSG_REQUIRE(iterations >= 0 && iterations <= kMaxListIterations, "iterations %d outside [0, %d]", iterations,
                 kMaxListIterations);
     SSG_REQUIRE(total_map_pixels < ((int64_t)1 << 31), "too many map pixels");
-    if (int e = fill_map(d_maps, total_map_pixels, 1e8f, st)) return e;
+    // the launches of the hole filling alternate between the two maps and end in d_maps
+    const bool to_raw = fill_passes(iterations) % 2 != 0;
+    if (int e = fill_map(to_raw ? d_raw : d_maps, total_map_pixels, 1e8f, st)) return e;
     reproject_uneven_kernel<<<dim3(grid_1d(max_map_pixels, kStitchBlock), jobs * max_references), kStitchBlock, 0,
-                              st>>>(d_jobs, max_references);
+                              st>>>(d_jobs, max_references, to_raw);
     if (int e = launch_status("reproject_uneven_kernel")) return e;
-    if (int e = inpaint_lists(JobMaps{d_jobs, jobs}, total_map_pixels, d_maps, d_stamps, d_holes, max_dist,
-                              iterations, st))
-        return e;
+    const auto maps = [&](int pass) { return JobFill{d_jobs, max_references, (pass % 2 != 0) == to_raw}; };
+    if (int e = fill_steps(maps, max_map_cols, max_map_rows, jobs * max_references, iterations, max_dist, st)) return e;
     merge_uneven_kernel<<<dim3(grid_1d(max_pano_pixels, kStitchBlock), jobs), kStitchBlock, 0, st>>>(d_jobs);
     return launch_status("merge_uneven_kernel");
 }
@@ -1743,28 +1923,7 @@ extern "C" int ssg_inpaint_noalloc(float* d_distance, const uint8_t* d_table, in
                     cols, rows, (long long)cols * rows, (long long)kNoAllocMaxPixels);
     float* scratch = nullptr;
     if (int e = noalloc_scratch_address(&scratch)) return e;
-    if (int e = enable_inpaint_smem()) return e;
     // every pass writes every pixel of its destination, so nothing left in the scratch by an
     // earlier call is read
-    const float hole = float_at_least(max_dist + 0.1);
-    const float ok = float_at_most(max_dist + (double)0.1f);
-    dim3 grid((cols + kTileW - 1) / kTileW, (rows + kTileH - 1) / kTileH, 1);
-    float* a = d_distance;
-    float* b = scratch;
-    for (int done = 0; done < iterations;) {
-        const int steps = iterations - done < kHalo ? iterations - done : kHalo;
-        inpaint_tile_kernel<<<grid, kInpaintBlock, kInpaintSmem, as_stream(stream)>>>(
-            a, b, reinterpret_cast<const uchar2*>(d_table), cols, rows, 1, steps, hole, ok);
-        if (int e = launch_status("inpaint_tile_kernel")) return e;
-        float* t = a;
-        a = b;
-        b = t;
-        done += steps;
-    }
-    if (a != d_distance) {
-        cudaError_t e = cudaMemcpyAsync(d_distance, a, sizeof(float) * (size_t)cols * rows, cudaMemcpyDeviceToDevice,
-                                        as_stream(stream));
-        if (e != cudaSuccess) return fail(SSG_ERR_CUDA, "cudaMemcpyAsync: %s", cudaGetErrorString(e));
-    }
-    return SSG_OK;
+    return fill_uniform(d_distance, scratch, d_table, cols, rows, 1, 1, max_dist, iterations, as_stream(stream));
 }

@@ -43,9 +43,9 @@ struct ssg_uneven_batch {
     std::vector<ssg::Step> steps;
     std::vector<ssg::StitchJob> jobs;
     size_t sweep_offset = 0, levels_offset = 0, jobs_offset = 0, plan_bytes = 0;
-    size_t maps_offset = 0, stamps_offset = 0, holes_offset = 0, scratch_bytes = 0;
+    size_t maps_offset = 0, raw_offset = 0, scratch_bytes = 0;
     int total_tiles = 0, storage = SSG_STORAGE_F16, iterations = 0, max_references = 1;
-    int max_map_pixels = 0, max_pano_pixels = 0;
+    int max_map_pixels = 0, max_map_cols = 0, max_map_rows = 0, max_pano_pixels = 0;
     int64_t total_map_pixels = 0;
     double max_dist = 0;
     unsigned char* d_plan = nullptr;
@@ -341,6 +341,8 @@ extern "C" int ssg_uneven_create(const ssg_uneven_instance* instances, int insta
         maps += P * in.references;
         b->max_references = std::max(b->max_references, in.references);
         b->max_map_pixels = (int)std::max<int64_t>(b->max_map_pixels, P);
+        b->max_map_cols = std::max(b->max_map_cols, in.cols);
+        b->max_map_rows = std::max(b->max_map_rows, in.rows);
         b->max_pano_pixels = (int)std::max<int64_t>(b->max_pano_pixels, (int64_t)in.pano_cols * in.pano_rows);
         b->jobs.push_back(s);
     }
@@ -363,10 +365,8 @@ extern "C" int ssg_uneven_create(const ssg_uneven_instance* instances, int insta
     size_t so = 256;  // the sweep's work counter
     b->maps_offset = so;
     so = align_up(so + sizeof(float) * (size_t)maps, 256);
-    b->stamps_offset = so;
-    so = align_up(so + (size_t)maps, 256);
-    b->holes_offset = so;
-    so = align_up(so + sizeof(int32_t) * (3 * (size_t)maps + SSG_HOLE_SCRATCH_HEADER), 256);
+    b->raw_offset = so;
+    so = align_up(so + sizeof(float) * (size_t)maps, 256);
     b->scratch_bytes = so;
     *plan_bytes = b->plan_bytes;
     *scratch_bytes = b->scratch_bytes;
@@ -380,7 +380,10 @@ extern "C" int ssg_uneven_upload(ssg_uneven_batch* b, void* d_plan, void* d_scra
     SSG_REQUIRE(((uintptr_t)d_plan & 255) == 0 && ((uintptr_t)d_scratch & 255) == 0,
                 "plan and scratch must be 256-byte aligned");
     unsigned char* scratch = static_cast<unsigned char*>(d_scratch);
-    for (StitchJob& j : b->jobs) j.reprojected = reinterpret_cast<float*>(scratch + b->maps_offset) + j.map_begin;
+    for (StitchJob& j : b->jobs) {
+        j.raw = reinterpret_cast<float*>(scratch + b->raw_offset) + j.map_begin;
+        j.reprojected = reinterpret_cast<float*>(scratch + b->maps_offset) + j.map_begin;
+    }
     cudaStream_t st = as_stream(stream);
     for (LevelDesc& d : b->levels) d.lut = range_table(d.var_inv_i, st);  // nullptr: evaluated per block
     std::vector<unsigned char> host(b->plan_bytes, 0);
@@ -414,16 +417,16 @@ extern "C" int ssg_uneven_run(const ssg_uneven_batch* b, void* stream)
     }
     if (b->jobs.empty()) return SSG_OK;
     return launch_stitch_uneven(reinterpret_cast<const StitchJob*>(b->d_plan + b->jobs_offset), (int)b->jobs.size(),
-                                reinterpret_cast<float*>(b->d_scratch + b->maps_offset), b->total_map_pixels,
-                                b->max_map_pixels, b->max_pano_pixels, b->max_references, b->max_dist, b->iterations,
-                                b->d_scratch + b->stamps_offset,
-                                reinterpret_cast<int32_t*>(b->d_scratch + b->holes_offset), st);
+                                reinterpret_cast<float*>(b->d_scratch + b->maps_offset),
+                                reinterpret_cast<float*>(b->d_scratch + b->raw_offset), b->total_map_pixels,
+                                b->max_map_pixels, b->max_map_cols, b->max_map_rows, b->max_pano_pixels,
+                                b->max_references, b->max_dist, b->iterations, st);
 }
 
 extern "C" int ssg_uneven_launches(const ssg_uneven_batch* b)
 {
     if (!b) return 0;
-    const int stitch = b->jobs.empty() ? 0 : 3 + (b->iterations > 0 ? 1 + b->iterations : 0);
+    const int stitch = b->jobs.empty() ? 0 : 3 + fill_passes(b->iterations);  // fill, reprojection, merge
     return 1 + (int)b->steps.size() + stitch;
 }
 

@@ -52,6 +52,7 @@ struct StitchJob {
     int pad1;
     const float* distance;      // references x rows x cols, filtered distance maps
     float* reprojected;         // references x rows x cols, in the concatenated maps
+    float* raw;                 // the same in the maps that the hole filling alternates with
     const uint8_t* tables;      // references x rows x cols x 2 inpainting tables
     const float2* lut;          // references x pano_rows x pano_cols
     const float* weights;       // references x pano_rows x pano_cols
@@ -79,10 +80,11 @@ int launch_down_uneven(const LevelDesc* d_descs, int count, int max_rows_out, in
 // guide = false: the single-candidate step does not form the filtered fine guide
 int launch_up_uneven(const LevelDesc* d_descs, int count, int max_rows_in, int max_cols_in, int width,
                      int storage_fine, bool select, bool guide, cudaStream_t st);
-// fill + reprojection + hole filling + merge of every job: maps concatenated job by job
-// (total_map_pixels), d_stamps one byte per map pixel, d_holes 3 x total_map_pixels + 4 int32
-int launch_stitch_uneven(const StitchJob* d_jobs, int jobs, float* d_maps, int64_t total_map_pixels,
-                         int max_map_pixels, int max_pano_pixels, int max_references, double max_dist,
-                         int iterations, uint8_t* d_stamps, int32_t* d_holes, cudaStream_t st);
+int fill_passes(int iterations);  // launches of a hole filling of `iterations` steps
+// fill + reprojection + hole filling (between d_maps and d_raw, ending in d_maps) + merge of every
+// job: maps concatenated job by job (total_map_pixels each)
+int launch_stitch_uneven(const StitchJob* d_jobs, int jobs, float* d_maps, float* d_raw, int64_t total_map_pixels,
+                         int max_map_pixels, int max_map_cols, int max_map_rows, int max_pano_pixels,
+                         int max_references, double max_dist, int iterations, cudaStream_t st);
 
 }  // namespace ssg

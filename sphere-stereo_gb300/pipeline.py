@@ -12,10 +12,10 @@ One batch of F frames runs the per-frame steps of RGBD_Estimator.estimate_RGBD_p
     ssg_isb_upsample_select_batch  last level + argmin / sub-candidate step             1
     ssg_isb_apply_batch            distance post-filter, fp32, N = 1                    2L - 2
     ssg_reproject_distance_batch_approx  fill + z-buffer                                2
-    ssg_inpaint_holes_batch        hole filling: a scan, steps on hole lists, a tail    6
+    ssg_inpaint_batch              hole filling                                         2
     ssg_merge_panorama_batch_approx panoramas                                           1
 
-so the launch count does not grow with F (about 45 at 1024^2).  Buffers are allocated once for
+so the launch count does not grow with F (about 30 at 1024^2).  Buffers are allocated once for
 the largest batch; outputs alias them, as the reference's outputs alias its stitcher buffers.
 """
 from __future__ import annotations
@@ -92,9 +92,7 @@ class BatchPipeline:
         self.index = torch.empty(F * R * P, dtype=torch.int32, device=dev)
         self.distance = torch.empty(F, R, self.rows, self.cols, **f32)
         self.reprojected = torch.empty(F * R * P, **f32)
-        self.stamps = torch.empty(F * R * P, **u8)
-        self.holes = torch.empty(3 * F * R * P + N.HOLE_SCRATCH_HEADER * self.MAX_GROUPS, dtype=torch.int32,
-                                 device=dev)
+        self.fill_scratch = torch.empty(F * R * P, **f32)  # the hole filling alternates between the two
         self.images_u8 = torch.empty(F, R, st.image_rows, st.image_cols, 3, **u8)
         # the panoramas: output_slots buffers used in turn; rgb / pano_distance are the current one
         self._out_slots = [(torch.empty(F, st.pano_rows, st.pano_cols, 3, **u8),
@@ -237,12 +235,14 @@ class BatchPipeline:
             # float -> uint8 truncation (depth_estimation.py:239)
             N.call("ssg_convert_u8", s_img.data_ptr(), images_u8.data_ptr(),
                    frames * R * st.image_rows * st.image_cols * 3, stream)
-        reprojected = self.reprojected.data_ptr() + 4 * i0 * P
+        reprojected, scratch = (t.data_ptr() + 4 * i0 * P for t in (self.reprojected, self.fill_scratch))
         N.call("ssg_reproject_distance_batch_approx", dist.data_ptr(), reprojected, cols, rows, inst, R, st._intr,
                st._trans, 1, stream)
-        holes = self.holes.data_ptr() + 4 * (3 * i0 * P + N.HOLE_SCRATCH_HEADER * group)
-        N.call("ssg_inpaint_holes_batch", reprojected, self.tables.data_ptr(), self.stamps.data_ptr() + i0 * P, holes,
-               cols, rows, inst, R, st.max_dist, st.inpainting_iterations, stream)
+        if st.inpainting_iterations > N.MAX_FILL_STEPS or inst * P >= 1 << 31:
+            raise ValueError(f"{inst} maps of {cols}x{rows} pixels or {st.inpainting_iterations} inpainting_iterations "
+                             f"are too many (below 2^31 pixels, at most {N.MAX_FILL_STEPS})")
+        N.call("ssg_inpaint_batch", reprojected, self.tables.data_ptr(), scratch, cols, rows, inst, R, st.max_dist,
+               st.inpainting_iterations, stream)
         if images_u8 is None:
             N.call("ssg_merge_panorama_batch_approx_images", st.blending_sampling.data_ptr(),
                    st.blending_weights.data_ptr(), reprojected, dist.data_ptr(),
@@ -383,8 +383,7 @@ class BatchPipeline:
     # in tuning order: a register bound before the staging it pairs with (a staging choice is timed
     # at the bound already picked)
     TUNED_KNOBS = ("sweep_variant", "sweep_tiles", "isb_up_blocks", "up_whole", "isb_select_blocks", "select_whole",
-                   "isb_tile_tma", "isb_tail", "post_tail", "hole_blocks_per_sm", "hole_persistent", "hole_tail",
-                   "merge_frames")
+                   "isb_tile_tma", "isb_tail", "post_tail", "merge_frames")
     GROUP_CHOICES = (1, 2, 4)
 
     def _apply_tuning(self, match, stitch, frames) -> None:
@@ -417,6 +416,6 @@ class BatchPipeline:
         L = self.L
         isb = N.isb_filter_launches(self.rows, self.cols, L) + 1 if L >= 2 else 1
         post = N.isb_apply_launches(self.rows, self.cols, L, 1) if L >= 2 else 0
-        inpaint = N.hole_filling_launches(self.st.inpainting_iterations)
+        inpaint = N.fill_launches(self.st.inpainting_iterations)
         per_group = 2 + isb + post + (1 if float_stitch else 0) + 2 + inpaint + 1
         return per_group * len(self._groups(frames, self._group_count(frames)))

@@ -67,8 +67,10 @@ class Stitcher:
         self.reprojected_distances_list = [self.reprojected_distances[i] for i in range(R)]
         self.distances_list = [self.distances_stacked[i] for i in range(R)]
         self.images_to_stitch_list = [self.images_to_stitch[i] for i in range(R)]
-        self.inpainting_weights_list = [torch.zeros([H, W, 2], dtype=torch.uint8, device=device) for _ in range(R)]
-        self.inpainting_scratch = torch.empty([H, W], device=device)
+        self.inpainting_tables = torch.zeros([R, H, W, 2], dtype=torch.uint8, device=device)
+        self.inpainting_weights_list = [self.inpainting_tables[i] for i in range(R)]
+        # the hole filling alternates between the reprojected maps and this
+        self.inpainting_scratch = torch.empty([R, H, W], device=device)
         self.blending_sampling = torch.zeros([R, Hp, Wp, 2], device=device)
         self.blending_weights = torch.zeros([R, Hp, Wp], device=device)
         self.RGB_panorama = torch.zeros([Hp, Wp, 3], dtype=torch.uint8, device=device)
@@ -133,14 +135,19 @@ class Stitcher:
     def reproject_and_inpaint(self, reference: int, distance_map: torch.Tensor) -> None:
         """Reprojected, hole-filled distance map of one reference (python/stitcher.py:184-200)
         into ``self.reprojected_distances[reference]``."""
-        out = self.reprojected_distances_list[reference]
-        stream = N.stream_of(distance_map)
-        N.call("ssg_reproject_distance", distance_map.data_ptr(), out.data_ptr(), self.cols, self.rows,
-               N.intrinsics_array([self.intrinsics[reference]]),
-               N.floats(self.translations_host[3 * reference:3 * reference + 3].tolist()), 1, stream)
-        N.call("ssg_inpaint", out.data_ptr(), self.inpainting_weights_list[reference].data_ptr(),
-               self.inpainting_scratch.data_ptr(), self.cols, self.rows, self.max_dist, self.inpainting_iterations,
-               stream)
+        self._reproject_and_inpaint(distance_map, reference, 1)
+
+    def _reproject_and_inpaint(self, maps: torch.Tensor, first: int, count: int) -> None:
+        """reproject_and_inpaint of references first .. first + count - 1, whose maps are contiguous."""
+        stream = N.stream_of(maps)
+        reprojected = self.reprojected_distances[first].data_ptr()
+        intrinsics = N.intrinsics_array(self.intrinsics[first:first + count])
+        translations = N.floats(self.translations_host[3 * first:3 * (first + count)].tolist())
+        N.call("ssg_reproject_distance_batch", maps.data_ptr(), reprojected, self.cols, self.rows, count, count,
+               intrinsics, translations, 1, stream)
+        N.call("ssg_inpaint_batch", reprojected, self.inpainting_tables[first].data_ptr(),
+               self.inpainting_scratch[first].data_ptr(), self.cols, self.rows, count, count, self.max_dist,
+               self.inpainting_iterations, stream)
 
     def merge(self) -> None:
         """Blend the stacked maps and images into the panorama (python/stitcher.py:205-218)."""
@@ -166,10 +173,10 @@ class Stitcher:
         for r, (image, distance_map) in enumerate(zip(images, distance_maps)):
             N.require(image, f"images[{r}]", torch.uint8, (self.image_rows, self.image_cols, 3), self.device)
             N.require(distance_map, f"distance_maps[{r}]", torch.float32, (self.rows, self.cols), self.device)
-            self.reproject_and_inpaint(r, distance_map)
             if image.data_ptr() != self.images_to_stitch_list[r].data_ptr():
                 self.images_to_stitch_list[r].copy_(image)
             if distance_map.data_ptr() != self.distances_list[r].data_ptr():
                 self.distances_list[r].copy_(distance_map)
+        self._reproject_and_inpaint(self.distances_stacked, 0, self.reference_count)
         self.merge()
         return self.RGB_panorama, self.distance_panorama

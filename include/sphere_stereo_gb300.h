@@ -166,6 +166,21 @@ SSG_API int ssg_sweep_cost(int cols, int rows, int camera_count, const ssg_camer
                    const float* relative_poses, const float* const* d_images, const int8_t* d_selected,
                    const float* candidates, int candidate_count, float* d_cost, void* stream);
 
+/* The images to match as 16-byte texels (R, G, B, 0), camera after camera, for ssg_sweep_cost_references;
+ * and the guides (ssg_rgb_to_guide) of the listed reference cameras, slot after slot.
+ * d_images: camera_count pointers to pixels x 3 float32; d_packed: camera_count x pixels x 4 float32,
+ * 16-byte aligned; d_guides: reference_count x pixels x 3 (unused where reference_count is 0). */
+SSG_API int ssg_pack_images(const float* const* d_images, int camera_count, int64_t pixels, const int* references,
+                            int reference_count, float* d_packed, uint8_t* d_guides, void* stream);
+
+/* ssg_sweep_cost of several reference cameras from packed images, the same values.  relative_poses:
+ * reference_count x camera_count x 12; d_selected: reference_count x rows x cols; d_cost:
+ * reference_count x candidate_count x rows x cols.  One launch per four references. */
+SSG_API int ssg_sweep_cost_references(int cols, int rows, int camera_count, const ssg_camera* cameras,
+                                      int reference_count, const int* references, const float* relative_poses,
+                                      const float* d_packed, const int8_t* d_selected, const float* candidates,
+                                      int candidate_count, float* d_cost, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * ISB filter
  * ------------------------------------------------------------------------------------------- */
@@ -191,6 +206,28 @@ SSG_API int ssg_isb_level_count(int cols, int rows);
  * levels 1.. are scratch of ceil(rows / 2^l) x ceil(cols / 2^l) (python/isb_filter.py:62-70). */
 SSG_API int ssg_isb_apply(uint8_t* const* d_guides, float* const* d_costs, int level_count, int rows, int cols,
                   int candidate_count, double sigma_i, double sigma_s, void* stream);
+
+/* The filter's steps down to the coarsest level and back up to level 1 for `instances` contiguous planar
+ * volumes (level l: instances x candidate_count x rows_l x cols_l float32, guides instances x rows_l x
+ * cols_l x 3): levels 1 .. level_count - 1 are filtered, level 0 is left as it is.  The filtered
+ * guides of levels 1 .. level_count - 1 go to d_filtered_guides (d_guides itself, or another pyramid;
+ * the coarsest level's is its unfiltered guide), the unfiltered ones to d_guides. */
+SSG_API int ssg_isb_filter(uint8_t* const* d_guides, uint8_t* const* d_filtered_guides, float* const* d_costs,
+                           int level_count, int rows, int cols, int candidate_count, int instances, double sigma_i,
+                           double sigma_s, void* stream);
+
+/* ssg_isb_filter in place and the last step fused with the selection (ssg_isb_upsample_select), for
+ * `instances` volumes; neither level 0 nor its guide is written.  d_index and d_distance_copy may be
+ * NULL. */
+SSG_API int ssg_isb_filter_select(uint8_t* const* d_guides, float* const* d_costs, int level_count, int rows, int cols,
+                                  int candidate_count, int instances, double sigma_i, double sigma_s,
+                                  const float* candidates, float* d_distance, int32_t* d_index, float* d_distance_copy,
+                                  void* stream);
+
+/* ssg_isb_apply of `instances` contiguous one-candidate maps; SSG_ISB_SKIP_FINE_GUIDE leaves the level-0
+ * guides as they are. */
+SSG_API int ssg_isb_apply_maps(uint8_t* const* d_guides, float* const* d_maps, int level_count, int rows, int cols,
+                               int instances, double sigma_i, double sigma_s, int flags, void* stream);
 
 /* Distance selection: python/depth_estimation.py:179-198 (argmin / max over candidates,
  * parabolic sub-candidate step, flat-cost fallback, index -> distance).  d_cost: planar

@@ -107,10 +107,15 @@ SIGNATURES = {
     "ssg_rgb_to_guide": (_I, [_P, _I64, _P, _P]),
     "ssg_select_camera": (_I, [_I, _I, _I, _P, _I, _P, _P, _D, _D, _P, _P]),
     "ssg_sweep_cost": (_I, [_I, _I, _I, _P, _I, _P, _P, _P, _P, _I, _P, _P]),
+    "ssg_pack_images": (_I, [_P, _I, _I64, _P, _I, _P, _P, _P]),
+    "ssg_sweep_cost_references": (_I, [_I, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _P, _P]),
     "ssg_isb_downsample": (_I, [_P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _P]),
     "ssg_isb_upsample": (_I, [_P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _F, _F, _P]),
     "ssg_isb_level_count": (_I, [_I, _I]),
     "ssg_isb_apply": (_I, [_P, _P, _I, _I, _I, _I, _D, _D, _P]),
+    "ssg_isb_filter": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _D, _D, _P]),
+    "ssg_isb_filter_select": (_I, [_P, _P, _I, _I, _I, _I, _I, _D, _D, _P, _P, _P, _P, _P]),
+    "ssg_isb_apply_maps": (_I, [_P, _P, _I, _I, _I, _I, _D, _D, _I, _P]),
     "ssg_select_distance": (_I, [_P, _I, _I64, _P, _P, _P, _P]),
     "ssg_isb_upsample_select": (_I, [_P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _F, _F, _P, _P, _P, _P]),
     "ssg_inpainting_table": (_I, [_I, _I, _P, _P, _D, _D, _P, _P]),
@@ -295,12 +300,29 @@ def isb_filter_launches(rows: int, cols: int, levels: int) -> int:
     return 2 * first if first < levels else (levels - 1) + (levels - 2)
 
 
+def planar_filter_launches(rows: int, cols: int, levels: int, candidates: int, last: int) -> int:
+    """Kernels the filter of a planar volume of several candidates launches up to level ``last``: a
+    step per level, the small levels together (the library's rule: levels of at most 1024 pixels
+    that fit 1536 cells)."""
+    cells, first = 0, levels
+    for s in range(levels - 1, 0, -1) if candidates > 1 else ():
+        n = math.ceil(rows / 2 ** s) * math.ceil(cols / 2 ** s)
+        if n > 1024 or cells + n > 1536:
+            break
+        cells, first = cells + n, s
+    downs = first if first < levels else levels - 1  # the tail counted with them
+    return downs + min(first, levels - 1) - last
+
+
 def isb_apply_launches(rows: int, cols: int, levels: int, candidates: int) -> int:
-    """Kernels ssg_isb_apply_batch launches (the single-candidate filter fuses its small levels,
-    SSG_TUNE_POST_TAIL)."""
-    first = isb_tail_first(rows, cols, levels, library().ssg_tuning_get(TUNE_POST_TAIL)) if candidates == 1 \
-        else levels
-    return 2 * first + 1 if first < levels else 2 * max(0, levels - 1)
+    """Kernels ssg_isb_apply and ssg_isb_apply_batch launch (the single-candidate filter fuses its
+    small levels, SSG_TUNE_POST_TAIL)."""
+    if levels < 2:
+        return 0
+    if candidates > 1:
+        return planar_filter_launches(rows, cols, levels, candidates, 0)
+    first = isb_tail_first(rows, cols, levels, library().ssg_tuning_get(TUNE_POST_TAIL))
+    return 2 * first + 1 if first < levels else 2 * (levels - 1)
 
 
 def kernels_launched(name: str, args) -> int:
@@ -311,11 +333,19 @@ def kernels_launched(name: str, args) -> int:
     if name == "ssg_eval_panoramas":
         return 3
     if name == "ssg_isb_apply":
-        return 2 * max(0, int(args[2]) - 1)
+        return isb_apply_launches(int(args[3]), int(args[4]), int(args[2]), int(args[5]))
+    if name == "ssg_isb_apply_maps":
+        return isb_apply_launches(int(args[3]), int(args[4]), int(args[2]), 1)
+    if name == "ssg_isb_filter":
+        return planar_filter_launches(int(args[4]), int(args[5]), int(args[3]), int(args[6]), 1)
+    if name == "ssg_isb_filter_select":
+        return planar_filter_launches(int(args[3]), int(args[4]), int(args[2]), int(args[5]), 1) + 1
     if name == "ssg_isb_apply_batch":
         return isb_apply_launches(int(args[3]), int(args[4]), int(args[2]), int(args[5]))
     if name == "ssg_isb_filter_batch":
         return isb_filter_launches(int(args[3]), int(args[4]), int(args[2]))
+    if name == "ssg_sweep_cost_references":
+        return -(-int(args[4]) // 4)
     if name == "ssg_reproject_distance":
         return 2 if args[6] else 1
     if name in ("ssg_reproject_distance_batch", "ssg_reproject_distance_batch_approx"):

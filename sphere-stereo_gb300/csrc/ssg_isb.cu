@@ -13,6 +13,7 @@
 // Guides, range weights and cost sums use the reference's arithmetic in its order
 // (ssg_isb_common.cuh), so both layouts give the same bits; the batched path differs from the
 // reference only by the 16-bit rounding of its level-0 volume.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -853,7 +854,8 @@ constexpr int kTailThreads = W == 8 ? 256 : 512;
 // blockIdx.x: instance.  Down steps first -> first + 1 ... levels - 2 -> levels - 1, then up steps
 // levels - 1 -> levels - 2 ... first + 1 -> first (W = 1: one value per pixel, isb_up1_pixel; W = 8:
 // the chunked layout, isb_up8_pixel).  The up steps form the filtered fine guides.
-template <int W>
+// GL: the guides' layout, read through L2 (G4C or G3C)
+template <int W, typename GL>
 __global__ void __launch_bounds__(kTailThreads<W>) isb_tail_kernel(const __grid_constant__ TailParams T,
                                                                    float var_inv_i, const float* __restrict__ table)
 {
@@ -864,25 +866,25 @@ __global__ void __launch_bounds__(kTailThreads<W>) isb_tail_kernel(const __grid_
     for (int s = T.first + 1; s < T.levels; ++s) {
         const LevelGeom g{T.rows[s - 1], T.cols[s - 1], T.rows[s], T.cols[s]};
         const int64_t pin = (int64_t)g.rows_in * g.cols_in, pout = (int64_t)g.rows_out * g.cols_out;
-        const uint8_t* gi = T.guides[s - 1] + inst * pin * 4;
+        const uint8_t* gi = T.guides[s - 1] + inst * pin * GL::bytes;
         const float* ci = T.costs[s - 1] + inst * T.chunks * pin * W;
-        uint8_t* go = T.guides[s] + inst * pout * 4;
+        uint8_t* go = T.guides[s] + inst * pout * GL::bytes;
         float* co = T.costs[s] + inst * T.chunks * pout * W;
         for (int o = threadIdx.x; o < pout; o += blockDim.x)
-            isb_down_pixel<W, float, G4C, true>(gi, ci, go, co, g, T.chunks, o, lut);
+            isb_down_pixel<W, float, GL, true>(gi, ci, go, co, g, T.chunks, o, lut);
         __syncthreads();
     }
     for (int s = T.levels - 2; s >= T.first; --s) {
         const LevelGeom g{T.rows[s + 1], T.cols[s + 1], T.rows[s], T.cols[s]};
         const int64_t pc = (int64_t)g.rows_in * g.cols_in, pf = (int64_t)g.rows_out * g.cols_out;
-        const uint8_t* gi = T.guides[s + 1] + inst * pc * 4;
+        const uint8_t* gi = T.guides[s + 1] + inst * pc * GL::bytes;
         const float* ci = T.costs[s + 1] + inst * T.chunks * pc * W;
-        uint8_t* gio = T.guides[s] + inst * pf * 4;
+        uint8_t* gio = T.guides[s] + inst * pf * GL::bytes;
         float* cio = T.costs[s] + inst * T.chunks * pf * W;
         for (int k = threadIdx.x; k < pc; k += blockDim.x) {
             const int y = k / g.cols_in, x = k - y * g.cols_in;
             if constexpr (W == 1)
-                isb_up1_pixel<G4C, true, true>(gi, ci, gio, cio, g, T.weight_up[s], T.weight_down[s], x, y, lut);
+                isb_up1_pixel<GL, true, true>(gi, ci, gio, cio, g, T.weight_up[s], T.weight_down[s], x, y, lut);
             else
                 isb_up8_pixel(gi, ci, gio, cio, g, T.chunks, T.weight_up[s], T.weight_down[s], x, y, lut);
         }
@@ -1156,7 +1158,7 @@ static int launch_up(const uint8_t* gi, const float* ci, int rc, int cc, uint8_t
                 return launch_status("isb_up1_kernel");
             }
         }
-        return launch_up_planar<kSelect, GL>(gi, ci, rc, cc, gio, cf, rf, cf_cols, ncand, instances, wu, wd,
+        return launch_up_planar<kSelect, GL>(gi, ci, rc, cc, gio, gio, cf, rf, cf_cols, ncand, instances, wu, wd,
                                              var_inv_i, so, st);
     } else {
     CUtensorMap map;
@@ -1216,7 +1218,7 @@ static int tail_first(int rows, int cols, int levels, int max_pixels)
     return levels;
 }
 
-template <int W>
+template <int W, typename GL>
 static int launch_tail(uint8_t* const* guides, float* const* costs, int levels, int first, int rows, int cols,
                        int chunks, int instances, const float* weight_up, const float* weight_down, float var_inv_i,
                        cudaStream_t st)
@@ -1235,11 +1237,55 @@ static int launch_tail(uint8_t* const* guides, float* const* costs, int levels, 
             T.weight_down[s] = weight_down[s];
         }
     }
-    isb_tail_kernel<W><<<instances, kTailThreads<W>, 0, st>>>(T, var_inv_i, range_table(var_inv_i, st));
+    using Coherent = std::conditional_t<std::is_same<GL, G3>::value, G3C, G4C>;
+    isb_tail_kernel<W, Coherent><<<instances, kTailThreads<W>, 0, st>>>(T, var_inv_i, range_table(var_inv_i, st));
     return launch_status("isb_tail_kernel");
 }
 
-// the whole filter on planar levels (W = 1, chunks = candidates): python/isb_filter.py:72-136
+// The cost filter's steps on planar levels of several candidates down to the coarsest level and back
+// up to level `last` (the filtered guides of levels last .. levels - 1 go to `filtered`)
+template <typename GL>
+static int filter_planar(uint8_t* const* guides, uint8_t* const* filtered, float* const* costs, int levels, int rows,
+                         int cols, int ncand, int instances, const Levels& c, int last, cudaStream_t st)
+{
+    PlanarTail T{};
+    T.levels = levels;
+    T.ncand = ncand;
+    for (int s = 0; s < levels; ++s) {
+        T.rows[s] = level_rows(rows, s);
+        T.cols[s] = level_rows(cols, s);
+        T.guides[s] = guides[s];
+        T.filtered[s] = filtered[s];
+        T.costs[s] = costs[s];
+        T.weight_up[s] = c.weight_up[s];
+        T.weight_down[s] = c.weight_down[s];
+    }
+    const int first = T.first = planar_tail_first(T.rows, T.cols, levels, ncand);
+    for (int s = 1; s < levels && s < first; ++s)
+        if (int e = launch_down<1, float, GL>(guides[s - 1], costs[s - 1], T.rows[s - 1], T.cols[s - 1], guides[s],
+                                              costs[s], T.rows[s], T.cols[s], ncand, instances, c.var_inv_i, st))
+            return e;
+    if (first < levels) {
+        isb_planar_tail_kernel<GL><<<dim3(ncand, instances), kPlanarTailThreads, 0, st>>>(
+            T, c.var_inv_i, range_table(c.var_inv_i, st));
+        if (int e = launch_status("isb_planar_tail_kernel")) return e;
+    } else if (filtered[levels - 1] != guides[levels - 1]) {
+        // the coarsest level's guide is not filtered
+        const cudaError_t e = cudaMemcpyAsync(filtered[levels - 1], guides[levels - 1],
+                                              (size_t)GL::bytes * instances * T.rows[levels - 1] * T.cols[levels - 1],
+                                              cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) return fail(SSG_ERR_CUDA, "cudaMemcpyAsync: %s", cudaGetErrorString(e));
+    }
+    for (int s = std::min(first, levels - 1) - 1; s >= last; --s) {
+        if (int e = launch_up_planar<false, GL>(filtered[s + 1], costs[s + 1], T.rows[s + 1], T.cols[s + 1], guides[s], filtered[s],
+                                                costs[s], T.rows[s], T.cols[s], ncand, instances, c.weight_up[s],
+                                                c.weight_down[s], c.var_inv_i, SelectOut{}, st))
+            return e;
+    }
+    return SSG_OK;
+}
+
+// the whole filter on planar levels (python/isb_filter.py:72-136)
 template <typename GL>
 static int apply_planar(uint8_t* const* d_guides, float* const* d_costs, int level_count, int rows, int cols,
                         int candidate_count, int instances, double sigma_i, double sigma_s, cudaStream_t st,
@@ -1250,28 +1296,29 @@ static int apply_planar(uint8_t* const* d_guides, float* const* d_costs, int lev
         if (int e = check_levels(level_rows(rows, s - 1), level_rows(cols, s - 1), level_rows(rows, s),
                                  level_rows(cols, s)))
             return e;
-    // the batched single-candidate filter (the distance post-filter) runs its small levels as one
-    // fused tail (SSG_TUNE_POST_TAIL: the largest first level, in pixels; 0 = none)
-    const int first = std::is_same<GL, G4>::value && candidate_count == 1
-                          ? tail_first(rows, cols, level_count, tuning(SSG_TUNE_POST_TAIL))
-                          : level_count;
+    if (candidate_count > 1)
+        return filter_planar<GL>(d_guides, d_guides, d_costs, level_count, rows, cols, candidate_count, instances, c, 0,
+                                 st);
+    // the single-candidate filter (the distance post-filter) runs its small levels as one fused tail
+    // (SSG_TUNE_POST_TAIL: the largest first level, in pixels; 0 = none)
+    const int first = tail_first(rows, cols, level_count, tuning(SSG_TUNE_POST_TAIL));
     for (int s = 1; s < level_count && s <= first; ++s) {
         const int ri = level_rows(rows, s - 1), ci = level_rows(cols, s - 1), ro = level_rows(rows, s),
                   co = level_rows(cols, s);
         if (int e = launch_down<1, float, GL>(d_guides[s - 1], d_costs[s - 1], ri, ci, d_guides[s], d_costs[s], ro,
-                                              co, candidate_count, instances, c.var_inv_i, st))
+                                              co, 1, instances, c.var_inv_i, st))
             return e;
     }
     if (first < level_count)
-        if (int e = launch_tail<1>(d_guides, d_costs, level_count, first, rows, cols, 1, instances, c.weight_up,
-                                   c.weight_down, c.var_inv_i, st))
+        if (int e = launch_tail<1, GL>(d_guides, d_costs, level_count, first, rows, cols, 1, instances, c.weight_up,
+                                       c.weight_down, c.var_inv_i, st))
             return e;
     for (int s = (first < level_count ? first : level_count - 1) - 1; s >= 0; --s) {
         const int rc = level_rows(rows, s + 1), cc = level_rows(cols, s + 1), rf = level_rows(rows, s),
                   cf = level_rows(cols, s);
         if (int e = launch_up<1, float, false, GL>(d_guides[s + 1], d_costs[s + 1], rc, cc, d_guides[s], d_costs[s],
-                                                   rf, cf, candidate_count, candidate_count, instances,
-                                                   c.weight_up[s], c.weight_down[s], c.var_inv_i, SelectOut{}, st,
+                                                   rf, cf, 1, 1, instances, c.weight_up[s], c.weight_down[s],
+                                                   c.var_inv_i, SelectOut{}, st,
                                                    s > 0 || !(flags & SSG_ISB_SKIP_FINE_GUIDE)))
             return e;
     }
@@ -1336,6 +1383,52 @@ extern "C" int ssg_isb_apply(uint8_t* const* d_guides, float* const* d_costs, in
         return e;
     return apply_planar<G3>(d_guides, d_costs, level_count, rows, cols, candidate_count, 1, sigma_i, sigma_s,
                         as_stream(stream));
+}
+
+extern "C" int ssg_isb_filter(uint8_t* const* d_guides, uint8_t* const* d_filtered_guides, float* const* d_costs,
+                              int level_count, int rows, int cols, int candidate_count, int instances,
+                              double sigma_i, double sigma_s, void* stream)
+{
+    if (int e = check_apply_args(d_guides, d_costs, level_count, rows, cols, candidate_count, sigma_i, sigma_s))
+        return e;
+    SSG_REQUIRE(level_count >= 2, "a pyramid of %d levels has nothing to filter", level_count);
+    SSG_REQUIRE(instances >= 1 && instances <= 65535, "instances out of range");
+    SSG_REQUIRE(d_filtered_guides, "null level array");
+    for (int s = 1; s < level_count; ++s) {
+        SSG_REQUIRE(d_filtered_guides[s], "level %d is NULL", s);
+        if (int e = check_levels(level_rows(rows, s - 1), level_rows(cols, s - 1), level_rows(rows, s),
+                                 level_rows(cols, s)))
+            return e;
+    }
+    return filter_planar<G3>(d_guides, d_filtered_guides, d_costs, level_count, rows, cols, candidate_count, instances,
+                             isb_constants(level_count, sigma_i, sigma_s), 1, as_stream(stream));
+}
+
+extern "C" int ssg_isb_filter_select(uint8_t* const* d_guides, float* const* d_costs, int level_count, int rows,
+                                     int cols, int candidate_count, int instances, double sigma_i, double sigma_s,
+                                     const float* candidates, float* d_distance, int32_t* d_index,
+                                     float* d_distance_copy, void* stream)
+{
+    SSG_REQUIRE(candidates && d_distance, "null pointer");
+    if (int e = ssg_isb_filter(d_guides, d_guides, d_costs, level_count, rows, cols, candidate_count, instances, sigma_i,
+                               sigma_s, stream))
+        return e;
+    const Levels c = isb_constants(level_count, sigma_i, sigma_s);
+    SelectOut so = select_constants(candidates, candidate_count, d_distance, d_index);
+    so.distance2 = d_distance_copy;
+    return launch_up_planar<true, G3>(d_guides[1], d_costs[1], level_rows(rows, 1), level_rows(cols, 1), d_guides[0],
+                                      nullptr, d_costs[0], rows, cols, candidate_count, instances, c.weight_up[0],
+                                      c.weight_down[0], c.var_inv_i, so, as_stream(stream));
+}
+
+extern "C" int ssg_isb_apply_maps(uint8_t* const* d_guides, float* const* d_maps, int level_count, int rows, int cols,
+                                  int instances, double sigma_i, double sigma_s, int flags, void* stream)
+{
+    if (int e = check_apply_args(d_guides, d_maps, level_count, rows, cols, 1, sigma_i, sigma_s)) return e;
+    SSG_REQUIRE(instances >= 1 && instances <= 65535, "instances out of range");
+    SSG_REQUIRE((flags & ~SSG_ISB_SKIP_FINE_GUIDE) == 0, "unknown flags 0x%x", flags);
+    return apply_planar<G3>(d_guides, d_maps, level_count, rows, cols, 1, instances, sigma_i, sigma_s,
+                            as_stream(stream), flags);
 }
 
 extern "C" int ssg_isb_apply_batch(uint8_t* const* d_guides, float* const* d_costs, int level_count, int rows,
@@ -1454,7 +1547,7 @@ extern "C" int ssg_isb_filter_batch(uint8_t* const* d_guides, void* const* d_cos
     if (first < level_count) {
         float* costs[SSG_MAX_LEVELS] = {};
         for (int s = 1; s < level_count; ++s) costs[s] = static_cast<float*>(d_costs[s]);
-        if (int e = launch_tail<8>(d_guides, costs, level_count, first, rows, cols, chunks, instances, weight_up,
+        if (int e = launch_tail<8, G4>(d_guides, costs, level_count, first, rows, cols, chunks, instances, weight_up,
                                    weight_down, var_inv_i, st))
             return e;
     }

@@ -108,6 +108,16 @@ struct G4C : G4 {
     }
 };
 
+struct G3C : G3 {  // the same for three-byte guides
+    __device__ static __forceinline__ Pix load(const uint8_t* g, int64_t idx)
+    {
+        Pix p;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p.c[k] = __ldcg(g + 3 * idx + k);
+        return p;
+    }
+};
+
 struct ExpRange {  // evaluates the weight of a colour distance
     float var_inv_i;
     __device__ __forceinline__ float operator()(int d) const { return range_weight((float)d, var_inv_i); }

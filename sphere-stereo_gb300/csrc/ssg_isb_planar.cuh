@@ -158,9 +158,9 @@ constexpr int kUpDepth = 2;
 
 // Weights of fine pixel F of coarse pixel (x, y) into column `px` of sw, and its filtered guide
 template <int F, int kPx, typename GL>
-__device__ __forceinline__ void planar_fine_setup(const uint8_t* __restrict__ guide_in, uint8_t* __restrict__ guide_io,
-                                                  const LevelGeom& g, int x, int y, bool in_level, float weight_up,
-                                                  float weight_down, const TableRange& range, int px,
+__device__ __forceinline__ void planar_fine_setup(const uint8_t* __restrict__ guide_in, const uint8_t* guide_fine,
+                                                  uint8_t* guide_out, const LevelGeom& g, int x, int y, bool in_level,
+                                                  float weight_up, float weight_down, const TableRange& range, int px,
                                                   float (&sw)[kUpRows][kPx])
 {
     const int fx = 2 * x + (F >= 2 ? 1 : 0), fy = 2 * y + (F & 1);
@@ -169,16 +169,17 @@ __device__ __forceinline__ void planar_fine_setup(const uint8_t* __restrict__ gu
     typename GL::Pix gd[9];
     coarse_neighbourhood<int, GL>(guide_in, g.rows_in, g.cols_in, x, y, ci, gd);  // unused taps are not loaded
     const int index = fy * g.cols_out + fx;
-    const typename GL::Pix up = GL::load(guide_io, index);
+    const typename GL::Pix up = GL::load(guide_fine, index);
     float w[UpTaps<F>::n], gs[3];
     const float inv = fine_weights<F, TableRange, GL>(gd, up, weight_up, weight_down, range, w, gs);
 #pragma unroll
     for (int i = 0; i < UpTaps<F>::n; ++i) sw[up_weight_row<F>() + i][px] = w[i];
     sw[kUpInvRow + F][px] = inv;
+    if (!guide_out) return;
     uint32_t v[3];
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch) v[ch] = __float2uint_rz(fmul(gs[ch], inv));
-    GL::store(guide_io, index, v);
+    GL::store(guide_out, index, v);
 }
 
 // What one range of consecutive candidates contributes to a pixel's selection: a Selector that saw
@@ -280,11 +281,12 @@ __device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in,
 // Up step of a level pair: coarse filtered level -> fine level in place, or (kSelect) the last
 // step fused with the selection, its candidates shared out in consecutive ranges and combined in
 // candidate order.  A block takes 32 coarse pixels; a warp filters one of their two fine rows in
-// one of kRanges ranges of candidates.  blockIdx.x: group of coarse pixels; blockIdx.y: instance.
+// one of kRanges ranges of candidates.  The filtered fine guide goes to guide_out (guide_fine itself,
+// another pyramid's level, or none).  blockIdx.x: group of coarse pixels; blockIdx.y: instance.
 template <int kRanges, bool kSelect, bool kPairs, typename GL>
 __global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges) isb_up_planar_kernel(
-    const uint8_t* __restrict__ guide_in, const float* __restrict__ cost_in, uint8_t* __restrict__ guide_io,
-    float* cost_io, LevelGeom g, int ncand, float weight_up, float weight_down, float var_inv_i,
+    const uint8_t* __restrict__ guide_in, const float* __restrict__ cost_in, const uint8_t* guide_fine,
+    uint8_t* guide_out, float* cost_io, LevelGeom g, int ncand, float weight_up, float weight_down, float var_inv_i,
     const float* __restrict__ table, SelectOut so)
 {
     constexpr int kPx = 32;
@@ -293,7 +295,8 @@ __global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges)
     const int pin = g.rows_in * g.cols_in, pio = g.rows_out * g.cols_out;  // below 2^31 (check_levels)
     const int64_t inst = blockIdx.y;
     guide_in += inst * pin * GL::bytes;
-    guide_io += inst * pio * GL::bytes;
+    guide_fine += inst * pio * GL::bytes;
+    if (guide_out) guide_out += inst * pio * GL::bytes;
     cost_in += inst * ncand * pin;
     cost_io += inst * ncand * pio;
     const int px = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -304,10 +307,17 @@ __global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges)
     const TableRange rw{table, var_inv_i};
     for (int f = warp; f < 4; f += 2 * kRanges) {
         switch (f) {
-        case 0: planar_fine_setup<0, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
-        case 1: planar_fine_setup<1, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
-        case 2: planar_fine_setup<2, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
-        default: planar_fine_setup<3, kPx, GL>(guide_in, guide_io, g, x, y, in, weight_up, weight_down, rw, px, sw); break;
+        case 0:
+            planar_fine_setup<0, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
+            break;
+        case 1:
+            planar_fine_setup<1, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
+            break;
+        case 2:
+            planar_fine_setup<2, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
+            break;
+        default:
+            planar_fine_setup<3, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
         }
     }
     __syncthreads();
@@ -353,6 +363,188 @@ __global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges)
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The small levels of the pyramid in one launch: one block per (candidate, instance) takes the down
+// step into level `first`, every level below it and the up steps back to level `first`, in shared
+// memory.  Every block forms the guides and weights for itself (they are few), the first candidate's
+// writes the guides; no other block reads what it writes.  The steps are those of the kernels
+// above, value by value (same bits).  A launch per step takes 5 to 8 us on such a level; the
+// pyramid of 1024^2 x 32 took seven of them, 48 us, and takes 12.5 us here.
+// ---------------------------------------------------------------------------------------------
+constexpr int kPlanarTailPixels = 1024;  // of level `first`
+constexpr int kPlanarTailCells = 1536;   // of level `first` and below: the next level of an r x c level
+                                         // with r, c >= 8 holds at most 81 / 256 of its pixels
+constexpr int kPlanarTailThreads = 512;
+
+struct PlanarTail {
+    int levels, first, ncand;
+    int rows[SSG_MAX_LEVELS], cols[SSG_MAX_LEVELS];
+    uint8_t* guides[SSG_MAX_LEVELS];    // unfiltered; level first - 1 is read
+    uint8_t* filtered[SSG_MAX_LEVELS];  // filtered (the same arrays, or others)
+    float* costs[SSG_MAX_LEVELS];
+    float weight_up[SSG_MAX_LEVELS], weight_down[SSG_MAX_LEVELS];
+};
+
+// one coarse pixel of a down step, from global (GL) or shared (G4) memory
+template <typename GL>
+__device__ __forceinline__ void tail_down(const uint8_t* guide_in, const float* cost_in, int rows_in, int cols_in, int x,
+                                          int y, const float* lut, uint32_t& guide, float& cost)
+{
+    const int x2 = 2 * x, y2 = 2 * y;
+    const int xp = min(x2 + 1, cols_in - 1), yp = min(y2 + 1, rows_in - 1), xm = max(x2 - 1, 0), ym = max(y2 - 1, 0);
+    const int idx[8] = {ym * cols_in + xm, y2 * cols_in + xm, yp * cols_in + xm, yp * cols_in + x2,
+                        yp * cols_in + xp, y2 * cols_in + xp, ym * cols_in + xp, ym * cols_in + x2};
+    const int centre = y2 * cols_in + x2;
+    const typename GL::Pix cur = GL::load(guide_in, centre);
+    float gs[3] = {(float)GL::ch(cur, 0), (float)GL::ch(cur, 1), (float)GL::ch(cur, 2)};
+    float wsum = 1.0f, acc = cost_in[centre];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const typename GL::Pix nb = GL::load(guide_in, idx[i]);
+        const float w = fmul(i % 2 ? 0.5f : 0.25f, lut[GL::dist(cur, nb)]);
+        wsum = fadd(wsum, w);
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) gs[ch] = fadd(gs[ch], fmul((float)GL::ch(nb, ch), w));
+        acc = fadd(acc, fmul(cost_in[idx[i]], w));
+    }
+    const float den = fdiv(1.0f, wsum);
+    guide = 0;
+#pragma unroll
+    for (int ch = 0; ch < 3; ++ch) guide |= __float2uint_rz(fmul(gs[ch], den)) << (8 * ch);
+    cost = fdiv(acc, wsum);
+}
+
+// fine pixel F of coarse pixel (x, y) of an up step in shared memory
+template <int F>
+__device__ __forceinline__ void tail_up(const uint32_t* guide_in, const float* cost_in, uint32_t* guide_io, float* cost_io,
+                                        const LevelGeom& g, int x, int y, float weight_up, float weight_down,
+                                        const LutRange& range)
+{
+    const int fx = 2 * x + (F >= 2 ? 1 : 0), fy = 2 * y + (F & 1);
+    if (fx >= g.cols_out || fy >= g.rows_out) return;
+    const int rr[3] = {max(y - 1, 0) * g.cols_in, y * g.cols_in, min(y + 1, g.rows_in - 1) * g.cols_in};
+    const int cc[3] = {max(x - 1, 0), x, min(x + 1, g.cols_in - 1)};
+    const int index = fy * g.cols_out + fx;
+    G4::Pix gd[9];
+    float cd[9];
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+        if (uses_tap<F>(t)) {
+            gd[t] = guide_in[rr[t / 3] + cc[t % 3]];
+            cd[t] = cost_in[rr[t / 3] + cc[t % 3]];
+        }
+    float w[UpTaps<F>::n], gs[3];
+    const float inv = fine_weights<F, LutRange, G4>(gd, guide_io[index], weight_up, weight_down, range, w, gs);
+    float s = fmul(weight_up, cost_io[index]);
+#pragma unroll
+    for (int i = 0; i < UpTaps<F>::n; ++i) s = fadd(s, fmul(w[i], cd[UpTaps<F>::tap(i)]));
+    cost_io[index] = fmul(s, inv);
+    uint32_t v = 0;
+#pragma unroll
+    for (int ch = 0; ch < 3; ++ch) v |= __float2uint_rz(fmul(gs[ch], inv)) << (8 * ch);
+    guide_io[index] = v;
+}
+
+template <typename GL>
+__device__ __forceinline__ void tail_store_guides(const PlanarTail& T, uint8_t* const* to, int64_t inst,
+                                                  const uint32_t* guides)
+{
+    int at = 0;
+    for (int s = T.first; s < T.levels; ++s) {
+        const int n = T.rows[s] * T.cols[s];
+        for (int i = threadIdx.x; i < n; i += kPlanarTailThreads) {
+            const uint32_t q = guides[at + i], v[3] = {q & 255u, (q >> 8) & 255u, (q >> 16) & 255u};
+            GL::store(to[s] + inst * n * GL::bytes, i, v);
+        }
+        at += n;
+    }
+}
+
+// blockIdx.x: candidate; blockIdx.y: instance
+template <typename GL>
+__global__ void __launch_bounds__(kPlanarTailThreads) isb_planar_tail_kernel(const __grid_constant__ PlanarTail T,
+                                                                             float var_inv_i,
+                                                                             const float* __restrict__ table)
+{
+    __shared__ __align__(16) float lut[kRangeLutStride];
+    __shared__ uint32_t guides[kPlanarTailCells];
+    __shared__ float costs[kPlanarTailCells];
+    load_range_lut(lut, table, var_inv_i);
+    __syncthreads();
+    const int64_t inst = blockIdx.y;
+    const int cand = blockIdx.x;
+    int begin[2] = {0, 0};  // of the finer and the coarser level of a step
+    for (int s = T.first; s < T.levels; ++s) {
+        const int n = T.rows[s] * T.cols[s];
+        const int rows_in = T.rows[s - 1], cols_in = T.cols[s - 1], nin = rows_in * cols_in;
+        for (int i = threadIdx.x; i < n; i += kPlanarTailThreads) {
+            const int y = i / T.cols[s], x = i - y * T.cols[s];
+            uint32_t g;
+            float c;
+            if (s == T.first)
+                tail_down<GL>(T.guides[s - 1] + inst * nin * GL::bytes, T.costs[s - 1] + (inst * T.ncand + cand) * nin,
+                              rows_in, cols_in, x, y, lut, g, c);
+            else
+                tail_down<G4>(reinterpret_cast<const uint8_t*>(guides + begin[0]), costs + begin[0], rows_in, cols_in, x, y,
+                              lut, g, c);
+            guides[begin[1] + i] = g;
+            costs[begin[1] + i] = c;
+        }
+        begin[0] = begin[1];
+        begin[1] += n;
+        __syncthreads();
+    }
+    const bool writes_guides = cand == 0;
+    if (writes_guides && T.filtered[T.first] != T.guides[T.first]) {
+        tail_store_guides<GL>(T, T.guides, inst, guides);
+        __syncthreads();
+    }
+    const LutRange range{lut};
+    for (int s = T.levels - 2; s >= T.first; --s) {
+        const LevelGeom g{T.rows[s + 1], T.cols[s + 1], T.rows[s], T.cols[s]};
+        const int coarse = begin[0], fine = coarse - g.rows_out * g.cols_out, n = g.rows_in * g.cols_in;
+        // a warp takes one of the four fine pixels of 32 coarse ones
+        for (int k = threadIdx.x; k < 4 * ((n + 31) & ~31); k += kPlanarTailThreads) {
+            const int i = (k >> 7) * 32 + (k & 31);
+            if (i >= n) continue;
+            const int y = i / g.cols_in, x = i - y * g.cols_in;
+            const uint32_t* gi = guides + coarse;
+            const float* ci = costs + coarse;
+            switch ((k >> 5) & 3) {
+            case 0: tail_up<0>(gi, ci, guides + fine, costs + fine, g, x, y, T.weight_up[s], T.weight_down[s], range); break;
+            case 1: tail_up<1>(gi, ci, guides + fine, costs + fine, g, x, y, T.weight_up[s], T.weight_down[s], range); break;
+            case 2: tail_up<2>(gi, ci, guides + fine, costs + fine, g, x, y, T.weight_up[s], T.weight_down[s], range); break;
+            default: tail_up<3>(gi, ci, guides + fine, costs + fine, g, x, y, T.weight_up[s], T.weight_down[s], range);
+            }
+        }
+        begin[0] = fine;
+        __syncthreads();
+    }
+    int at = 0;
+    for (int s = T.first; s < T.levels; ++s) {
+        const int n = T.rows[s] * T.cols[s];
+        float* out = T.costs[s] + (inst * T.ncand + cand) * n;
+        for (int i = threadIdx.x; i < n; i += kPlanarTailThreads) out[i] = costs[at + i];
+        at += n;
+    }
+    if (writes_guides) tail_store_guides<GL>(T, T.filtered, inst, guides);
+}
+
+// The first level of a pyramid's tail: the first level s >= 1 of at most kPlanarTailPixels pixels that
+// with the levels below it fits the block; `levels` when no level does, or for one candidate.
+static int planar_tail_first(const int* rows, const int* cols, int levels, int ncand)
+{
+    if (ncand < 2) return levels;
+    int cells = 0, first = levels;
+    for (int s = levels - 1; s >= 1; --s) {
+        const int64_t n = (int64_t)rows[s] * cols[s];
+        if (n > kPlanarTailPixels || cells + n > kPlanarTailCells) break;
+        cells += (int)n;
+        first = s;
+    }
+    return first;
+}
+
 // Into how many ranges a step's candidates are shared out: a power of two of at most `ncand`.  Every
 // range more repeats the set-up of the pixel's weights, which costs about as much as 10
 // candidates, and a level too small to fill the GPU needs the ranges to keep enough loads in
@@ -396,8 +588,8 @@ static int launch_down_planar(const uint8_t* gi, const float* ci, int ri, int cl
 }
 
 template <bool kSelect, typename GL>
-static int launch_up_planar(const uint8_t* gi, const float* ci, int rc, int cc, uint8_t* gio, float* cf, int rf,
-                            int cf_cols, int ncand, int instances, float wu, float wd, float var_inv_i,
+static int launch_up_planar(const uint8_t* gi, const float* ci, int rc, int cc, const uint8_t* gf, uint8_t* go,
+                            float* cf, int rf, int cf_cols, int ncand, int instances, float wu, float wd, float var_inv_i,
                             const SelectOut& so, cudaStream_t st)
 {
     const LevelGeom g{rc, cc, rf, cf_cols};
@@ -407,7 +599,7 @@ static int launch_up_planar(const uint8_t* gi, const float* ci, int rc, int cc, 
     const int ranges = up_ranges(pin * instances, ncand);
     const dim3 grid(grid_1d(pin, 32), instances);
 #define SSG_UP_PLANAR(R, P) \
-    isb_up_planar_kernel<R, kSelect, P, GL><<<grid, 64 * R, 0, st>>>(gi, ci, gio, cf, g, ncand, wu, wd, var_inv_i, \
+    isb_up_planar_kernel<R, kSelect, P, GL><<<grid, 64 * R, 0, st>>>(gi, ci, gf, go, cf, g, ncand, wu, wd, var_inv_i, \
                                                                            table, so)
     if (ranges == 8) {
         if (pairs) SSG_UP_PLANAR(8, true);

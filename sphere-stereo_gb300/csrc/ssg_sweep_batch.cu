@@ -1142,8 +1142,10 @@ template <bool kAligned>
 __global__ void __launch_bounds__(kBatchBlock) convert_u8_kernel(const float* __restrict__ src,
                                                                  uint8_t* __restrict__ dst, int64_t n)
 {
-    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 16;
-    if (kAligned && i + 16 <= n) {
+    // a block converts 16 x kBatchBlock consecutive values
+    const int64_t base = (int64_t)blockIdx.x * (16 * kBatchBlock);
+    if (kAligned && base + 16 * kBatchBlock <= n) {
+        const int64_t i = base + 16 * threadIdx.x;
         uint32_t w[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1153,7 +1155,12 @@ __global__ void __launch_bounds__(kBatchBlock) convert_u8_kernel(const float* __
         }
         reinterpret_cast<uint4*>(dst + i)[0] = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
-        for (int64_t k = i; k < n; ++k) dst[k] = (uint8_t)__float2uint_rz(src[k]);
+        // misaligned arrays and the last block: consecutive values by consecutive threads
+#pragma unroll 4
+        for (int q = 0; q < 16; ++q) {
+            const int64_t k = base + q * kBatchBlock + threadIdx.x;
+            if (k < n) dst[k] = (uint8_t)__float2uint_rz(src[k]);
+        }
     }
 }
 

@@ -2,18 +2,17 @@
 (python/depth_estimation.py:38-243), same constructor, methods and return conventions.
 
 Per reference camera and frame the reference runs ~20 torch operations per camera over
-[N, H, W, 3] volumes, the ISB filter, ~15 torch reductions and a second filter.  Here that is:
+[N, H, W, 3] volumes, the ISB filter, ~15 torch reductions and a second filter.  Here that is, for
+all reference cameras of a frame together:
 
-    rgb_to_guide            guide = rgb2yCbCr(image).uint8                      (1 launch)
-    ssg_sweep_cost          fused sweep + L1 cost, [N, H, W] float32            (1 launch)
-    ssg_isb_downsample      L - 1 levels                                         (L - 1 launches)
-    ssg_isb_upsample        levels L - 2 .. 1                                    (L - 2 launches)
-    ssg_isb_upsample_select last level fused with argmin / sub-candidate step    (1 launch)
-    ssg_isb_apply           distance post-filter (N = 1, sigma / 2)             (2L - 2 launches)
+    ssg_pack_images            16-byte texels, guides = rgb2yCbCr(image).uint8        (1 launch)
+    ssg_sweep_cost_references  fused sweep + L1 cost, [N, H, W] float32               (1 launch per 4 references)
+    ssg_isb_filter_select      the cost filter, its small levels in one launch, the last step
+                               fused with argmin / sub-candidate step
+    ssg_isb_apply_maps         distance post-filter (N = 1, sigma / 2)
 
-followed by the stitcher (reproject + inpaint per reference, one merge).  Every launch goes on
-the caller's current CUDA stream; nothing synchronises the host, so a whole frame can be
-captured in a CUDA graph.
+followed by the stitcher (reproject, inpaint, merge).  Every launch goes on the caller's current
+CUDA stream; nothing synchronises the host, so a whole frame can be captured in a CUDA graph.
 
 Inputs are validated before any launch (shapes, dtypes, devices, contiguity, candidate and
 camera limits); the reference performs no such checks.
@@ -23,15 +22,39 @@ from __future__ import annotations
 import torch
 
 from . import _native as N
-from .isb_filter import ISB_Filter, level_shapes, level_weights
+from .isb_filter import ISB_Filter, level_shapes
 from .stitcher import Stitcher
-from .utils import _cpu32, camera_struct, relative_poses, rgb_to_guide
+from .utils import camera_struct, relative_poses
 
 
 def distance_candidates(min_dist, max_dist, candidate_count) -> torch.Tensor:
     """1 / linspace(1 / min_dist, 1 / max_dist, N) in float32 on the CPU
     (python/depth_estimation.py:145-146)."""
     return 1 / torch.linspace(1 / min_dist, 1 / max_dist, candidate_count)
+
+
+class _Fp32Buffers:
+    """What the fp32 path works on: packed images, and per reference of a group the guides, the cost
+    pyramid (candidate_count float32 planes per level) and the post-filter's pyramid."""
+
+    # References are worked on together as long as their pyramids fit these bytes (the launches of one
+    # reference do not fill the GPU at small sizes; at large ones nothing is gained)
+    GROUP_BYTES = 2 << 30
+
+    def __init__(self, cameras: int, references: int, candidates: int, shapes, device):
+        rows, cols = shapes[0]
+        u8, f32 = dict(dtype=torch.uint8, device=device), dict(dtype=torch.float32, device=device)
+        per_reference = sum(4 * candidates * r * c for r, c in shapes)
+        self.group = max(1, min(references, 4, self.GROUP_BYTES // per_reference))
+        G = self.group
+        self.packed = torch.empty(cameras, rows, cols, 4, **f32)
+        self.guides = [torch.zeros(G, r, c, 3, **u8) for r, c in shapes]
+        self.costs = [torch.zeros(G, candidates, r, c, **f32) for r, c in shapes]
+        self.df_guides = [torch.empty(G, r, c, 3, **u8) for r, c in shapes[1:]]
+        self.df_costs = [torch.empty(G, r, c, **f32) for r, c in shapes[1:]]
+        self.guide_levels = N.pointers([g.data_ptr() for g in self.guides])
+        self.cost_levels = N.pointers([c.data_ptr() for c in self.costs])
+        self.df_guide_levels = N.pointers([g.data_ptr() for g in [self.guides[0], *self.df_guides]])
 
 
 class RGBD_Estimator:
@@ -93,8 +116,8 @@ class RGBD_Estimator:
 
         if cost_storage not in ("fp32", "fp16", "unorm16"):
             raise ValueError("cost_storage must be 'fp32', 'fp16' or 'unorm16'")
-        # the fp32 path's filters (pyramids of candidate_count float32 planes) are allocated on
-        # first use: the 16-bit paths have their own buffers
+        # the fp32 path's buffers are allocated on first use: the 16-bit paths have their own
+        self._fp32 = None
         self._cost_filter = None
         self._distance_filter = None
         calibrations_for_stitch = [calibrations[r] for r in self.references_indices]
@@ -106,11 +129,9 @@ class RGBD_Estimator:
         self.distance_candidates_host = distance_candidates(min_dist, max_dist, candidate_count)
         self._candidates = N.floats(self.distance_candidates_host.tolist())
         self._cams = N.cameras_array([camera_struct(c) for c in calibrations])
-        self._poses_list = {r: relative_poses(calibrations, r) for r in self.references_indices}
-        self._poses = {r: N.floats(v) for r, v in self._poses_list.items()}
+        self._set_poses({r: relative_poses(calibrations, r) for r in self.references_indices})
         cols, rows = self.matching_resolution
         self._shapes = level_shapes(self.matching_resolution)
-        self._guide = torch.empty([rows, cols, 3], dtype=torch.uint8, device=device)
         # per reference: the distance map before the post-filter (depth_estimation.py:196-198)
         self.distance_raw_maps = torch.empty([len(self.references_indices), rows, cols], device=device)
         # per reference: the selected candidate index (torch.min's index, depth_estimation.py:180)
@@ -124,11 +145,32 @@ class RGBD_Estimator:
         self.output_slots = int(output_slots)
         self._pipeline = None
 
+    def _set_poses(self, poses: dict) -> None:
+        """The sweep's relative poses: per reference, camera_count x 12 floats."""
+        self._poses_list = poses
+        self._poses = {r: N.floats(v) for r, v in poses.items()}
+
+    def _set_selected(self, selected: list) -> None:
+        """The camera selection of every reference, [rows, cols] int8 each."""
+        self._selected_maps = torch.stack(selected)
+        self._selected = list(self._selected_maps)
+        self.selected_cameras = [t.long().unsqueeze(0) for t in self._selected]
+
+    def _fp32_buffers(self) -> _Fp32Buffers:
+        if self._fp32 is None:
+            self._fp32 = _Fp32Buffers(len(self.calibrations), len(self.references_indices), self.candidate_count,
+                                      self._shapes, self.device)
+        return self._fp32
+
     @property
     def cost_filter(self) -> ISB_Filter:
-        """The fp32 path's cost filter (python/depth_estimation.py:67)."""
+        """The fp32 path's cost filter (python/depth_estimation.py:67), over the buffers of the last
+        reference worked on."""
         if self._cost_filter is None:
-            self._cost_filter = ISB_Filter(self.candidate_count, self.matching_resolution, self.device)
+            b = self._fp32_buffers()
+            last = (len(self.references_indices) - 1) % b.group
+            self._cost_filter = ISB_Filter.over(self.candidate_count, self.matching_resolution,
+                                                [g[last] for g in b.guides], [c[last] for c in b.costs])
         return self._cost_filter
 
     @property
@@ -161,17 +203,17 @@ class RGBD_Estimator:
                 if t.min() < -1 or t.max() >= len(self.calibrations):
                     raise ValueError("camera indices out of range")
                 sel8.append(t.to(torch.int8).contiguous())
-            self._selected = sel8
-            self.selected_cameras = [t.long().unsqueeze(0) for t in sel8]
+            self._set_selected(sel8)
         if relative_poses is not None:
             if len(relative_poses) != len(self.references_indices):
                 raise ValueError("one pose table per reference is required")
+            poses = dict(self._poses_list)
             for r, v in zip(self.references_indices, relative_poses):
                 v = [float(x) for x in torch.as_tensor(v).reshape(-1).tolist()]
                 if len(v) != 12 * len(self.calibrations):
                     raise ValueError("each pose table needs camera_count x 12 floats")
-                self._poses_list[r] = v
-                self._poses[r] = N.floats(v)
+                poses[r] = v
+            self._set_poses(poses)
         self._pipeline = None
 
     def pipeline(self):
@@ -208,8 +250,7 @@ class RGBD_Estimator:
                 new.append(t.to(c.rt.device) if isinstance(c.rt, torch.Tensor) else t)
             for c, t in zip(self.calibrations, new):
                 c.rt = t
-            self._poses_list = {r: relative_poses(self.calibrations, r) for r in self.references_indices}
-            self._poses = {r: N.floats(v) for r, v in self._poses_list.items()}
+            self._set_poses({r: relative_poses(self.calibrations, r) for r in self.references_indices})
             self.select_camera(self._masks)
         if reprojection_viewpoint is not None:
             self.reprojection_viewpoint = reprojection_viewpoint
@@ -226,64 +267,56 @@ class RGBD_Estimator:
         mask_stack = torch.stack([torch.as_tensor(m, dtype=torch.float32).reshape(rows, cols) for m in masks])
         mask_stack = mask_stack.to(self.device).contiguous()
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        self._selected = []
-        self.selected_cameras = []
+        selected = []
         for r in self.references_indices:
             sel = torch.empty([rows, cols], dtype=torch.int8, device=self.device)
             N.call("ssg_select_camera", cols, rows, len(self.calibrations), self._cams, r, self._poses[r],
                    mask_stack.data_ptr(), float(self.min_dist), float(self.max_dist), sel.data_ptr(), stream)
-            self._selected.append(sel)
-            self.selected_cameras.append(sel.long().unsqueeze(0))
+            selected.append(sel)
+        self._set_selected(selected)
 
     # --------------------------------------------------------------------------------------
     def _validate_images(self, images, shape, name):
         for i, im in enumerate(images):
             N.require(im, f"{name}[{i}]", torch.float32, shape, self.device)
 
-    def _distance(self, slot: int, reference: int, guide: torch.Tensor, images, out: torch.Tensor) -> torch.Tensor:
-        """Filtered distance map of one reference camera into ``out`` ([rows, cols] float32)
-        (python/depth_estimation.py:137-203)."""
+    def _distances(self, first: int, count: int, images, guides, out: torch.Tensor) -> None:
+        """Filtered distance maps of reference slots first .. first + count - 1 into ``out``
+        ([count, rows, cols] float32, contiguous) (python/depth_estimation.py:137-203).  guides: [count,
+        rows, cols, 3] uint8, or None for the images' own."""
+        b = self._fp32_buffers()
         cols, rows = self.matching_resolution
-        n = self.candidate_count
-        stream = N.stream_of(guide)
-        cf = self.cost_filter
-        cost = cf.costs[0]
-        guides = cf.guides
-        costs = [cost] + cf.costs[1:]
-        N.call("ssg_sweep_cost", cols, rows, len(self.calibrations), self._cams, reference, self._poses[reference],
-               N.pointers([im.data_ptr() for im in images]), self._selected[slot].data_ptr(), self._candidates, n,
-               cost.data_ptr(), stream)
-        # cost filter on a copy of the guide (python/depth_estimation.py:177)
-        guides[0].copy_(guide)
-        L = len(self._shapes)
-        var_inv_i = 1 / (2 * self.sigma_i * self.sigma_i)
-        raw = self.distance_raw_maps[slot]
-        if L >= 2:
-            weights = level_weights(L, self.sigma_s)
-            for s in range(1, L):
-                (ri, ci), (ro, co) = self._shapes[s - 1], self._shapes[s]
-                N.call("ssg_isb_downsample", guides[s - 1].data_ptr(), costs[s - 1].data_ptr(), ri, ci,
-                       guides[s].data_ptr(), costs[s].data_ptr(), ro, co, n, var_inv_i, stream)
-            for s in range(L - 2, 0, -1):
-                (rc, cc), (rf, cfn) = self._shapes[s + 1], self._shapes[s]
-                wu, wd = weights[s]
-                N.call("ssg_isb_upsample", guides[s + 1].data_ptr(), costs[s + 1].data_ptr(), rc, cc,
-                       guides[s].data_ptr(), costs[s].data_ptr(), rf, cfn, n, wu, wd, var_inv_i, stream)
-            (rc, cc) = self._shapes[1]
-            wu, wd = weights[0]
-            N.call("ssg_isb_upsample_select", guides[1].data_ptr(), costs[1].data_ptr(), rc, cc,
-                   guides[0].data_ptr(), cost.data_ptr(), rows, cols, n, wu, wd, var_inv_i, self._candidates,
-                   raw.data_ptr(), self.index_maps[slot].data_ptr(), stream)
-        else:
-            N.call("ssg_select_distance", cost.data_ptr(), n, rows * cols, self._candidates, raw.data_ptr(),
-                   self.index_maps[slot].data_ptr(), stream)
-        # distance post-filter with higher edge preservation (python/depth_estimation.py:200-203)
-        df = self.distance_filter
-        df.guides[0].copy_(guide)
-        out3 = out.view(1, rows, cols)
-        out3.copy_(raw.view(1, rows, cols))
-        df.apply(df.guides[0], out3, self.sigma_i / 2, self.sigma_s / 2)
-        return out
+        n, C, L = self.candidate_count, len(self.calibrations), len(self._shapes)
+        stream = N.stream_of(out)
+        pointers = N.pointers([im.data_ptr() for im in images])
+        for g0 in range(0, count, b.group):
+            group = min(b.group, count - g0)
+            refs = self.references_indices[first + g0:first + g0 + group]
+            refs_c = N.ints(refs)
+            poses = self._poses[refs[0]] if group == 1 else N.floats([v for r in refs for v in self._poses_list[r]])
+            # the images stay packed for the later groups; the guides are each group's own
+            N.call("ssg_pack_images", pointers, C, rows * cols, refs_c, group if guides is None else 0,
+                   b.packed.data_ptr(), b.guides[0].data_ptr(), stream)
+            if guides is not None:
+                b.guides[0][:group].copy_(guides[g0:g0 + group])
+            N.call("ssg_sweep_cost_references", cols, rows, C, self._cams, group, refs_c, poses, b.packed.data_ptr(),
+                   self._selected_maps[first + g0].data_ptr(), self._candidates, n, b.costs[0].data_ptr(), stream)
+            raw, index = self.distance_raw_maps[first + g0], self.index_maps[first + g0]
+            maps = out[g0:g0 + group]
+            if L < 2:
+                for i in range(group):
+                    N.call("ssg_select_distance", b.costs[0][i].data_ptr(), n, rows * cols, self._candidates,
+                           self.distance_raw_maps[first + g0 + i].data_ptr(),
+                           self.index_maps[first + g0 + i].data_ptr(), stream)
+                maps.copy_(self.distance_raw_maps[first + g0:first + g0 + group])
+                continue
+            # the selection writes the raw distance and, for the post-filter to filter in place, a copy
+            N.call("ssg_isb_filter_select", b.guide_levels, b.cost_levels, L, rows, cols, n, group, float(self.sigma_i),
+                   float(self.sigma_s), self._candidates, raw.data_ptr(), index.data_ptr(), maps.data_ptr(), stream)
+            # distance post-filter with higher edge preservation (python/depth_estimation.py:200-203)
+            N.call("ssg_isb_apply_maps", b.df_guide_levels,
+                   N.pointers([maps.data_ptr(), *(c.data_ptr() for c in b.df_costs)]), L, rows, cols, group,
+                   float(self.sigma_i) / 2, float(self.sigma_s) / 2, N.ISB_SKIP_FINE_GUIDE, stream)
 
     def estimate_fisheye_distance(self, reference_image, guide, reference_calibration, selected_camera, images):
         """Distance map of one reference fisheye image (python/depth_estimation.py:137-203).
@@ -298,8 +331,9 @@ class RGBD_Estimator:
         cols, rows = self.matching_resolution
         self._validate_images(hwc, (rows, cols, 3), "images")
         N.require(guide, "guide", torch.uint8, (rows, cols, 3), self.device)
-        out = torch.empty([rows, cols], device=self.device)
-        return self._distance(slot, reference, guide, hwc, out)
+        out = torch.empty([1, rows, cols], device=self.device)
+        self._distances(slot, 1, hwc, guide.unsqueeze(0), out)
+        return out[0]
 
     def estimate_RGBD_panorama(self, images_to_match, images_to_stitch):
         """Distance on every reference fisheye image, then a disparity-aware stitch.
@@ -325,11 +359,10 @@ class RGBD_Estimator:
             raise ValueError(f"expected {len(self.references_indices)} images to stitch")
         self._validate_images(images_to_match, (rows, cols, 3), "images_to_match")
         self._validate_images(images_to_stitch, (st.image_rows, st.image_cols, 3), "images_to_stitch")
-        for slot, reference in enumerate(self.references_indices):
-            rgb_to_guide(images_to_match[reference], self._guide)
-            self._distance(slot, reference, self._guide, images_to_match, st.distances_list[slot])
-        for slot, image in enumerate(images_to_stitch):
-            st.images_to_stitch_list[slot].copy_(image)  # float -> uint8 truncation (depth_estimation.py:239-240)
+        self._distances(0, len(self.references_indices), images_to_match, None, st.distances_stacked)
+        for image, target in zip(images_to_stitch, st.images_to_stitch_list):
+            # float -> uint8 truncation (depth_estimation.py:239-240)
+            N.call("ssg_convert_u8", image.data_ptr(), target.data_ptr(), image.numel(), N.stream_of(image))
         return st.stitch(st.images_to_stitch_list, st.distances_list)
 
     def estimate_RGBD_panoramas(self, images_to_match, images_to_stitch=None):

@@ -50,6 +50,15 @@ class ISB_Filter:
         self.costs = [torch.zeros([candidate_count, r, c], device=device) for r, c in shapes]
         N.library()
 
+    @classmethod
+    def over(cls, candidate_count, resolution, guides, costs) -> "ISB_Filter":
+        """A filter whose intermediate scales are the given tensors ([rows, cols, 3] uint8 and
+        [candidate_count, rows, cols] float32 per level)."""
+        f = cls.__new__(cls)
+        f.candidate_count, f.resolution, f.device = candidate_count, tuple(resolution), guides[0].device
+        f.scale_count, f.guides, f.costs = len(guides), list(guides), list(costs)
+        return f
+
     def apply(self, guide, cost, sigma_i, sigma_s):
         """Filter ``cost`` guided by ``guide``, both in place (python/isb_filter.py:72-136).
 

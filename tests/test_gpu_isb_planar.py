@@ -3,6 +3,8 @@ are shared out, at the edges of pixel groups, rows and ranges, equals the oracle
 the fused selection equals the two separate steps on costs that are not finite."""
 from __future__ import annotations
 
+import importlib
+
 import numpy as np
 import pytest
 import torch
@@ -74,3 +76,59 @@ def test_fused_selection_of_costs_that_are_not_finite(ss, native, n):
         out.append((d.cpu().numpy(), i.cpu().numpy(), g.cpu().numpy()))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("cols,rows,n,instances", [(65, 33, 3, 2), (64, 64, 32, 1), (131, 70, 9, 3), (40, 300, 5, 2),
+                                                   (258, 257, 2, 1), (96, 80, 1, 2)])
+def test_filter_of_several_volumes_equals_a_launch_per_step(ss, native, cols, rows, n, instances):
+    """ssg_isb_filter, its small levels in one launch, with the filtered guides apart and in place, and
+    ssg_isb_filter_select, against ssg_isb_downsample / _upsample / _upsample_select per volume."""
+    isb = importlib.import_module("sphere-stereo_gb300.isb_filter")
+    N = ss._native
+    stream = torch.cuda.current_stream().cuda_stream
+    shapes, si, sg = isb.level_shapes((cols, rows)), 9.0, 7.5
+    L = len(shapes)
+    weights, var = isb.level_weights(L, sg), 1 / (2 * si * si)
+    cases = [_case(cols, rows, n, 31 * i + n) for i in range(instances)]
+    g0 = torch.as_tensor(np.stack([g for g, _ in cases]), device=DEV)
+    c0 = torch.as_tensor(np.stack([c for _, c in cases]), device=DEV)
+
+    def levels(level0, channels, dtype):
+        return [level0.clone()] + [torch.zeros(instances, *channels(r, c), dtype=dtype, device=DEV) for r, c in shapes[1:]]
+
+    def guides():
+        return levels(g0, lambda r, c: (r, c, 3), torch.uint8)
+
+    def costs():
+        return levels(c0, lambda r, c: (n, r, c), torch.float32)
+
+    def ptrs(ts):
+        return N.pointers([t.data_ptr() for t in ts])
+
+    want_orig, want, want_c = guides(), guides(), costs()
+    cand = N.floats(ss.distance_candidates(0.55, 100.0, n).tolist())
+    want_d = torch.empty(instances, rows, cols, device=DEV)
+    want_i = torch.empty(instances, rows, cols, dtype=torch.int32, device=DEV)
+    for i in range(instances):
+        for s in range(1, L):
+            N.call("ssg_isb_downsample", want_orig[s - 1][i].data_ptr(), want_c[s - 1][i].data_ptr(), *shapes[s - 1],
+                   want_orig[s][i].data_ptr(), want_c[s][i].data_ptr(), *shapes[s], n, var, stream)
+            want[s][i].copy_(want_orig[s][i])
+        for s in range(L - 2, 0, -1):
+            N.call("ssg_isb_upsample", want[s + 1][i].data_ptr(), want_c[s + 1][i].data_ptr(), *shapes[s + 1],
+                   want[s][i].data_ptr(), want_c[s][i].data_ptr(), *shapes[s], n, *weights[s], var, stream)
+        fine = g0[i].clone()
+        N.call("ssg_isb_upsample_select", want[1][i].data_ptr(), want_c[1][i].data_ptr(), *shapes[1], fine.data_ptr(),
+               want_c[0][i].data_ptr(), rows, cols, n, *weights[0], var, cand, want_d[i].data_ptr(),
+               want_i[i].data_ptr(), stream)
+    g, f, c = guides(), [torch.zeros_like(t) for t in guides()], costs()
+    N.call("ssg_isb_filter", ptrs(g), ptrs(f), ptrs(c), L, rows, cols, n, instances, si, sg, stream)
+    for s in range(L):
+        assert torch.equal(g[s], want_orig[s]) and torch.equal(c[s], want_c[s])
+        assert s == 0 or torch.equal(f[s], want[s])
+    g, c = guides(), costs()
+    d, copy, i = torch.empty_like(want_d), torch.empty_like(want_d), torch.empty_like(want_i)
+    N.call("ssg_isb_filter_select", ptrs(g), ptrs(c), L, rows, cols, n, instances, si, sg, cand, d.data_ptr(),
+           i.data_ptr(), copy.data_ptr(), stream)
+    assert torch.equal(d, want_d) and torch.equal(copy, want_d) and torch.equal(i, want_i)
+    assert torch.equal(g[0], g0) and all(torch.equal(g[s], want[s]) for s in range(1, L))

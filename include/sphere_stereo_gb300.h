@@ -570,6 +570,46 @@ SSG_API int ssg_sweep_cost_backward(int cols, int rows, int camera_count, const 
                                     int candidate_count, const float* d_grad_cost, double* d_grad_pose,
                                     void* d_scratch, void* stream);
 
+/* ---- The differentiable sweep of several references at once (contiguous volumes, maps and guides,
+ * instance after instance; the values of the per-step functions above) ---- */
+
+/* Soft-argmin of the filtered level-0 costs of `instances` volumes (ssg_isb_upsample_softargmin): the
+ * coarse guides and costs are the filtered level 1, the fine ones the unfiltered level 0. */
+SSG_API int ssg_soft_argmin(const uint8_t* d_guide_coarse, const float* d_cost_coarse, const uint8_t* d_guide_fine,
+                            const float* d_cost_fine, int rows, int cols, int candidate_count, int instances,
+                            double sigma_i, double sigma_s, const float* candidates, float temperature,
+                            float* d_inverse_distance, void* stream);
+
+/* dL/dF of the filtered level 0 (ssg_isb_upsample_softargmin_backward) of `instances` volumes. */
+SSG_API int ssg_soft_argmin_backward(const uint8_t* d_guide_coarse, const float* d_cost_coarse,
+                                     const uint8_t* d_guide_fine, const float* d_cost_fine, int rows, int cols,
+                                     int candidate_count, int instances, double sigma_i, double sigma_s,
+                                     const float* candidates, float temperature, const float* d_grad_inverse_distance,
+                                     float* d_grad_filtered, void* stream);
+
+/* float32 values of one instance's table of filter weights (scratch of ssg_isb_filter_transpose) */
+SSG_API size_t ssg_isb_table_floats(int rows, int cols, int level_count);
+
+/* The whole filter transposed (every ssg_isb_upsample_transpose up, every ssg_isb_downsample_transpose
+ * back down): d_grad_filtered[0] in, d_grad_costs[0] out; the other levels of both are scratch, as is
+ * d_tables (instances x ssg_isb_table_floats).  Guides as ssg_isb_filter left them.  d_absmax: per
+ * instance the bits of the largest |dL/dcost|, for ssg_sweep_backward_references. */
+SSG_API int ssg_isb_filter_transpose(uint8_t* const* d_guides, uint8_t* const* d_filtered_guides, int level_count,
+                                     int rows, int cols, int candidate_count, int instances, double sigma_i,
+                                     double sigma_s, float* const* d_grad_filtered, float* const* d_grad_costs,
+                                     float* d_tables, uint32_t* d_absmax, void* stream);
+
+/* ssg_sweep_cost_backward of several references from packed images (ssg_pack_images), added to the
+ * images' and the poses' gradients; layouts as ssg_sweep_cost_references.  d_scratch: 256-byte aligned,
+ * ssg_sweep_backward_references_scratch_bytes. */
+SSG_API size_t ssg_sweep_backward_references_scratch_bytes(int cols, int rows, int camera_count, int reference_count);
+SSG_API int ssg_sweep_backward_references(int cols, int rows, int camera_count, const ssg_camera* cameras,
+                                          int reference_count, const int* references, const float* relative_poses,
+                                          const float* d_packed, float* const* d_grad_images,
+                                          const int8_t* d_selected, const float* candidates, int candidate_count,
+                                          const float* d_grad_cost, const uint32_t* d_absmax, double* d_grad_pose,
+                                          void* d_scratch, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Uneven batches (no counterpart in the reference, which estimates one rig's frame per call of
  * estimate_RGBD_panorama, python/depth_estimation.py:205-242): many RGB-D panorama jobs of

@@ -199,12 +199,11 @@ __device__ __forceinline__ float2 load_fine(const float* __restrict__ c, int at,
 }
 
 // Candidates [k0, k1) of the two fine pixels FA, FB of one fine row of coarse pixel (x, y) in column
-// `px` of sw: filtered in place, or (kSelect) selected into sel_a, sel_b.
-template <int FA, int FB, bool kSelect, bool kPairs>
-__device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in, float* cost_io, const LevelGeom& g,
-                                              int x, int y, int k0, int k1, float weight_up,
-                                              const float (&sw)[kUpRows][32], int px, RangeSelection* sel_a,
-                                              RangeSelection* sel_b)
+// `px` of sw, filtered; sink.take(k, at, a, b) gets each pair, `at` the pair's place in the level.
+template <int FA, int FB, bool kPairs, typename Sink>
+__device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in, const float* cost_fine,
+                                              const LevelGeom& g, int x, int y, int k0, int k1, float weight_up,
+                                              const float (&sw)[kUpRows][32], int px, Sink& sink)
 {
     const int fy = 2 * y + (FA & 1);
     const bool second = 2 * x + 1 < g.cols_out;
@@ -216,7 +215,7 @@ __device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in,
     // coarse taps, which neighbouring threads share in the caches, one ahead
     float2 own[kUpDepth];
     const float* c = cost_in + (int64_t)k0 * pin;
-    float* f = cost_io + (int64_t)k0 * pio;
+    const float* f = cost_fine + (int64_t)k0 * pio;
 #pragma unroll
     for (int j = 0; j < kUpDepth; ++j)
         if (k0 + j < k1) own[j] = load_fine<kPairs>(f + (int64_t)j * pio, f0, second);
@@ -230,8 +229,6 @@ __device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in,
 #pragma unroll
     for (int i = 0; i < UpTaps<FB>::n; ++i) wb[i] = sw[up_weight_row<FB>() + i][px];
     const float inv_a = sw[kUpInvRow + FA][px], inv_b = sw[kUpInvRow + FB][px];
-    Selector sa, sb;
-    float first_a = 0.0f, first_b = 0.0f;
     for (int k = k0; k < k1; k += kUpDepth) {
 #pragma unroll
         for (int j = 0; j < kUpDepth; ++j) {
@@ -253,28 +250,76 @@ __device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in,
             va = fmul(va, inv_a);
             vb = fmul(vb, inv_b);
             if (k + j + kUpDepth < k1) own[j] = load_fine<kPairs>(f + (int64_t)kUpDepth * pio, f0, second);
-            if constexpr (kSelect) {
-                if (k + j == k0) {
-                    first_a = va;
-                    first_b = vb;
-                }
-                sa.push(k + j, va);
-                sb.push(k + j, vb);
-            } else if constexpr (kPairs) {
-                *reinterpret_cast<float2*>(f + f0) = make_float2(va, vb);
-            } else {
-                f[f0] = va;
-                if (second) f[f0 + 1] = vb;
-            }
+            sink.take(k + j, f0, va, vb);
             f += pio;
 #pragma unroll
             for (int t = 0; t < 9; ++t)
                 if (uses_tap<FA>(t) || uses_tap<FB>(t)) cd[t] = nd[t];
         }
     }
-    if constexpr (kSelect) {
-        *sel_a = RangeSelection{sa.m, sa.M, sa.L, sa.R, first_a, sa.prev, 2 * sa.idx + (sa.need_right ? 1 : 0)};
-        *sel_b = RangeSelection{sb.m, sb.M, sb.L, sb.R, first_b, sb.prev, 2 * sb.idx + (sb.need_right ? 1 : 0)};
+}
+
+// writes the pairs to a level
+template <bool kPairs>
+struct StoreSink {
+    float* level;
+    int pio;
+    bool second;
+    __device__ __forceinline__ void take(int k, int at, float a, float b)
+    {
+        float* p = level + (int64_t)k * pio + at;
+        if constexpr (kPairs) {
+            *reinterpret_cast<float2*>(p) = make_float2(a, b);
+        } else {
+            p[0] = a;
+            if (second) p[1] = b;
+        }
+    }
+};
+
+// selects among the candidates of a range that starts at k0
+struct SelectSink {
+    int k0;
+    Selector a, b;
+    float first_a = 0.0f, first_b = 0.0f;
+    __device__ __forceinline__ void take(int k, int, float va, float vb)
+    {
+        if (k == k0) {
+            first_a = va;
+            first_b = vb;
+        }
+        a.push(k, va);
+        b.push(k, vb);
+    }
+    __device__ __forceinline__ static RangeSelection range(const Selector& s, float first)
+    {
+        return RangeSelection{s.m, s.M, s.L, s.R, first, s.prev, 2 * s.idx + (s.need_right ? 1 : 0)};
+    }
+};
+
+// The weights of a block's 32 coarse pixels into sw, the four fine pixels by four of its warps (the
+// caller synchronises the block)
+template <typename GL>
+__device__ __forceinline__ void planar_setup(const uint8_t* __restrict__ guide_in, const uint8_t* guide_fine,
+                                             uint8_t* guide_out, const LevelGeom& g, int x, int y, bool in,
+                                             float weight_up, float weight_down, const TableRange& range,
+                                             float (&sw)[kUpRows][32])
+{
+    const int px = threadIdx.x & 31;
+    for (int f = threadIdx.x >> 5; f < 4; f += blockDim.x >> 5) {
+        switch (f) {
+        case 0:
+            planar_fine_setup<0, 32, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, range, px, sw);
+            break;
+        case 1:
+            planar_fine_setup<1, 32, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, range, px, sw);
+            break;
+        case 2:
+            planar_fine_setup<2, 32, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, range, px, sw);
+            break;
+        default:
+            planar_fine_setup<3, 32, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, range, px, sw);
+        }
     }
 }
 
@@ -303,35 +348,23 @@ __global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges)
     const int o = blockIdx.x * kPx + px;
     const bool in = o < pin;
     const int y = o / g.cols_in, x = o - y * g.cols_in;
-    // weights: the four fine pixels go to four warps
-    const TableRange rw{table, var_inv_i};
-    for (int f = warp; f < 4; f += 2 * kRanges) {
-        switch (f) {
-        case 0:
-            planar_fine_setup<0, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
-            break;
-        case 1:
-            planar_fine_setup<1, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
-            break;
-        case 2:
-            planar_fine_setup<2, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
-            break;
-        default:
-            planar_fine_setup<3, kPx, GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, rw, px, sw);
-        }
-    }
+    planar_setup<GL>(guide_in, guide_fine, guide_out, g, x, y, in, weight_up, weight_down, TableRange{table, var_inv_i}, sw);
     __syncthreads();
     const int share = (ncand + kRanges - 1) / kRanges, range = warp >> 1;
     const int k0 = range * share, k1 = min(k0 + share, ncand);
-    if (in && k0 < k1) {
-        if ((warp & 1) == 0)
-            planar_up_row<0, 2, kSelect, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px,
-                                                 &part[kSelect ? range : 0][kSelect ? px : 0],
-                                                 &part[kSelect ? range : 0][kSelect ? 2 * kPx + px : 0]);
-        else if (2 * y + 1 < g.rows_out)
-            planar_up_row<1, 3, kSelect, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px,
-                                                 &part[kSelect ? range : 0][kSelect ? kPx + px : 0],
-                                                 &part[kSelect ? range : 0][kSelect ? 3 * kPx + px : 0]);
+    const bool upper = (warp & 1) == 0;  // the fine row of F = 0, 2, or of F = 1, 3
+    if (in && k0 < k1 && (upper || 2 * y + 1 < g.rows_out)) {
+        if constexpr (kSelect) {
+            SelectSink sink{k0};
+            if (upper) planar_up_row<0, 2, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px, sink);
+            else planar_up_row<1, 3, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px, sink);
+            part[range][(upper ? 0 : kPx) + px] = SelectSink::range(sink.a, sink.first_a);
+            part[range][(upper ? 2 * kPx : 3 * kPx) + px] = SelectSink::range(sink.b, sink.first_b);
+        } else {
+            StoreSink<kPairs> sink{cost_io, pio, 2 * x + 1 < g.cols_out};
+            if (upper) planar_up_row<0, 2, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px, sink);
+            else planar_up_row<1, 3, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px, sink);
+        }
     }
     if constexpr (kSelect) {
         __syncthreads();

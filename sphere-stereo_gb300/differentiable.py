@@ -23,32 +23,56 @@ from __future__ import annotations
 
 import math
 
+import numpy as np
 import torch
 
 from . import _native as N
-from .isb_filter import level_shapes, level_weights
-from .utils import _cpu32, camera_struct, relative_poses, rgb_to_guide
+from .isb_filter import level_shapes
+from .utils import _cpu32, camera_struct, relative_poses
 
 
-def skew(w):
-    return torch.tensor([[0.0, -w[2], w[1]], [w[2], 0.0, -w[0]], [-w[1], w[0], 0.0]], dtype=torch.float64)
+def skew(w) -> np.ndarray:
+    return np.array([[0.0, -w[2], w[1]], [w[2], 0.0, -w[0]], [-w[1], w[0], 0.0]])
 
 
-def so3_exp(w: torch.Tensor) -> torch.Tensor:
-    th = float(torch.linalg.norm(w))
+def so3_exp(w) -> np.ndarray:
+    th = float(np.linalg.norm(w))
     k = skew(w)
     if th < 1e-8:
-        return torch.eye(3, dtype=torch.float64) + k + 0.5 * k @ k
-    return torch.eye(3, dtype=torch.float64) + math.sin(th) / th * k + (1 - math.cos(th)) / th ** 2 * k @ k
+        return np.eye(3) + k + 0.5 * k @ k
+    return np.eye(3) + math.sin(th) / th * k + (1 - math.cos(th)) / th ** 2 * k @ k
 
 
-def so3_right_jacobian(w: torch.Tensor) -> torch.Tensor:
-    th = float(torch.linalg.norm(w))
+def so3_right_jacobian(w) -> np.ndarray:
+    th = float(np.linalg.norm(w))
     k = skew(w)
     if th < 1e-6:
-        return torch.eye(3, dtype=torch.float64) - 0.5 * k + k @ k / 6
-    return (torch.eye(3, dtype=torch.float64) - (1 - math.cos(th)) / th ** 2 * k
-            + (th - math.sin(th)) / th ** 3 * k @ k)
+        return np.eye(3) - 0.5 * k + k @ k / 6
+    return np.eye(3) - (1 - math.cos(th)) / th ** 2 * k + (th - math.sin(th)) / th ** 3 * k @ k
+
+
+class _Poses:
+    """The composed poses of one evaluation, in float64 on the host: T_c [Exp(omega_c), v_c] and, per
+    reference, the relative poses of every camera."""
+
+    def __init__(self, base: np.ndarray, refs: list[int], deltas: np.ndarray):
+        self.deltas = deltas
+        E = np.tile(np.eye(4), (len(deltas), 1, 1))
+        for c, d in enumerate(deltas):
+            E[c, :3, :3] = so3_exp(d[:3])
+        E[:, :3, 3] = deltas[:, 3:]
+        T = base @ E
+        inverse = np.linalg.inv(T)
+        self.relative = [(inverse @ T[r])[:, :3].reshape(-1) for r in refs]  # camera_count x 12 each
+
+    def to_deltas(self) -> np.ndarray:
+        """[cameras, 6, 6]: gradients of local right perturbations at T [Exp(omega), v] -> gradients with
+        respect to (omega, v)."""
+        out = np.zeros((len(self.deltas), 6, 6))
+        for c, d in enumerate(self.deltas):
+            out[c, :3, :3] = so3_right_jacobian(d[:3]).T
+            out[c, 3:, 3:] = so3_exp(d[:3])
+        return out
 
 
 class DifferentiableSweep:
@@ -79,121 +103,107 @@ class DifferentiableSweep:
         self.candidates = (1 / torch.linspace(1 / min_dist, 1 / max_dist, candidate_count)).tolist()
         self._cand = N.floats(self.candidates)
         self._cams = N.cameras_array([camera_struct(c) for c in calibrations])
-        self.base_poses = [_cpu32(c.rt).double() for c in calibrations]
+        self.base_poses = np.stack([_cpu32(c.rt).double().numpy() for c in calibrations])
         dev = device
         # camera selection of the unperturbed rig (a discrete choice: no gradient)
         mask_stack = torch.stack([torch.as_tensor(m, dtype=torch.float32).reshape(self.rows, self.cols)
                                   for m in masks]).to(dev).contiguous()
-        self.selected = []
-        for r in self.refs:
-            sel = torch.empty([self.rows, self.cols], dtype=torch.int8, device=dev)
+        selected = torch.empty([len(self.refs), self.rows, self.cols], dtype=torch.int8, device=dev)
+        for slot, r in enumerate(self.refs):
             N.call("ssg_select_camera", self.cols, self.rows, self.C, self._cams, r,
                    N.floats(relative_poses(calibrations, r)), mask_stack.data_ptr(), float(min_dist),
-                   float(max_dist), sel.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
-            self.selected.append(sel)
+                   float(max_dist), selected[slot].data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+        self._selected = selected
+        self.selected = list(selected)
+        # References are worked on together as long as their volumes (costs, and the two gradients of
+        # the filter) fit GROUP_BYTES: the launches of one reference do not fill the GPU
         f32 = dict(dtype=torch.float32, device=dev)
         u8 = dict(dtype=torch.uint8, device=dev)
-        self.costs = [torch.empty(self.N * r * c, **f32) for r, c in self.shapes]
-        self.g_orig = [torch.empty(r * c * 3, **u8) for r, c in self.shapes]
-        self.g_filt = [torch.empty(r * c * 3, **u8) for r, c in self.shapes]
-        self.gf = [torch.empty(self.N * r * c, **f32) for r, c in self.shapes]
-        self.gc = [torch.empty(self.N * r * c, **f32) for r, c in self.shapes]
-        self.weights = level_weights(self.L, self.sigma_s)
-        self.var_inv_i = 1 / (2 * self.sigma_i * self.sigma_i)
-        # the sweep backward's fixed-point image sums and pose block sums
-        scratch = N.library().ssg_sweep_backward_scratch_bytes(self.cols, self.rows, self.C)
-        self._bwd_scratch = torch.empty((scratch + 255) // 256 * 256, dtype=torch.uint8, device=dev)
+        pyramid = sum(r * c for r, c in self.shapes)
+        per_reference = 12 * self.N * pyramid + 24 * self.C * self.P
+        self.group = G = max(1, min(len(self.refs), 4, self.GROUP_BYTES // per_reference))
+        self.packed = torch.empty(self.C, self.rows, self.cols, 4, **f32)
+        self.g_orig = [torch.empty(G * r * c * 3, **u8) for r, c in self.shapes]
+        self.g_filt = [self.g_orig[0]] + [torch.empty(G * r * c * 3, **u8) for r, c in self.shapes[1:]]
+        self.costs, self.gf, self.gc = ([torch.empty(G * self.N * r * c, **f32) for r, c in self.shapes]
+                                        for _ in range(3))
+        lib = N.library()
+        self._tables = torch.empty(G * lib.ssg_isb_table_floats(self.rows, self.cols, self.L), **f32)
+        self._absmax = torch.empty(G, dtype=torch.int32, device=dev)
+        scratch = lib.ssg_sweep_backward_references_scratch_bytes(self.cols, self.rows, self.C, G)
+        self._bwd_scratch = torch.empty((scratch + 255) // 256 * 256, **u8)
+        self._levels = {name: N.pointers([t.data_ptr() for t in getattr(self, name)])
+                        for name in ("g_orig", "g_filt", "costs", "gf", "gc")}
+
+    GROUP_BYTES = 4 << 30
 
     def set_selection(self, selected):
         """Use another run's camera-selection maps ([references][rows, cols])."""
-        self.selected = [torch.as_tensor(s).reshape(self.rows, self.cols).to(self.device, torch.int8).contiguous()
-                         for s in selected]
+        self._selected = torch.stack([torch.as_tensor(s).reshape(self.rows, self.cols).to(self.device, torch.int8)
+                                      for s in selected])
+        self.selected = list(self._selected)
 
     # ------------------------------------------------------------------------------------
-    def _poses(self, deltas: torch.Tensor):
-        """Float64 composition: T_c [Exp(omega_c), v_c] and, per reference, the relative poses."""
-        d = deltas.detach().to("cpu", torch.float64)
-        T = []
-        for c in range(self.C):
-            E = torch.eye(4, dtype=torch.float64)
-            E[:3, :3] = so3_exp(d[c, :3])
-            E[:3, 3] = d[c, 3:]
-            T.append(self.base_poses[c] @ E)
-        rel = {r: N.floats([float(v) for c in range(self.C) for v in (torch.linalg.inv(T[c]) @ T[r])[:3].reshape(12)])
-               for r in self.refs}
-        return d, rel
+    def _poses(self, deltas: torch.Tensor) -> _Poses:
+        return _Poses(self.base_poses, self.refs, deltas.detach().to("cpu", torch.float64).numpy().copy())
 
-    def _pyramid(self, r: int, images: torch.Tensor, rel, stream) -> None:
-        """Sweep + ISB down / up steps (levels 1..L-1 filtered; level 0 left raw)."""
-        cols, rows, n = self.cols, self.rows, self.N
-        rgb_to_guide(images[r], self.g_orig[0].view(rows, cols, 3))
-        N.call("ssg_sweep_cost", cols, rows, self.C, self._cams, r, rel[r],
-               N.pointers([images[c].data_ptr() for c in range(self.C)]), self.selected[self.refs.index(r)].data_ptr(),
-               self._cand, n, self.costs[0].data_ptr(), stream)
-        for s in range(1, self.L):
-            (ri, ci), (ro, co) = self.shapes[s - 1], self.shapes[s]
-            N.call("ssg_isb_downsample", self.g_orig[s - 1].data_ptr(), self.costs[s - 1].data_ptr(), ri, ci,
-                   self.g_orig[s].data_ptr(), self.costs[s].data_ptr(), ro, co, n, self.var_inv_i, stream)
-        for s in range(1, self.L):
-            self.g_filt[s].copy_(self.g_orig[s])
-        for s in range(self.L - 2, 0, -1):
-            (rc, cc), (rf, cf) = self.shapes[s + 1], self.shapes[s]
-            wu, wd = self.weights[s]
-            N.call("ssg_isb_upsample", self.g_filt[s + 1].data_ptr(), self.costs[s + 1].data_ptr(), rc, cc,
-                   self.g_filt[s].data_ptr(), self.costs[s].data_ptr(), rf, cf, n, wu, wd, self.var_inv_i, stream)
+    def _groups(self):
+        """(first slot, references, how many) of each group of references."""
+        for g0 in range(0, len(self.refs), self.group):
+            refs = self.refs[g0:g0 + self.group]
+            yield g0, refs, len(refs)
 
-    def forward(self, images: torch.Tensor, deltas: torch.Tensor) -> torch.Tensor:
+    def _pyramid(self, g0: int, refs: list[int], images: torch.Tensor, poses: _Poses, stream):
+        """Sweep + filter of a group of references (levels 1..L-1 filtered; level 0 left raw).  Returns
+        what the sweep was called with: the references and their relative poses."""
+        count = len(refs)
+        refs_c, rel = N.ints(refs), N.floats(np.concatenate(poses.relative[g0:g0 + count]))
+        N.call("ssg_pack_images", N.pointers([images[c].data_ptr() for c in range(self.C)]), self.C, self.P, refs_c,
+               count, self.packed.data_ptr(), self.g_orig[0].data_ptr(), stream)
+        N.call("ssg_sweep_cost_references", self.cols, self.rows, self.C, self._cams, count, refs_c, rel,
+               self.packed.data_ptr(), self._selected[g0].data_ptr(), self._cand, self.N, self.costs[0].data_ptr(),
+               stream)
+        N.call("ssg_isb_filter", self._levels["g_orig"], self._levels["g_filt"], self._levels["costs"], self.L,
+               self.rows, self.cols, self.N, count, self.sigma_i, self.sigma_s, stream)
+        return refs_c, rel
+
+    def _last_level(self, count: int):
+        """The arguments of the soft-argmin's last filter level."""
+        return (self.g_filt[1].data_ptr(), self.costs[1].data_ptr(), self.g_orig[0].data_ptr(),
+                self.costs[0].data_ptr(), self.rows, self.cols, self.N, count, self.sigma_i, self.sigma_s, self._cand,
+                self.temperature)
+
+    def forward(self, images: torch.Tensor, deltas: torch.Tensor, poses: _Poses | None = None) -> torch.Tensor:
+        """poses: the composed poses of ``deltas``, where the caller has them."""
         N.require(images, "images", torch.float32, (self.C, self.rows, self.cols, 3), self.device)
         stream = N.stream_of(images)
-        _, rel = self._poses(deltas)
+        poses = self._poses(deltas) if poses is None else poses
         q = torch.empty(len(self.refs), self.rows, self.cols, device=self.device)
-        (rc, cc) = self.shapes[1]
-        wu, wd = self.weights[0]
-        for slot, r in enumerate(self.refs):
-            self._pyramid(r, images, rel, stream)
-            N.call("ssg_isb_upsample_softargmin", self.g_filt[1].data_ptr(), self.costs[1].data_ptr(), rc, cc,
-                   self.g_orig[0].data_ptr(), self.costs[0].data_ptr(), self.rows, self.cols, self.N, wu, wd,
-                   self.var_inv_i, self._cand, self.temperature, q[slot].data_ptr(), stream)
+        for g0, refs, count in self._groups():
+            self._pyramid(g0, refs, images, poses, stream)
+            N.call("ssg_soft_argmin", *self._last_level(count), q[g0].data_ptr(), stream)
         return q
 
-    def backward(self, images: torch.Tensor, deltas: torch.Tensor, grad_q: torch.Tensor):
+    def backward(self, images: torch.Tensor, deltas: torch.Tensor, grad_q: torch.Tensor, poses: _Poses | None = None):
         stream = N.stream_of(images)
-        d, rel = self._poses(deltas)
+        poses = self._poses(deltas) if poses is None else poses
         grad_images = torch.zeros_like(images)
         grad_local = torch.zeros(self.C, 6, dtype=torch.float64, device=self.device)
-        cols, rows, n = self.cols, self.rows, self.N
-        for slot, r in enumerate(self.refs):
-            self._pyramid(r, images, rel, stream)
-            (rc, cc) = self.shapes[1]
-            wu, wd = self.weights[0]
-            # dL/dF of the filtered level 0, then every up step transposed from level 0 upwards:
-            # each writes its level's own-pixel gradient and the next level's filtered gradient
-            N.call("ssg_isb_upsample_softargmin_backward", self.g_filt[1].data_ptr(), self.costs[1].data_ptr(), rc, cc,
-                   self.g_orig[0].data_ptr(), self.costs[0].data_ptr(), rows, cols, n, wu, wd, self.var_inv_i,
-                   self._cand, self.temperature, grad_q[slot].data_ptr(), self.gf[0].data_ptr(), stream)
-            for s in range(0, self.L - 1):
-                (rc, cc), (rf, cf) = self.shapes[s + 1], self.shapes[s]
-                wu, wd = self.weights[s]
-                N.call("ssg_isb_upsample_transpose", self.g_filt[s + 1].data_ptr(), rc, cc, self.g_orig[s].data_ptr(),
-                       rf, cf, n, wu, wd, self.var_inv_i, self.gf[s].data_ptr(), self.gc[s].data_ptr(),
-                       self.gf[s + 1].data_ptr(), stream)
-            self.gc[self.L - 1].copy_(self.gf[self.L - 1])  # f_{L-1} = c_{L-1}
-            for s in range(self.L - 1, 0, -1):
-                (ri, ci), (ro, co) = self.shapes[s - 1], self.shapes[s]
-                N.call("ssg_isb_downsample_transpose", self.g_orig[s - 1].data_ptr(), ri, ci, ro, co, n,
-                       self.var_inv_i, self.gc[s].data_ptr(), self.gc[s - 1].data_ptr(), stream)
-            N.call("ssg_sweep_cost_backward", cols, rows, self.C, self._cams, r, rel[r],
-                   N.pointers([images[c].data_ptr() for c in range(self.C)]),
-                   N.pointers([grad_images[c].data_ptr() for c in range(self.C)]),
-                   self.selected[slot].data_ptr(), self._cand, n, self.gc[0].data_ptr(), grad_local.data_ptr(),
-                   self._bwd_scratch.data_ptr(), stream)
-        # local right perturbations at T [Exp(omega), v]  ->  gradients with respect to (omega, v)
-        g = grad_local.cpu()
-        out = torch.empty_like(g)
-        for c in range(self.C):
-            w = d[c, :3]
-            out[c, :3] = so3_right_jacobian(w).T @ g[c, :3]
-            out[c, 3:] = so3_exp(w) @ g[c, 3:]
+        targets = N.pointers([grad_images[c].data_ptr() for c in range(self.C)])
+        for g0, refs, count in self._groups():
+            refs_c, rel = self._pyramid(g0, refs, images, poses, stream)
+            # dL/dF of the filtered level 0, then the filter transposed, then the sweep
+            N.call("ssg_soft_argmin_backward", *self._last_level(count), grad_q[g0].data_ptr(), self.gf[0].data_ptr(),
+                   stream)
+            N.call("ssg_isb_filter_transpose", self._levels["g_orig"], self._levels["g_filt"], self.L, self.rows,
+                   self.cols, self.N, count, self.sigma_i, self.sigma_s, self._levels["gf"], self._levels["gc"],
+                   self._tables.data_ptr(), self._absmax.data_ptr(), stream)
+            N.call("ssg_sweep_backward_references", self.cols, self.rows, self.C, self._cams, count, refs_c, rel,
+                   self.packed.data_ptr(), targets, self._selected[g0].data_ptr(), self._cand, self.N,
+                   self.gc[0].data_ptr(), self._absmax.data_ptr(), grad_local.data_ptr(), self._bwd_scratch.data_ptr(),
+                   stream)
+        to_deltas = torch.from_numpy(poses.to_deltas()).to(self.device, non_blocking=True)
+        out = (to_deltas * grad_local[:, None, :]).sum(-1)
         return grad_images, out.to(deltas.device)
 
     def __call__(self, images: torch.Tensor, pose_deltas: torch.Tensor | None = None) -> torch.Tensor:
@@ -210,10 +220,11 @@ class _SoftSweep(torch.autograd.Function):
         images_c = images.detach().contiguous()
         ctx.save_for_backward(images_c, pose_deltas.detach())
         ctx.sweep = sweep
-        return sweep.forward(images_c, pose_deltas)
+        ctx.poses = sweep._poses(pose_deltas)  # host values: the backward need not read the deltas again
+        return sweep.forward(images_c, pose_deltas, ctx.poses)
 
     @staticmethod
     def backward(ctx, grad_q):
         images, deltas = ctx.saved_tensors
-        gi, gd = ctx.sweep.backward(images, deltas, grad_q.contiguous())
+        gi, gd = ctx.sweep.backward(images, deltas, grad_q.contiguous(), ctx.poses)
         return gi, gd, None

@@ -286,53 +286,45 @@ __device__ __forceinline__ bool down_reader(const LevelGeom& g, int n, int X, in
 
 constexpr int kTransposeBlock = 256, kTransposeRanges = kTransposeBlock / 32;
 
-// Up step transposed: g_c(fine) = own weight * g_f(fine), g_f(coarse) = sum over the cell's readers.
-// A block takes 32 coarse cells; its 8 warps share out their weights and then the candidates.
-// blockIdx.y: instance.
+// Up step transposed: g_f(coarse) = sum over the cell's readers.  (A fine pixel's own part, own weight *
+// g_f(fine), is formed by the down step's kernel, which reads g_f once more instead of adding to a
+// volume written here.)  A block takes 32 coarse cells; its 8 warps share out their weights and then
+// the candidates.  blockIdx.y: instance.
 __global__ void __launch_bounds__(kTransposeBlock) isb_up_transpose_table_kernel(
-    const float* __restrict__ tables, int64_t table_stride, LevelGeom g, int ncand, float weight_up,
-    const float* __restrict__ grad_f_fine, float* __restrict__ grad_c_fine, float* __restrict__ grad_f_coarse)
+    const float* __restrict__ tables, int64_t table_stride, LevelGeom g, int ncand,
+    const float* __restrict__ grad_f_fine, float* __restrict__ grad_f_coarse)
 {
-    __shared__ float sk[kEntries + 4][32];
+    __shared__ float sk[kEntries][32];
     const int pin = g.rows_in * g.cols_in, pio = g.rows_out * g.cols_out;
     const int64_t inst = blockIdx.y;
     tables += inst * table_stride;
     grad_f_fine += inst * ncand * pio;
-    grad_c_fine += inst * ncand * pio;
     grad_f_coarse += inst * ncand * pin;
     const int px = threadIdx.x & 31, range = threadIdx.x >> 5;
     const int o = blockIdx.x * 32 + px, oc = min(o, pin - 1);
     const int Y = oc / g.cols_in, X = oc - Y * g.cols_in;
 #pragma unroll 1
-    for (int e = range; e < kEntries + 4; e += kTransposeRanges) {
-        if (e < kEntries) {
-            const TransposeEntry t = transpose_entry(e);
-            sk[e][px] = read_weight(t.f, tables, g, X + t.dx, Y + t.dy, X, Y);
-        } else {
-            sk[e][px] = own_weight(e - kEntries, tables, g, X, Y, weight_up);
-        }
+    for (int e = range; e < kEntries; e += kTransposeRanges) {
+        const TransposeEntry t = transpose_entry(e);
+        sk[e][px] = read_weight(t.f, tables, g, X + t.dx, Y + t.dy, X, Y);
     }
     __syncthreads();
-    float k[kEntries], own[4];
+    float k[kEntries];
     bool full = true;
 #pragma unroll
     for (int e = 0; e < kEntries; ++e) {
         k[e] = sk[e][px];
         full = full && k[e] != 0.0f;
     }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) own[f] = sk[kEntries + f][px];
     const int share = (ncand + kTransposeRanges - 1) / kTransposeRanges;
     const int z0 = range * share, z1 = min(z0 + share, ncand);
-    const bool set1 = 2 * Y + 1 < g.rows_out, set2 = 2 * X + 1 < g.cols_out;
     const int corner = (2 * Y - 2) * g.cols_out + 2 * X - 2;  // of the 5 x 5 fine pixels
     const bool in = o < pin;
     full = __all_sync(0xffffffffu, full) != 0;
 #pragma unroll 2
     for (int z = z0; z < z1; ++z) {
         const float* gf = grad_f_fine + (int64_t)z * pio;
-        float* gc = grad_c_fine + (int64_t)z * pio;
-        float acc = 0.0f, mine[4];
+        float acc = 0.0f;
         if (full) {
             float v[5][5];
 #pragma unroll
@@ -344,8 +336,6 @@ __global__ void __launch_bounds__(kTransposeBlock) isb_up_transpose_table_kernel
                 const TransposeEntry t = transpose_entry(e);
                 acc = fmaf(k[e], v[2 * t.dy + (t.f & 1) + 2][2 * t.dx + (t.f >= 2) + 2], acc);
             }
-#pragma unroll
-            for (int f = 0; f < 4; ++f) mine[f] = v[2 + (f & 1)][2 + (f >= 2)];
         } else {
 #pragma unroll
             for (int e = 0; e < kEntries; ++e) {
@@ -354,69 +344,104 @@ __global__ void __launch_bounds__(kTransposeBlock) isb_up_transpose_table_kernel
                     acc = fmaf(k[e], __ldg(gf + corner + (2 * t.dy + (t.f & 1) + 2) * g.cols_out + 2 * t.dx + (t.f >= 2) + 2),
                                acc);
             }
-#pragma unroll
-            for (int f = 0; f < 4; ++f)
-                mine[f] = (!(f & 1) || set1) && (f < 2 || set2)
-                              ? __ldg(gf + corner + (2 + (f & 1)) * g.cols_out + 2 + (f >= 2)) : 0.0f;
         }
-        if (!in) continue;
-        grad_f_coarse[(int64_t)z * pin + o] = acc;
-        float* p = gc + 2 * Y * g.cols_out + 2 * X;
-        p[0] = own[0] * mine[0];
-        if (set1) p[g.cols_out] = own[1] * mine[1];
-        if (set2) p[1] = own[2] * mine[2];
-        if (set1 && set2) p[g.cols_out + 1] = own[3] * mine[3];
+        if (in) grad_f_coarse[(int64_t)z * pin + o] = acc;
     }
 }
 
-// Down step transposed: g_c(fine) += sum over the coarse pixels that read the cell.  A block takes 32
-// fine cells.  absmax (level 0, else nullptr): the largest |g_c| of the instance, as float bits.
-__global__ void __launch_bounds__(kTransposeBlock) isb_down_transpose_table_kernel(
-    const float* __restrict__ tables, int64_t table_stride, LevelGeom g, int ncand,
-    const float* __restrict__ grad_c_coarse, float* __restrict__ grad_c_fine, uint32_t* __restrict__ absmax)
+// Down step transposed: g_c(fine) = own weight * g_f(fine) + sum over the coarse pixels that read the
+// cell.  A thread takes the 2 x 2 fine pixels of a coarse one, which are read by it and its right and
+// lower neighbours (9 weights); a block takes 32 of them, its warps share out the weights and then the
+// candidates.  kPairs: fine rows are read and written in pairs.  absmax (level 0, else nullptr): the
+// largest |g_c| of the instance, as float bits.
+struct QuadEntry {
+    int a, b, n;  // fine column and row, reader
+};
+__host__ __device__ constexpr QuadEntry quad_entry(int e)
 {
-    __shared__ float sk[4][32];
+    return e == 0 ? QuadEntry{0, 0, 0}
+         : e < 3  ? QuadEntry{1, 0, e - 1}
+         : e < 5  ? QuadEntry{0, 1, (e - 3) * 2}
+                  : QuadEntry{1, 1, e - 5};
+}
+constexpr int kQuadEntries = 9;
+
+template <bool kPairs>
+__global__ void __launch_bounds__(kTransposeBlock) isb_down_transpose_table_kernel(
+    const float* __restrict__ tables, int64_t table_stride, LevelGeom g, int ncand, float weight_up,
+    const float* __restrict__ grad_f_fine, const float* __restrict__ grad_c_coarse, float* __restrict__ grad_c_fine,
+    uint32_t* __restrict__ absmax)
+{
+    __shared__ float sk[kQuadEntries + 4][32];
     const int pin = g.rows_in * g.cols_in, pio = g.rows_out * g.cols_out;
     const int64_t inst = blockIdx.y;
     tables += inst * table_stride;
-    grad_c_coarse += inst * ncand * pin;
-    grad_c_fine += inst * ncand * pio;
-    const int px = threadIdx.x & 31, range = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + px, ic = min(i, pio - 1);
-    const int Y = ic / g.cols_out, X = ic - Y * g.cols_out;
-    if (range < 4) {
-        int x, y;
-        sk[range][px] = down_reader(g, range, X, Y, x, y) ? down_read_weight(tables, g, x, y, X, Y) : 0.0f;
+    const int px = threadIdx.x & 31, range = threadIdx.x >> 5, ranges = blockDim.x >> 5;
+    const int o = blockIdx.x * 32 + px, oc = min(o, pin - 1);
+    const int y = oc / g.cols_in, x = oc - y * g.cols_in;
+    const bool set1 = 2 * y + 1 < g.rows_out, set2 = 2 * x + 1 < g.cols_out;
+#pragma unroll 1
+    for (int e = range; e < kQuadEntries + 4; e += ranges) {
+        if (e < kQuadEntries) {
+            const QuadEntry q = quad_entry(e);
+            const int X = 2 * x + q.a, Y = 2 * y + q.b;
+            int rx, ry;
+            sk[e][px] = X < g.cols_out && Y < g.rows_out && down_reader(g, q.n, X, Y, rx, ry)
+                            ? down_read_weight(tables, g, rx, ry, X, Y) : 0.0f;
+        } else {
+            sk[e][px] = own_weight(e - kQuadEntries, tables, g, x, y, weight_up);
+        }
     }
     __syncthreads();
-    float k[4];
-    int co[4];
+    float k[kQuadEntries], own[4];
+    bool full = true;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-        int x, y;
-        down_reader(g, n, X, Y, x, y);
-        k[n] = sk[n][px];
-        co[n] = y * g.cols_in + x;  // read only where the weight is not 0
+    for (int e = 0; e < kQuadEntries; ++e) {
+        k[e] = sk[e][px];
+        full = full && k[e] != 0.0f;
     }
-    const int share = (ncand + kTransposeRanges - 1) / kTransposeRanges;
-    const int z0 = range * share, z1 = min(z0 + share, ncand);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) own[f] = sk[kQuadEntries + f][px];
+    const int share = (ncand + ranges - 1) / ranges;
+    const int z0 = range * share, z1 = o < pin ? min(z0 + share, ncand) : 0;
+    const int right = min(x + 1, g.cols_in - 1) - x, below = (min(y + 1, g.rows_in - 1) - y) * g.cols_in;
+    const float* gc = grad_c_coarse + (inst * ncand + z0) * pin + oc;
+    const int64_t fine = (inst * ncand + z0) * pio + 2 * y * g.cols_out + 2 * x;
+    const float* gf = grad_f_fine + fine;
+    float* out = grad_c_fine + fine;
+    const int down = set1 ? g.cols_out : 0;
     uint32_t largest = 0;
-    if (i < pio)
-#pragma unroll 4
-        for (int z = z0; z < z1; ++z) {
-            const float* gc = grad_c_coarse + (int64_t)z * pin;
-            float acc = 0.0f;
+#pragma unroll 2
+    for (int z = z0; z < z1; ++z, gc += pin, gf += pio, out += pio) {
+        const float v[4] = {__ldg(gc), __ldg(gc + right), __ldg(gc + below), __ldg(gc + below + right)};
+        const float2 top = load_fine<kPairs>(gf, 0, set2), bottom = load_fine<kPairs>(gf, down, set2);
+        const float mine[4] = {top.x, bottom.x, top.y, bottom.y};  // by f
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int n = 0; n < 4; ++n)
-                if (k[n] != 0.0f) acc = fmaf(k[n], __ldg(gc + co[n]), acc);
-            float* p = grad_c_fine + (int64_t)z * pio + i;
-            const float v = *p + acc;
-            *p = v;
-            largest = max(largest, __float_as_uint(v) & 0x7FFFFFFFu);
+        for (int e = 0; e < kQuadEntries; ++e) {
+            const QuadEntry q = quad_entry(e);
+            const int f = q.b + 2 * q.a;
+            if (full || k[e] != 0.0f) acc[f] = fmaf(k[e], v[q.n], acc[f]);
         }
-    if (absmax) {
+        float r[4];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) largest = max(largest, __shfl_down_sync(0xffffffffu, largest, off));
+        for (int f = 0; f < 4; ++f) {
+            r[f] = fadd(fmul(own[f], mine[f]), acc[f]);
+            if (((f & 1) && !set1) || (f >= 2 && !set2)) r[f] = 0.0f;
+            largest = max(largest, __float_as_uint(r[f]) & 0x7FFFFFFFu);
+        }
+        if constexpr (kPairs) {
+            *reinterpret_cast<float2*>(out) = make_float2(r[0], r[2]);
+            if (set1) *reinterpret_cast<float2*>(out + g.cols_out) = make_float2(r[1], r[3]);
+        } else {
+            out[0] = r[0];
+            if (set2) out[1] = r[2];
+            if (set1) out[g.cols_out] = r[1];
+            if (set1 && set2) out[g.cols_out + 1] = r[3];
+        }
+    }
+    if (absmax) {
+        largest = __reduce_max_sync(0xffffffffu, largest);
         // most warps find a larger value already there
         if (px == 0 && largest > *reinterpret_cast<volatile uint32_t*>(absmax + inst)) atomicMax(absmax + inst, largest);
     }
@@ -511,14 +536,18 @@ struct SweepBwdReferences {
     float cand[SSG_MAX_CANDIDATES];
 };
 
-// v rounded to the nearest integer (__float2ll_rn, without the FP64 pipe); |v| < 2^63
+// v rounded to the nearest integer (__float2ll_rn, without the FP64 pipe), |v| < 2^62: multiples of 2^40
+// and of 2^20 are taken off by sums with 1.5 x 2^63 and 1.5 x 2^43, whose last bits they are, and the
+// rest is rounded by a sum with 1.5 x 2^23.  The differences are exact, and the parts taken off are
+// even, so a tie rounds as v's does.  (inf and NaN give some number.)
 __device__ __forceinline__ long long fixed_of(float v)
 {
-    const uint32_t u = __float_as_uint(v);
-    const int e = (int)((u >> 23) & 255u);
-    if (e < 150) return (long long)__float2int_rn(v);  // |v| < 2^23; above, v is an integer
-    const long long m = (long long)((unsigned long long)((u & 0x7FFFFFu) | 0x800000u) << ((e - 150) & 63));
-    return (int32_t)u < 0 ? -m : m;
+    const float a = fadd(v, 0x1.8p63f), va = fsub(v, fsub(a, 0x1.8p63f));
+    const float b = fadd(va, 0x1.8p43f), vb = fsub(va, fsub(b, 0x1.8p43f));
+    const float c = fadd(vb, 0x1.8p23f);
+    const int ia = __float_as_int(a) - 0x5F400000, ib = __float_as_int(b) - 0x55400000;
+    const int ic = __float_as_int(c) - 0x4B400000;
+    return ((long long)ia << 40) + (long long)ib * (1 << 20) + ic;
 }
 
 // __ll2float_rn without the FP64 pipe: 24 leading bits, rounded to nearest even
@@ -545,6 +574,12 @@ __device__ __forceinline__ long long shfl_up64(long long v, int d)
     return (long long)(((unsigned long long)(uint32_t)hi << 32) | (uint32_t)lo);
 }
 
+__device__ __forceinline__ long long signed_part(long long q, int sign, int ch)
+{
+    const int s = (sign >> (2 * ch)) & 3;
+    return s == 1 ? q : s == 2 ? -q : 0;
+}
+
 __device__ __forceinline__ void fixed_add(long long* p, long long q)
 {
     if (q) atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)q);
@@ -561,6 +596,50 @@ __device__ __forceinline__ void halve(double (&v)[8], int off)
         const double give = upper ? v[j] : v[j + kCount / 2], keep = upper ? v[j + kCount / 2] : v[j];
         v[j] = keep + __shfl_xor_sync(0xffffffffu, give, off);
     }
+}
+
+// project_jacobian, its quotients by d1 and d2 from their reciprocals
+__device__ __forceinline__ void project_jacobian_packed(const float p[3], const TorchCam& k, float ju[3], float jv[3])
+{
+    const float x = p[0], y = p[1], z = p[2];
+    const float d1 = sqrtf(x * x + y * y + z * z);
+    const float c = k.xi * d1 + z;
+    const float d2 = sqrtf(x * x + y * y + c * c);
+    const float nrm = k.alpha * d2 + k.one_minus_alpha * c;
+    float q1[3] = {k.xi * x, k.xi * y, k.xi * z}, q2[3], dc[3];
+    const bool fine = d1 > 1e-10f && d1 < 1e10f && d2 > 1e-10f && d2 < 1e10f;
+    if (fine) {
+        const float r1 = __frcp_rn(d1);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) q1[j] = div_by_reciprocal(q1[j], d1, r1);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) q1[j] = fdiv(q1[j], d1);
+    }
+    dc[0] = q1[0];
+    dc[1] = q1[1];
+    dc[2] = q1[2] + 1.0f;
+    q2[0] = k.alpha * (x + c * dc[0]);
+    q2[1] = k.alpha * (y + c * dc[1]);
+    q2[2] = k.alpha * (c * dc[2]);
+    if (fine) {
+        const float r2 = __frcp_rn(d2);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) q2[j] = div_by_reciprocal(q2[j], d2, r2);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) q2[j] = fdiv(q2[j], d2);
+    }
+    float dn[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) dn[j] = q2[j] + k.one_minus_alpha * dc[j];
+    const float in = 1.0f / nrm, in2 = in * in;
+    ju[0] = k.fx * (in - x * dn[0] * in2);
+    ju[1] = k.fx * (-x * dn[1] * in2);
+    ju[2] = k.fx * (-x * dn[2] * in2);
+    jv[0] = k.fy * (-y * dn[0] * in2);
+    jv[1] = k.fy * (in - y * dn[1] * in2);
+    jv[2] = k.fy * (-y * dn[2] * in2);
 }
 
 // A block takes 32 x 8 pixels of one reference (blockIdx.z), a warp 8 x 4 of them: the samples of
@@ -604,12 +683,10 @@ __global__ void __launch_bounds__(kBwdBlock, 2) sweep_backward_references_kernel
         if (active && k + 1 < p.ncand) g_next = __ldg(grad_cost + (int64_t)(k + 1) * P);
         bool live = active && g != 0.0f;
         if (!__any_sync(0xffffffffu, live)) continue;
-        // contributions to the texels left / right of the sample, in its upper and lower row
-        long long ql[2][3], qr[2][3];
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int ch = 0; ch < 3; ++ch) ql[a][ch] = qr[a][ch] = 0;
+        // |contribution| to the texels left / right of the sample in its upper and lower row; a channel's
+        // is that, its negative or 0 (sign: 2 bits per channel)
+        long long left[2] = {0, 0}, right[2] = {0, 0};
+        int sign = 0;
         int tx = 0, ty = 0;
         bool lands = false;  // on a texel of the image
         if (live) {
@@ -662,24 +739,22 @@ __global__ void __launch_bounds__(kBwdBlock, 2) sweep_backward_references_kernel
                     const float sg = res[ch] > 0.0f ? 1.0f : (res[ch] < 0.0f ? -1.0f : 0.0f);
                     gs[ch] = g * sg;
                     gref[ch] -= gs[ch];
+                    sign |= (res[ch] > 0.0f ? 1 : res[ch] < 0.0f ? 2 : 0) << (2 * ch);
                 }
                 lands = in[0] || in[1] || in[2] || in[3];
                 if (lands) {
                     tx = (int)x0;
                     ty = (int)y0;
-#pragma unroll
-                    for (int ch = 0; ch < 3; ++ch) {
-                        if (in[0]) ql[0][ch] = fixed_of(gs[ch] * w[0] * scale);
-                        if (in[1]) qr[0][ch] = fixed_of(gs[ch] * w[1] * scale);
-                        if (in[2]) ql[1][ch] = fixed_of(gs[ch] * w[2] * scale);
-                        if (in[3]) qr[1][ch] = fixed_of(gs[ch] * w[3] * scale);
-                    }
+                    if (in[0]) left[0] = fixed_of(g * w[0] * scale);
+                    if (in[1]) right[0] = fixed_of(g * w[1] * scale);
+                    if (in[2]) left[1] = fixed_of(g * w[2] * scale);
+                    if (in[3]) right[1] = fixed_of(g * w[3] * scale);
                 }
                 // d ix / d u = d iy / d v = 1 (the normalisation round trip is the identity)
                 const float gu = gs[0] * sx[0] + gs[1] * sx[1] + gs[2] * sx[2];
                 const float gv = gs[0] * sy[0] + gs[1] * sy[1] + gs[2] * sy[2];
                 float ju[3], jv[3];
-                project_jacobian(q, cam, ju, jv);
+                project_jacobian_packed(q, cam, ju, jv);
                 const float gp[3] = {gu * ju[0] + gv * jv[0], gu * ju[1] + gv * jv[1], gu * ju[2] + gv * jv[2]};
                 // source camera: p' = exp(-delta) p  ->  dL/domega = g x p, dL/dv = -g
                 gsrc[0] += gp[1] * q[2] - gp[2] * q[1];
@@ -707,13 +782,17 @@ __global__ void __launch_bounds__(kBwdBlock, 2) sweep_backward_references_kernel
         const int kx = __shfl_up_sync(0xffffffffu, tx, 1), ky = __shfl_up_sync(0xffffffffu, ty, 1);
         const int ks = __shfl_up_sync(0xffffffffu, key, 1);
         const bool from_left = (lane & 7) != 0 && lands && ks == key && ky == ty && kx + 1 == tx;
+        const int left_sign = __shfl_up_sync(0xffffffffu, sign, 1);
+        long long ql[2][3];
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
+        for (int a = 0; a < 2; ++a) {
+            const long long t = shfl_up64(right[a], 1);
 #pragma unroll
             for (int ch = 0; ch < 3; ++ch) {
-                const long long t = shfl_up64(qr[a][ch], 1);
-                if (from_left) ql[a][ch] += t;
+                ql[a][ch] = signed_part(left[a], sign, ch);
+                if (from_left) ql[a][ch] += signed_part(t, left_sign, ch);
             }
+        }
         const int right_took = __shfl_down_sync(0xffffffffu, (int)from_left, 1);  // every lane shuffles
         const bool given = (lane & 7) != 7 && right_took != 0;
         const int vx = __shfl_up_sync(0xffffffffu, tx, 8), vy = __shfl_up_sync(0xffffffffu, ty, 8);
@@ -727,23 +806,22 @@ __global__ void __launch_bounds__(kBwdBlock, 2) sweep_backward_references_kernel
         const int below_took = __shfl_down_sync(0xffffffffu, (int)from_above, 8);
         const bool given_down = lane < 24 && below_took != 0;
         if (lands) {
-            long long* a = gimg + 3 * ((int64_t)ty * p.cols + tx);
-            const int64_t pitch = 3 * (int64_t)p.cols;
+            long long* a = gimg + ((int64_t)ty * p.cols + tx);
 #pragma unroll
-            for (int ch = 0; ch < 3; ++ch) {
-                fixed_add(a + ch, ql[0][ch]);
-                if (!given_down) fixed_add(a + pitch + ch, ql[1][ch]);
+            for (int ch = 0; ch < 3; ++ch, a += P) {
+                fixed_add(a, ql[0][ch]);
+                if (!given_down) fixed_add(a + p.cols, ql[1][ch]);
                 if (!given) {
-                    fixed_add(a + 3 + ch, qr[0][ch]);
-                    fixed_add(a + pitch + 3 + ch, qr[1][ch]);
+                    fixed_add(a + 1, signed_part(right[0], sign, ch));
+                    fixed_add(a + p.cols + 1, signed_part(right[1], sign, ch));
                 }
             }
         }
     }
     if (active) {
-        long long* gr = image_acc + ((int64_t)reference * P + i) * 3;
+        long long* gr = image_acc + (int64_t)reference * 3 * P + i;
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch) fixed_add(gr + ch, fixed_of(gref[ch] * scale));
+        for (int ch = 0; ch < 3; ++ch) fixed_add(gr + ch * P, fixed_of(gref[ch] * scale));
     }
     // the pose gradient of the block, per camera: a pixel's candidates were summed in float32; pixels
     // are summed in float64 in a fixed order over the lanes of a warp, and the warps in order
@@ -785,26 +863,32 @@ struct GradTargets {
 };
 
 // grad_images[c] += the references' sums in order, image_acc * 2^-e each (NaN where a reference's
-// incoming gradient was not finite)
+// incoming gradient was not finite).  image_acc: channels in planes, so that what a warp adds at
+// neighbouring texels lies in one sector.  blockIdx.y: camera
 __global__ void __launch_bounds__(kBwdBlock) image_grad_references_kernel(const long long* __restrict__ image_acc,
-                                                                          int64_t per_camera, int cameras,
-                                                                          int references,
+                                                                          int64_t pixels, int cameras, int references,
                                                                           const uint32_t* __restrict__ absmax,
                                                                           double count,
                                                                           const __grid_constant__ GradTargets out)
 {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= per_camera) return;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= pixels) return;
     const int c = blockIdx.y;
-    float v = out.ptr[c][e];
+    float* o = out.ptr[c] + 3 * i;
+    float v[3] = {o[0], o[1], o[2]};
     for (int r = 0; r < references; ++r) {
         const float scale = fixed_scale(absmax[r], count);
         const float inv = scale > 0.0f ? 1.0f / scale : 0.0f;  // a power of two: exact
-        const long long q = image_acc[((int64_t)r * cameras + c) * per_camera + e];
-        if (!(__uint_as_float(absmax[r]) <= 3.0e38f)) v = __int_as_float(0x7FFFFFFF);
-        else if (q) v += float_of(q) * inv;
+        const bool finite = __uint_as_float(absmax[r]) <= 3.0e38f;
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+            const long long q = image_acc[(((int64_t)r * cameras + c) * 3 + ch) * pixels + i];
+            if (!finite) v[ch] = __int_as_float(0x7FFFFFFF);
+            else if (q) v[ch] += float_of(q) * inv;
+        }
     }
-    out.ptr[c][e] = v;
+#pragma unroll
+    for (int ch = 0; ch < 3; ++ch) o[ch] = v[ch];
 }
 
 // grad_pose[c][j] += the block sums: 256 threads' shares in a fixed order.  blockIdx.x: 6 c + j
@@ -937,8 +1021,7 @@ extern "C" int ssg_isb_filter_transpose(uint8_t* const* d_guides, uint8_t* const
     for (int s = 0; s + 1 < level_count && s < first; ++s) {
         const LevelGeom g = pair(s);
         isb_up_transpose_table_kernel<<<dim3(grid_1d((int64_t)g.rows_in * g.cols_in, 32), instances), kTransposeBlock, 0, st>>>(
-            d_tables + T.offset[s], T.stride, g, candidate_count, c.weight_up[s], d_grad_filtered[s], d_grad_costs[s],
-            d_grad_filtered[s + 1]);
+            d_tables + T.offset[s], T.stride, g, candidate_count, d_grad_filtered[s], d_grad_filtered[s + 1]);
         if (int err = launch_status("isb_up_transpose_table_kernel")) return err;
     }
     if (first < level_count) {
@@ -959,9 +1042,12 @@ extern "C" int ssg_isb_filter_transpose(uint8_t* const* d_guides, uint8_t* const
         const LevelGeom g = pair(s - 1);
         // f = c at the coarsest level
         const float* coarse = s == level_count - 1 && first == level_count ? d_grad_filtered[s] : d_grad_costs[s];
-        isb_down_transpose_table_kernel<<<dim3(grid_1d((int64_t)g.rows_out * g.cols_out, 32), instances), kTransposeBlock, 0, st>>>(
-            d_tables + T.offset[s - 1], T.stride, g, candidate_count, coarse, d_grad_costs[s - 1],
-            s == 1 ? d_absmax : nullptr);
+        const dim3 grid(grid_1d((int64_t)g.rows_in * g.cols_in, 32), instances);
+        const bool pairs = g.cols_out % 2 == 0 && (((uintptr_t)d_grad_filtered[s - 1] | (uintptr_t)d_grad_costs[s - 1]) & 7) == 0;
+        const auto kernel = pairs ? isb_down_transpose_table_kernel<true> : isb_down_transpose_table_kernel<false>;
+        kernel<<<grid, kTransposeBlock, 0, st>>>(d_tables + T.offset[s - 1], T.stride, g, candidate_count,
+                                                 c.weight_up[s - 1], d_grad_filtered[s - 1], coarse, d_grad_costs[s - 1],
+                                                 s == 1 ? d_absmax : nullptr);
         if (int err = launch_status("isb_down_transpose_table_kernel")) return err;
     }
     return SSG_OK;
@@ -1035,8 +1121,8 @@ extern "C" int ssg_sweep_backward_references(int cols, int rows, int camera_coun
             d_absmax + r0, image_acc + r0 * camera_count * P * 3, pose_partial + r0 * blocks * camera_count * 6);
         if (int err = launch_status("sweep_backward_references_kernel")) return err;
     }
-    image_grad_references_kernel<<<dim3(grid_1d(P * 3, kBwdBlock), camera_count), kBwdBlock, 0, st>>>(
-        image_acc, P * 3, camera_count, reference_count, d_absmax, 2.0 * (double)P * candidate_count, out);
+    image_grad_references_kernel<<<dim3(grid_1d(P, kBwdBlock), camera_count), kBwdBlock, 0, st>>>(
+        image_acc, P, camera_count, reference_count, d_absmax, 2.0 * (double)P * candidate_count, out);
     if (int err = launch_status("image_grad_references_kernel")) return err;
     pose_grad_references_kernel<<<camera_count * 6, kBwdBlock, 0, st>>>(pose_partial, blocks * reference_count,
                                                                        camera_count, d_grad_pose);

@@ -78,7 +78,7 @@ Knob g_knobs[] = {
     {kMergeFramesValues, 3, {4}},  // SSG_TUNE_MERGE_FRAMES
     {kUnevenSpans, 3, {1}},        // SSG_TUNE_UNEVEN_SPAN
     {kIsbUpBlocks, 2, {2}},        // SSG_TUNE_ISB_UP_BLOCKS
-    {kIsbUpBlocks, 2, {2}},        // SSG_TUNE_ISB_SELECT_BLOCKS
+    {kIsbUpBlocks, 2, {3}},        // SSG_TUNE_ISB_SELECT_BLOCKS
     {kOnOff, 2, {0}},              // SSG_TUNE_ISB_TILE_TMA
     {kOnOff, 2, {0}},              // SSG_TUNE_TMA_WITHHOLD
     {kOnOff, 2, {0}},              // SSG_TUNE_HOLE_PERSISTENT

@@ -645,7 +645,7 @@ __device__ __forceinline__ void project_jacobian_packed(const float p[3], const 
 // A block takes 32 x 8 pixels of one reference (blockIdx.z), a warp 8 x 4 of them: the samples of
 // neighbouring pixels land on neighbouring texels, and what two lanes have for one texel is added in
 // the warp.  Per pixel the candidates are taken in order (the float32 sums of the pose gradient).
-__global__ void __launch_bounds__(kBwdBlock, 2) sweep_backward_references_kernel(
+__global__ void __launch_bounds__(kBwdBlock, 3) sweep_backward_references_kernel(
     const __grid_constant__ SweepBwdReferences p, const float4* __restrict__ packed, const int8_t* __restrict__ selected,
     const float* __restrict__ grad_cost, const uint32_t* __restrict__ absmax, long long* __restrict__ image_acc,
     double* __restrict__ pose_partial)

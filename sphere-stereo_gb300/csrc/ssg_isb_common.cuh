@@ -386,6 +386,56 @@ struct Selector {
     }
 };
 
+// least / greatest of three, a NaN left out as fminf and fmaxf do (one instruction from sm_100 on)
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Selector taking four consecutive candidates at a time: the group of the first strict minimum is
+// kept and searched once, at the end (13 comparisons and selections a group instead of 24 to 28).
+// Candidates that do not exist are pushed as NaN, which changes neither minimum nor maximum; the
+// values they give to R belong to a minimum at the last candidate, where R is not used.
+struct GroupSelector {
+    float m = __builtin_huge_valf(), M = -__builtin_huge_valf(), before = 0.0f, after = 0.0f, prev = 0.0f;
+    float b[4] = {__builtin_huge_valf(), 0.0f, 0.0f, 0.0f};
+    int group = 0;
+    bool last = false;  // the minimum's group is the last one taken
+    __device__ __forceinline__ void push(int g, const float (&c)[4])
+    {
+        after = last ? c[0] : after;
+        const float low = fminf(min3(c[0], c[1], c[2]), c[3]);
+        last = low < m;
+        m = fminf(low, m);
+        M = max3(max3(c[0], c[1], c[2]), c[3], M);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = last ? c[j] : b[j];
+        before = last ? prev : before;
+        group = last ? g : group;
+        prev = c[3];
+    }
+    __device__ __forceinline__ Selector whole() const
+    {
+        Selector s;
+        const int j = b[0] == m ? 0 : b[1] == m ? 1 : b[2] == m ? 2 : 3;
+        s.m = m;
+        s.M = M;
+        s.idx = 4 * group + j;
+        s.L = j == 0 ? before : j == 1 ? b[0] : j == 2 ? b[1] : b[2];
+        s.R = j == 0 ? b[1] : j == 1 ? b[2] : j == 2 ? b[3] : after;
+        s.need_right = j == 3 && last;
+        return s;
+    }
+};
+
 // depth_estimation.py:188-198
 __device__ __forceinline__ float select_from(Selector s, int ncand, float d0, float dl, float q)
 {

@@ -76,7 +76,7 @@ typedef struct {
                                          3 = 128 x 7 (72 registers) */
 #define SSG_TUNE_HOLE_BLOCKS_PER_SM 1 /* blocks per SM of the hole-filling steps: 2, 4, 8 */
 #define SSG_TUNE_MERGE_FRAMES 2       /* frames one thread of the batched merge handles: 2, 4, 8 */
-#define SSG_TUNE_UNEVEN_SPAN 3        /* 256-pixel tiles per work item of the uneven sweep: 1, 2, 4 */
+#define SSG_TUNE_UNEVEN_SPAN 3        /* 128-pixel tiles per work item of the uneven sweep: 1, 2, 4 */
 #define SSG_TUNE_ISB_UP_BLOCKS 4      /* blocks per SM the chunked ISB upsampling (coarse levels) is
                                          register-bounded for: 2, 3 */
 #define SSG_TUNE_ISB_SELECT_BLOCKS 5  /* the same for the last level fused with the selection: 2, 3 */
@@ -614,7 +614,7 @@ SSG_API int ssg_sweep_backward_references(int cols, int rows, int camera_count, 
  * Uneven batches (no counterpart in the reference, which estimates one rig's frame per call of
  * estimate_RGBD_panorama, python/depth_estimation.py:205-242): many RGB-D panorama jobs of
  * different rigs, matching resolutions and candidate counts in one fixed sequence of launches --
- * one persistent sweep launch over every instance (a work queue of 256-pixel tiles, largest
+ * one persistent sweep launch over every instance (a work queue of 128-pixel tiles, largest
  * instances first), one launch per cost-filter step, one fused selection, one launch per
  * post-filter step, then fill, reprojection, hole filling and merge over every job.  The 16-bit
  * path's arithmetic (ssg_sweep_cost_batch, ssg_isb_*_batch, ssg_merge_panorama_batch_approx).

@@ -73,9 +73,9 @@ constexpr int kHoleTail[] = {0, 3, 4, 6, 8};
 constexpr int kIsbTail[] = {0, 256, 1024, 4096};
 constexpr int kPostTail[] = {0, 1024, 4096, 16384};
 Knob g_knobs[] = {
-    {kSweepVariants, 4, {0}},      // SSG_TUNE_SWEEP_VARIANT
+    {kSweepVariants, 4, {3}},      // SSG_TUNE_SWEEP_VARIANT
     {kHoleBlocks, 3, {4}},         // SSG_TUNE_HOLE_BLOCKS_PER_SM
-    {kMergeFramesValues, 3, {4}},  // SSG_TUNE_MERGE_FRAMES
+    {kMergeFramesValues, 3, {2}},  // SSG_TUNE_MERGE_FRAMES
     {kUnevenSpans, 3, {1}},        // SSG_TUNE_UNEVEN_SPAN
     {kIsbUpBlocks, 2, {2}},        // SSG_TUNE_ISB_UP_BLOCKS
     {kIsbUpBlocks, 2, {3}},        // SSG_TUNE_ISB_SELECT_BLOCKS

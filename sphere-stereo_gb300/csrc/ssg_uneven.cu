@@ -2,7 +2,7 @@
 // counts in one sequence of launches (no counterpart in the reference, which runs one rig's frame
 // per call of estimate_RGBD_panorama, python/depth_estimation.py:205-242).
 //
-//   sweep + cost           one persistent launch: a work queue of 256-pixel tiles over every
+//   sweep + cost           one persistent launch: a work queue of 128-pixel tiles over every
 //                          instance, largest instances first
 //   cost filter            one launch per pyramid step over the instances that have the step
 //   selection              one launch (the last up step, fused), writing the raw and the

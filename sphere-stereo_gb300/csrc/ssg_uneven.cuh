@@ -9,7 +9,7 @@
 
 namespace ssg {
 
-constexpr int kSweepTile = kBatchBlock;  // reference pixels per work item of the persistent sweep
+constexpr int kSweepTile = 128;  // reference pixels per work item of the persistent sweep
 
 // One instance of the persistent sweep.  Instances are ordered by decreasing work
 // (pixels x chunks) and tile_begin is the prefix of their tile counts, so the work queue hands

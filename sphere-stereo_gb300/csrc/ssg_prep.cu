@@ -13,14 +13,12 @@
 //     there): floats (a + b + c + d) * 0.25, bytes (a + b + c + d + 2) >> 2.
 // cv2 is not available here, so these statements are not pinned against OpenCV's own outputs.
 #include <cmath>
+#include <type_traits>
 
 #include "ssg_common.cuh"
 #include "ssg_resize.cuh"
 
 namespace ssg {
-
-__device__ __forceinline__ float in_value(const float* s, int64_t i) { return __ldg(s + i); }
-__device__ __forceinline__ float in_value(const uint8_t* s, int64_t i) { return (float)__ldg(s + i); }
 
 __device__ __forceinline__ int fixed_weight(float f)
 {
@@ -28,65 +26,136 @@ __device__ __forceinline__ int fixed_weight(float f)
     return min(max(__float2int_rn(w), -32768), 32767);
 }
 
-// One block per kTileX x kTileY destination pixels of one image (blockIdx.z): the tile's column
-// and row taps are formed once (in double, as OpenCV forms its tables) into shared memory, then
-// one thread per destination pixel (all channels) blends.
-constexpr int kTileX = 32, kTileY = 8;
+// A thread takes four consecutive values of a destination row (one 16-byte store of floats) and runs
+// down kResizeRows rows; a block takes kResizeThreads of them, whose column taps are formed once (in
+// double, as OpenCV forms its tables, and FP64 is slow).  A source row blended for one destination
+// row is kept for the next one that reads it.  Bound by the bytes it writes and reads: 4 x 1216 x 1216
+// pixels of 3 bytes to 1024 x 1024 floats are 68 MB, 10 us of the copy bandwidth.  (A thread per
+// pixel, blocks of 32 x 8: 41 us, with three-float strided stores and taps formed per 256 pixels.)
+constexpr int kResizeThreads = 192, kResizeRows = 16;
+constexpr int kResizeValues = 4 * kResizeThreads;  // of a row, per block: whole pixels of 1, 2, 3 or 4 channels
 
-template <typename Tin, typename Tout>
-__global__ void __launch_bounds__(kTileX * kTileY) resize_linear_kernel(const __grid_constant__ ResizeParams p,
-                                                                        const Tin* __restrict__ src,
-                                                                        Tout* __restrict__ dst)
+// four values of one source row, blended along the row
+template <typename Tin, typename H>
+__device__ __forceinline__ void blend_row(const Tin* __restrict__ row, const int64_t (&at)[4], const int (&step)[4],
+                                          const H (&a0)[4], const H (&a1)[4], H (&h)[4])
 {
-    __shared__ Tap cols_tap[kTileX], rows_tap[kTileY];
-    const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY;
-    const int C = p.channels;
-    src += (int64_t)blockIdx.z * p.src_cols * p.src_rows * C;
-    dst += (int64_t)blockIdx.z * p.dst_cols * p.dst_rows * C;
-    if (!p.area2) {
-        if (threadIdx.x < kTileX) cols_tap[threadIdx.x] = column_tap(p, min(x0 + (int)threadIdx.x, p.dst_cols - 1));
-        else if (threadIdx.x < kTileX + kTileY)
-            rows_tap[threadIdx.x - kTileX] = row_tap(p, min(y0 + (int)threadIdx.x - kTileX, p.dst_rows - 1));
-        __syncthreads();
+    Tin v0[4], v1[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        v0[j] = __ldg(row + at[j]);
+        v1[j] = __ldg(row + at[j] + step[j]);
     }
-    const int dx = x0 + (int)(threadIdx.x % kTileX), dy = y0 + (int)(threadIdx.x / kTileX);
-    if (dx >= p.dst_cols || dy >= p.dst_rows) return;
-    dst += ((int64_t)dy * p.dst_cols + dx) * C;
-    if (p.area2) {
-        const int64_t r0 = (int64_t)(2 * dy) * p.src_cols, r1 = r0 + p.src_cols;
-        for (int c = 0; c < C; ++c) {
-            const int64_t a = (r0 + 2 * dx) * C + c, b = a + C, d0 = (r1 + 2 * dx) * C + c, d1 = d0 + C;
-            if constexpr (sizeof(Tout) == 1) {
-                const int s = (int)__ldg(src + a) + __ldg(src + b) + __ldg(src + d0) + __ldg(src + d1);
-                dst[c] = (Tout)((s + 2) >> 2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if constexpr (sizeof(H) == 4 && std::is_same<H, int>::value) h[j] = (int)v0[j] * a0[j] + (int)v1[j] * a1[j];
+        else h[j] = __fadd_rn(__fmul_rn((float)v0[j], a0[j]), __fmul_rn((float)v1[j], a1[j]));
+    }
+}
+
+template <typename Tout, bool kVector>
+__device__ __forceinline__ void store_values(Tout* __restrict__ dst, const Tout (&v)[4], int n)
+{
+    if constexpr (kVector) {
+        if constexpr (sizeof(Tout) == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        else *reinterpret_cast<uchar4*>(dst) = make_uchar4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < n) dst[j] = v[j];
+    }
+}
+
+// blockIdx.x: kResizeValues values of a row; blockIdx.y: kResizeRows rows; blockIdx.z: image.
+// kVector: rows of a multiple of four values, dst aligned to four of them.
+template <typename Tin, typename Tout, bool kArea, bool kVector>
+__global__ void __launch_bounds__(kResizeThreads) resize_linear_kernel(const __grid_constant__ ResizeParams p,
+                                                                      const Tin* __restrict__ src,
+                                                                      Tout* __restrict__ dst)
+{
+    using H = std::conditional_t<sizeof(Tout) == 1, int, float>;  // a row's blended value
+    __shared__ Tap cols_tap[kResizeValues], rows_tap[kResizeRows];
+    const int C = p.channels, pixels = kResizeValues / C;
+    const int64_t x0 = (int64_t)blockIdx.x * pixels;  // the block's first pixel
+    const int y0 = blockIdx.y * kResizeRows;
+    const int64_t values = (int64_t)p.dst_cols * C, pitch = (int64_t)p.src_cols * C;
+    for (int k = threadIdx.x; k < pixels && x0 + k < p.dst_cols; k += kResizeThreads)
+        cols_tap[k] = column_tap(p, (int)(x0 + k));
+    if (threadIdx.x < kResizeRows) rows_tap[threadIdx.x] = row_tap(p, min(y0 + (int)threadIdx.x, p.dst_rows - 1));
+    __syncthreads();
+    const int64_t e = x0 * C + 4 * threadIdx.x;
+    if (e >= values) return;
+    const int n = (int)(values - e < 4 ? values - e : 4);
+    src += (int64_t)blockIdx.z * p.src_rows * pitch;
+    dst += ((int64_t)blockIdx.z * p.dst_rows + y0) * values + e;
+    int64_t at[4];
+    int step[4];
+    H a0[4], a1[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int k = 4 * threadIdx.x + min(j, n - 1), px = k / C;
+        const Tap t = cols_tap[px];
+        at[j] = (int64_t)t.s0 * C + (k - px * C);
+        step[j] = (t.s1 - t.s0) * C;
+        if constexpr (std::is_same<H, int>::value) {
+            a0[j] = fixed_weight(t.f);
+            a1[j] = 2048 - a0[j];
+        } else {
+            a0[j] = __fsub_rn(1.0f, t.f);
+            a1[j] = t.f;
+        }
+    }
+    const int rows = min(kResizeRows, p.dst_rows - y0);
+    H h0[4], h1[4];
+    int have = -1;  // the source row that h1 is of
+    for (int r = 0; r < rows; ++r, dst += values) {
+        const Tap ty = rows_tap[r];
+        const Tin* top = src + ty.s0 * pitch;
+        const Tin* bottom = src + ty.s1 * pitch;
+        Tout out[4];
+        if constexpr (kArea) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const Tin a = __ldg(top + at[j]), b = __ldg(top + at[j] + step[j]);
+                const Tin c = __ldg(bottom + at[j]), d = __ldg(bottom + at[j] + step[j]);
+                if constexpr (std::is_same<H, int>::value) out[j] = (Tout)(((int)a + b + c + d + 2) >> 2);
+                else out[j] = __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn((float)a, (float)b), (float)c), (float)d), 0.25f);
+            }
+        } else {
+            if (ty.s0 == have) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) h0[j] = h1[j];
             } else {
-                const float s = __fadd_rn(__fadd_rn(__fadd_rn(in_value(src, a), in_value(src, b)), in_value(src, d0)),
-                                          in_value(src, d1));
-                dst[c] = __fmul_rn(s, 0.25f);
+                blend_row<Tin, H>(top, at, step, a0, a1, h0);
+            }
+            blend_row<Tin, H>(bottom, at, step, a0, a1, h1);
+            have = ty.s1;
+            if constexpr (std::is_same<H, int>::value) {
+                const int b0 = fixed_weight(ty.f), b1 = 2048 - b0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    out[j] = (Tout)min(max((h0[j] * b0 + h1[j] * b1 + (1 << 21)) >> 22, 0), 255);
+            } else {
+                const float b0 = __fsub_rn(1.0f, ty.f), b1 = ty.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) out[j] = __fadd_rn(__fmul_rn(h0[j], b0), __fmul_rn(h1[j], b1));
             }
         }
-        return;
+        store_values<Tout, kVector>(dst, out, n);
     }
-    const Tap tx = cols_tap[threadIdx.x % kTileX], ty = rows_tap[threadIdx.x / kTileX];
-    const int64_t r0 = (int64_t)ty.s0 * p.src_cols, r1 = (int64_t)ty.s1 * p.src_cols;
-    if constexpr (sizeof(Tout) == 1) {
-        const int a0 = fixed_weight(tx.f), a1 = 2048 - a0, b0 = fixed_weight(ty.f), b1 = 2048 - b0;
-        for (int c = 0; c < C; ++c) {
-            const int h0 = (int)__ldg(src + (r0 + tx.s0) * C + c) * a0 + (int)__ldg(src + (r0 + tx.s1) * C + c) * a1;
-            const int h1 = (int)__ldg(src + (r1 + tx.s0) * C + c) * a0 + (int)__ldg(src + (r1 + tx.s1) * C + c) * a1;
-            const int v = (h0 * b0 + h1 * b1 + (1 << 21)) >> 22;
-            dst[c] = (Tout)min(max(v, 0), 255);
-        }
-    } else {
-        const float a0 = __fsub_rn(1.0f, tx.f), a1 = tx.f, b0 = __fsub_rn(1.0f, ty.f), b1 = ty.f;
-        for (int c = 0; c < C; ++c) {
-            const float h0 = __fadd_rn(__fmul_rn(in_value(src, (r0 + tx.s0) * C + c), a0),
-                                       __fmul_rn(in_value(src, (r0 + tx.s1) * C + c), a1));
-            const float h1 = __fadd_rn(__fmul_rn(in_value(src, (r1 + tx.s0) * C + c), a0),
-                                       __fmul_rn(in_value(src, (r1 + tx.s1) * C + c), a1));
-            dst[c] = __fadd_rn(__fmul_rn(h0, b0), __fmul_rn(h1, b1));
-        }
-    }
+}
+
+template <typename Tin, typename Tout>
+static int launch_resize(const ResizeParams& p, const void* src, void* dst, int images, cudaStream_t st)
+{
+    const int pixels = kResizeValues / p.channels;
+    const dim3 grid((unsigned)(((int64_t)p.dst_cols + pixels - 1) / pixels),
+                    (unsigned)((p.dst_rows + kResizeRows - 1) / kResizeRows), (unsigned)images);
+    const bool vector = (int64_t)p.dst_cols * p.channels % 4 == 0 && ((uintptr_t)dst & (4 * sizeof(Tout) - 1)) == 0;
+    const auto kernel = p.area2 ? (vector ? resize_linear_kernel<Tin, Tout, true, true> : resize_linear_kernel<Tin, Tout, true, false>)
+                                : (vector ? resize_linear_kernel<Tin, Tout, false, true> : resize_linear_kernel<Tin, Tout, false, false>);
+    kernel<<<grid, kResizeThreads, 0, st>>>(p, static_cast<const Tin*>(src), static_cast<Tout*>(dst));
+    return launch_status("resize_linear_kernel");
 }
 
 }  // namespace ssg
@@ -107,19 +176,9 @@ extern "C" int ssg_resize_linear(const void* d_src, int src_type, int src_cols, 
                     (dst_type == SSG_PIXEL_F32 || (dst_type == SSG_PIXEL_U8 && src_type == SSG_PIXEL_U8)),
                 "unsupported pixel types %d -> %d (u8 -> f32, f32 -> f32, u8 -> u8)", src_type, dst_type);
     const ResizeParams p = make_resize_params(src_cols, src_rows, dst_cols, dst_rows, channels);
-    const dim3 grid((unsigned)((dst_cols + kTileX - 1) / kTileX), (unsigned)((dst_rows + kTileY - 1) / kTileY),
-                    (unsigned)images);
-    SSG_REQUIRE(grid.y <= 65535, "destination of %d rows is too tall", dst_rows);
+    SSG_REQUIRE((dst_rows + 7) / 8 <= 65535, "destination of %d rows is too tall", dst_rows);
     cudaStream_t st = as_stream(stream);
-    constexpr int kThreads = kTileX * kTileY;
-    if (src_type == SSG_PIXEL_F32)
-        resize_linear_kernel<float, float>
-            <<<grid, kThreads, 0, st>>>(p, static_cast<const float*>(d_src), static_cast<float*>(d_dst));
-    else if (dst_type == SSG_PIXEL_F32)
-        resize_linear_kernel<uint8_t, float>
-            <<<grid, kThreads, 0, st>>>(p, static_cast<const uint8_t*>(d_src), static_cast<float*>(d_dst));
-    else
-        resize_linear_kernel<uint8_t, uint8_t>
-            <<<grid, kThreads, 0, st>>>(p, static_cast<const uint8_t*>(d_src), static_cast<uint8_t*>(d_dst));
-    return launch_status("resize_linear_kernel");
+    if (src_type == SSG_PIXEL_F32) return launch_resize<float, float>(p, d_src, d_dst, images, st);
+    if (dst_type == SSG_PIXEL_F32) return launch_resize<uint8_t, float>(p, d_src, d_dst, images, st);
+    return launch_resize<uint8_t, uint8_t>(p, d_src, d_dst, images, st);
 }

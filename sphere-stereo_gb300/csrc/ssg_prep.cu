@@ -29,29 +29,39 @@ __device__ __forceinline__ int fixed_weight(float f)
 // A thread takes four consecutive values of a destination row (one 16-byte store of floats) and runs
 // down kResizeRows rows; a block takes kResizeThreads of them, whose column taps are formed once (in
 // double, as OpenCV forms its tables, and FP64 is slow).  A source row blended for one destination
-// row is kept for the next one that reads it.  Bound by the bytes it writes and reads: 4 x 1216 x 1216
-// pixels of 3 bytes to 1024 x 1024 floats are 68 MB, 10 us of the copy bandwidth.  (A thread per
-// pixel, blocks of 32 x 8: 41 us, with three-float strided stores and taps formed per 256 pixels.)
-constexpr int kResizeThreads = 192, kResizeRows = 16;
+// row is kept for the next one that reads it, and a row's bytes are asked for while the row before is
+// blended.  4 x 1216 x 1216 pixels of 3 bytes to 1024 x 1024 floats, 68 MB read and written (10 us of
+// the copy bandwidth): 25.4 us, bound by the latency of its loads, at about a third of the issue rate; 27.5 us
+// with 16 rows, 28 us without asking ahead; 41 us with a thread per pixel in blocks of 32 x 8, which
+// stored floats 12 bytes apart.
+constexpr int kResizeThreads = 192, kResizeRows = 8;
 constexpr int kResizeValues = 4 * kResizeThreads;  // of a row, per block: whole pixels of 1, 2, 3 or 4 channels
 
-// four values of one source row, blended along the row
-template <typename Tin, typename H>
-__device__ __forceinline__ void blend_row(const Tin* __restrict__ row, const int64_t (&at)[4], const int (&step)[4],
-                                          const H (&a0)[4], const H (&a1)[4], H (&h)[4])
-{
+// four values of one source row, as read: both taps of each
+template <typename Tin>
+struct RowTaps {
     Tin v0[4], v1[4];
+    template <typename I>
+    __device__ __forceinline__ void load(const Tin* __restrict__ row, const I (&at)[4], const int (&step)[4])
+    {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        v0[j] = __ldg(row + at[j]);
-        v1[j] = __ldg(row + at[j] + step[j]);
+        for (int j = 0; j < 4; ++j) {
+            v0[j] = __ldg(row + at[j]);
+            v1[j] = __ldg(row + at[j] + step[j]);
+        }
     }
+    // blended along the row
+    __device__ __forceinline__ void blend(const int (&a0)[4], const int (&a1)[4], int (&h)[4]) const
+    {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if constexpr (sizeof(H) == 4 && std::is_same<H, int>::value) h[j] = (int)v0[j] * a0[j] + (int)v1[j] * a1[j];
-        else h[j] = __fadd_rn(__fmul_rn((float)v0[j], a0[j]), __fmul_rn((float)v1[j], a1[j]));
+        for (int j = 0; j < 4; ++j) h[j] = (int)v0[j] * a0[j] + (int)v1[j] * a1[j];
     }
-}
+    __device__ __forceinline__ void blend(const float (&a0)[4], const float (&a1)[4], float (&h)[4]) const
+    {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) h[j] = __fadd_rn(__fmul_rn((float)v0[j], a0[j]), __fmul_rn((float)v1[j], a1[j]));
+    }
+};
 
 template <typename Tout, bool kVector>
 __device__ __forceinline__ void store_values(Tout* __restrict__ dst, const Tout (&v)[4], int n)
@@ -67,8 +77,9 @@ __device__ __forceinline__ void store_values(Tout* __restrict__ dst, const Tout 
 }
 
 // blockIdx.x: kResizeValues values of a row; blockIdx.y: kResizeRows rows; blockIdx.z: image.
+// I: holds a source row's values (int below 2^31, else int64_t).
 // kVector: rows of a multiple of four values, dst aligned to four of them.
-template <typename Tin, typename Tout, bool kArea, bool kVector>
+template <typename Tin, typename Tout, typename I, bool kArea, bool kVector>
 __global__ void __launch_bounds__(kResizeThreads) resize_linear_kernel(const __grid_constant__ ResizeParams p,
                                                                       const Tin* __restrict__ src,
                                                                       Tout* __restrict__ dst)
@@ -79,6 +90,7 @@ __global__ void __launch_bounds__(kResizeThreads) resize_linear_kernel(const __g
     const int64_t x0 = (int64_t)blockIdx.x * pixels;  // the block's first pixel
     const int y0 = blockIdx.y * kResizeRows;
     const int64_t values = (int64_t)p.dst_cols * C, pitch = (int64_t)p.src_cols * C;
+    src += (int64_t)blockIdx.z * p.src_rows * pitch;
     for (int k = threadIdx.x; k < pixels && x0 + k < p.dst_cols; k += kResizeThreads)
         cols_tap[k] = column_tap(p, (int)(x0 + k));
     if (threadIdx.x < kResizeRows) rows_tap[threadIdx.x] = row_tap(p, min(y0 + (int)threadIdx.x, p.dst_rows - 1));
@@ -86,16 +98,15 @@ __global__ void __launch_bounds__(kResizeThreads) resize_linear_kernel(const __g
     const int64_t e = x0 * C + 4 * threadIdx.x;
     if (e >= values) return;
     const int n = (int)(values - e < 4 ? values - e : 4);
-    src += (int64_t)blockIdx.z * p.src_rows * pitch;
     dst += ((int64_t)blockIdx.z * p.dst_rows + y0) * values + e;
-    int64_t at[4];
+    I at[4];
     int step[4];
     H a0[4], a1[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int k = 4 * threadIdx.x + min(j, n - 1), px = k / C;
         const Tap t = cols_tap[px];
-        at[j] = (int64_t)t.s0 * C + (k - px * C);
+        at[j] = (I)t.s0 * C + (k - px * C);
         step[j] = (t.s1 - t.s0) * C;
         if constexpr (std::is_same<H, int>::value) {
             a0[j] = fixed_weight(t.f);
@@ -106,42 +117,51 @@ __global__ void __launch_bounds__(kResizeThreads) resize_linear_kernel(const __g
         }
     }
     const int rows = min(kResizeRows, p.dst_rows - y0);
+    // a row's taps are asked for while the row before is blended
     H h0[4], h1[4];
-    int have = -1;  // the source row that h1 is of
+    RowTaps<Tin> top, bottom, next_top, next_bottom;
+    top.load(src + rows_tap[0].s0 * pitch, at, step);
+    bottom.load(src + rows_tap[0].s1 * pitch, at, step);
+    bool kept = false;  // the row's upper source row is the lower one of the row before: h1
     for (int r = 0; r < rows; ++r, dst += values) {
-        const Tap ty = rows_tap[r];
-        const Tin* top = src + ty.s0 * pitch;
-        const Tin* bottom = src + ty.s1 * pitch;
+        bool keep = false;
+        if (r + 1 < rows) {
+            keep = !kArea && rows_tap[r + 1].s0 == rows_tap[r].s1;
+            if (!keep) next_top.load(src + rows_tap[r + 1].s0 * pitch, at, step);
+            next_bottom.load(src + rows_tap[r + 1].s1 * pitch, at, step);
+        }
         Tout out[4];
         if constexpr (kArea) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const Tin a = __ldg(top + at[j]), b = __ldg(top + at[j] + step[j]);
-                const Tin c = __ldg(bottom + at[j]), d = __ldg(bottom + at[j] + step[j]);
+                const Tin a = top.v0[j], b = top.v1[j], c = bottom.v0[j], d = bottom.v1[j];
                 if constexpr (std::is_same<H, int>::value) out[j] = (Tout)(((int)a + b + c + d + 2) >> 2);
                 else out[j] = __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn((float)a, (float)b), (float)c), (float)d), 0.25f);
             }
         } else {
-            if (ty.s0 == have) {
+            const float f = rows_tap[r].f;
+            if (kept) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) h0[j] = h1[j];
             } else {
-                blend_row<Tin, H>(top, at, step, a0, a1, h0);
+                top.blend(a0, a1, h0);
             }
-            blend_row<Tin, H>(bottom, at, step, a0, a1, h1);
-            have = ty.s1;
+            bottom.blend(a0, a1, h1);
             if constexpr (std::is_same<H, int>::value) {
-                const int b0 = fixed_weight(ty.f), b1 = 2048 - b0;
+                const int b0 = fixed_weight(f), b1 = 2048 - b0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     out[j] = (Tout)min(max((h0[j] * b0 + h1[j] * b1 + (1 << 21)) >> 22, 0), 255);
             } else {
-                const float b0 = __fsub_rn(1.0f, ty.f), b1 = ty.f;
+                const float b0 = __fsub_rn(1.0f, f), b1 = f;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) out[j] = __fadd_rn(__fmul_rn(h0[j], b0), __fmul_rn(h1[j], b1));
             }
         }
         store_values<Tout, kVector>(dst, out, n);
+        kept = keep;
+        top = next_top;
+        bottom = next_bottom;
     }
 }
 
@@ -152,8 +172,13 @@ static int launch_resize(const ResizeParams& p, const void* src, void* dst, int 
     const dim3 grid((unsigned)(((int64_t)p.dst_cols + pixels - 1) / pixels),
                     (unsigned)((p.dst_rows + kResizeRows - 1) / kResizeRows), (unsigned)images);
     const bool vector = (int64_t)p.dst_cols * p.channels % 4 == 0 && ((uintptr_t)dst & (4 * sizeof(Tout) - 1)) == 0;
-    const auto kernel = p.area2 ? (vector ? resize_linear_kernel<Tin, Tout, true, true> : resize_linear_kernel<Tin, Tout, true, false>)
-                                : (vector ? resize_linear_kernel<Tin, Tout, false, true> : resize_linear_kernel<Tin, Tout, false, false>);
+    const bool wide = (int64_t)p.src_cols * p.channels >= ((int64_t)1 << 31) - 4;
+    const auto kernel = wide      ? (p.area2 ? resize_linear_kernel<Tin, Tout, int64_t, true, false>
+                                             : resize_linear_kernel<Tin, Tout, int64_t, false, false>)
+                        : p.area2 ? (vector ? resize_linear_kernel<Tin, Tout, int, true, true>
+                                            : resize_linear_kernel<Tin, Tout, int, true, false>)
+                                  : (vector ? resize_linear_kernel<Tin, Tout, int, false, true>
+                                            : resize_linear_kernel<Tin, Tout, int, false, false>);
     kernel<<<grid, kResizeThreads, 0, st>>>(p, static_cast<const Tin*>(src), static_cast<Tout*>(dst));
     return launch_status("resize_linear_kernel");
 }

@@ -201,8 +201,11 @@ __global__ void __launch_bounds__(kBlock) rgb_to_guide_kernel(const float* __res
 // itself does what sweep_cost_kernel does, value by value (same bits), with its quotients taken
 // from a reciprocal (div_by_reciprocal).
 //
-// Bound by instruction issue and the gathers.  Measured per reference at 1024^2 x 32: 291 us from
-// 12-byte texels, 177 us from packed ones, and 21 us per frame to pack four images.
+// Bound by instruction issue (some 160 a sample) and the gathers, which share what neighbouring rows'
+// samples brought into L1: blocks are tiles of 16 x 16 pixels, four per SM.  Measured per reference at
+// 1024^2 x 32: 291 us from 12-byte texels, 177 us from packed ones in blocks of 256 pixels of a row,
+// 163 us in tiles (164 with 32 x 8, 170 with 8 x 32; 183 with three blocks per SM), and 21 us per
+// frame to pack four images.  Pairs of x and y in packed instructions: 195 us, for their moves.
 // ---------------------------------------------------------------------------------------------
 struct PackParams {
     const float* images[SSG_MAX_CAMERAS];
@@ -225,27 +228,16 @@ __global__ void __launch_bounds__(kBlock) pack_images_kernel(const __grid_consta
         if (p.references[s] == c) guide_of(r, g, b, guides + 3 * (s * P + i));
 }
 
-// sample_rgb on packed texels
-__device__ __forceinline__ void sample_packed(const float4* __restrict__ img, int cols, int rows, float ix, float iy,
-                                              float s[3])
+// sample_rgb on packed texels near the image's edge or outside it
+__device__ __forceinline__ void sample_packed_edge(const float4* __restrict__ img, int cols, int rows, float ix, float iy,
+                                                   float s[3])
 {
     const float x0 = floorf(ix), y0 = floorf(iy);
     const float x1 = fadd(x0, 1.0f), y1 = fadd(y0, 1.0f);
     const float wx0 = fsub(x1, ix), wx1 = fsub(ix, x0), wy0 = fsub(y1, iy), wy1 = fsub(iy, y0);
     const float w[4] = {fmul(wx0, wy0), fmul(wx1, wy0), fmul(wx0, wy1), fmul(wx1, wy1)};
-    s[0] = s[1] = s[2] = 0.0f;
-    if (x0 >= 0.0f && y0 >= 0.0f && x1 < (float)cols && y1 < (float)rows) {
-        const float4* q = img + ((int64_t)(int)y0 * cols + (int)x0);
-        const float4 t[4] = {__ldg(q), __ldg(q + 1), __ldg(q + cols), __ldg(q + cols + 1)};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            s[0] = fadd(s[0], fmul(t[k].x, w[k]));
-            s[1] = fadd(s[1], fmul(t[k].y, w[k]));
-            s[2] = fadd(s[2], fmul(t[k].z, w[k]));
-        }
-        return;
-    }
     const float xs[4] = {x0, x1, x0, x1}, ys[4] = {y0, y0, y1, y1};
+    s[0] = s[1] = s[2] = 0.0f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (xs[k] >= 0.0f && xs[k] < (float)cols && ys[k] >= 0.0f && ys[k] < (float)rows) {
@@ -257,11 +249,41 @@ __device__ __forceinline__ void sample_packed(const float4* __restrict__ img, in
     }
 }
 
+// sample_rgb on packed texels.  Inside (0 <= ix < limit_x and so on: all four taps in the image) the
+// floors are sums with 1.5 x 2^23 rounded down, whose bits are the texel's place, and the sum starts
+// at the first tap (0 + a is a but for the sign of a zero, which the cost does not see).  limit:
+// size - 1, below 0 where the size exceeds 2^22.
+__device__ __forceinline__ void sample_packed(const float4* __restrict__ img, int cols, int rows, float ix, float iy,
+                                              float limit_x, float limit_y, float s[3])
+{
+    if (!(ix >= 0.0f && iy >= 0.0f && ix < limit_x && iy < limit_y)) {
+        sample_packed_edge(img, cols, rows, ix, iy, s);
+        return;
+    }
+    const float mx = __fadd_rd(ix, 12582912.0f), my = __fadd_rd(iy, 12582912.0f);
+    const float4* q = img + ((int64_t)(__float_as_int(my) - 0x4B400000) * cols + (__float_as_int(mx) - 0x4B400000));
+    const float4 t[4] = {__ldg(q), __ldg(q + 1), __ldg(q + cols), __ldg(q + cols + 1)};
+    const float x0 = fsub(mx, 12582912.0f), y0 = fsub(my, 12582912.0f);
+    const float x1 = fadd(x0, 1.0f), y1 = fadd(y0, 1.0f);
+    const float wx0 = fsub(x1, ix), wx1 = fsub(ix, x0), wy0 = fsub(y1, iy), wy1 = fsub(iy, y0);
+    const float w[4] = {fmul(wx0, wy0), fmul(wx1, wy0), fmul(wx0, wy1), fmul(wx1, wy1)};
+    s[0] = fmul(t[0].x, w[0]);
+    s[1] = fmul(t[0].y, w[0]);
+    s[2] = fmul(t[0].z, w[0]);
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+        s[0] = fadd(s[0], fmul(t[k].x, w[k]));
+        s[1] = fadd(s[1], fmul(t[k].y, w[k]));
+        s[2] = fadd(s[2], fmul(t[k].z, w[k]));
+    }
+}
+
+constexpr int kTileX = 16;
 constexpr int kSweepReferences = 4;  // of one launch: bounds the parameters (an upload per launch) to 6 KB
 
 struct SweepReferencesParams {
     int cols, rows, ncam, ncand, ranges;
-    float colsf, rowsf, inv_cols, inv_rows;
+    float colsf, rowsf, inv_cols, inv_rows, limit_x, limit_y;
     int reference[kSweepReferences];
     TorchCam cams[SSG_MAX_CAMERAS];
     float rt[kSweepReferences][SSG_MAX_CAMERAS][12];
@@ -269,14 +291,17 @@ struct SweepReferencesParams {
 };
 
 // blockIdx.y: reference of the launch; blockIdx.z: range of the candidates
-__global__ void __launch_bounds__(kBlock) sweep_references_kernel(const __grid_constant__ SweepReferencesParams p,
+__global__ void __launch_bounds__(kBlock, 4) sweep_references_kernel(const __grid_constant__ SweepReferencesParams p,
                                                                   const float4* __restrict__ packed,
                                                                   const int8_t* __restrict__ selected,
                                                                   float* __restrict__ cost)
 {
     const int64_t P = (int64_t)p.cols * p.rows;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P) return;
+    const int tiles_x = (p.cols + kTileX - 1) / kTileX;
+    const int x = blockIdx.x % tiles_x * kTileX + threadIdx.x % kTileX;
+    const int y = blockIdx.x / tiles_x * (kBlock / kTileX) + threadIdx.x / kTileX;
+    if (x >= p.cols || y >= p.rows) return;
+    const int64_t i = (int64_t)y * p.cols + x;
     const int slot = blockIdx.y, share = (p.ncand + p.ranges - 1) / p.ranges;
     const int k0 = blockIdx.z * share, k1 = min(k0 + share, p.ncand);
     const int reference = p.reference[slot];
@@ -291,7 +316,7 @@ __global__ void __launch_bounds__(kBlock) sweep_references_kernel(const __grid_c
         return;
     }
     float pu[3];
-    unproject_torch((float)(int)(i % p.cols), (float)(int)(i / p.cols), p.cams[reference], pu);
+    unproject_torch((float)x, (float)y, p.cams[reference], pu);
     const TorchCam cam = p.cams[sel];
     float rt[12];
 #pragma unroll
@@ -306,7 +331,7 @@ __global__ void __launch_bounds__(kBlock) sweep_references_kernel(const __grid_c
         project_packed(q, cam, uv);
         const float ix = packed_sample_coord(uv[0], p.colsf, p.inv_cols);
         const float iy = packed_sample_coord(uv[1], p.rowsf, p.inv_rows);
-        sample_packed(img, p.cols, p.rows, ix, iy, s);
+        sample_packed(img, p.cols, p.rows, ix, iy, p.limit_x, p.limit_y, s);
         float c = fadd(fadd(fabsf(fsub(s[0], ref.x)), fabsf(fsub(s[1], ref.y))), fabsf(fsub(s[2], ref.z)));
         c = c > 500.0f ? 500.0f : c;
         *cost = c;
@@ -454,6 +479,9 @@ extern "C" int ssg_sweep_cost_references(int cols, int rows, int camera_count, c
     p.rowsf = (float)rows;
     p.inv_cols = 1.0f / (float)cols;
     p.inv_rows = 1.0f / (float)rows;
+    // the floors of sample_packed hold below 2^22
+    p.limit_x = cols <= (1 << 22) ? (float)(cols - 1) : -1.0f;
+    p.limit_y = rows <= (1 << 22) ? (float)(rows - 1) : -1.0f;
     for (int c = 0; c < camera_count; ++c) p.cams[c] = make_torch_cam(cameras[c]);
     for (int k = 0; k < candidate_count; ++k) p.cand[k] = candidates[k];
     const int64_t P = (int64_t)cols * rows;
@@ -469,7 +497,7 @@ extern "C" int ssg_sweep_cost_references(int cols, int rows, int camera_count, c
         // took 2 x 44 us in a launch each, 31 us in one
         p.ranges = 1;
         while (p.ranges < 4 && P * count * p.ranges < 600000 && candidate_count >= 16 * p.ranges) p.ranges *= 2;
-        sweep_references_kernel<<<dim3(grid_1d(P, kBlock), count, p.ranges), kBlock, 0, as_stream(stream)>>>(
+        sweep_references_kernel<<<dim3(((cols + kTileX - 1) / kTileX) * ((rows + kBlock / kTileX - 1) / (kBlock / kTileX)), count, p.ranges), kBlock, 0, as_stream(stream)>>>(
             p, reinterpret_cast<const float4*>(d_packed), d_selected + r0 * P, d_cost + r0 * P * candidate_count);
         if (int e = launch_status("sweep_references_kernel")) return e;
     }

@@ -1233,22 +1233,6 @@ struct MergeParams {
     float t[SSG_MAX_REFERENCES][3];
 };
 
-// interp (stitcher.cu:56-83) on uint8 RGB
-__device__ __forceinline__ void interp_rgb(const uint8_t* __restrict__ img, float u, float v, int cols, float out[3])
-{
-    const int u1 = __float2int_rd(u), v1 = __float2int_rd(v), u2 = u1 + 1, v2 = v1 + 1;
-    const float w1 = fmul(fsub((float)u2, u), fsub((float)v2, v)), w2 = fmul(fsub((float)u2, u), fsub(v, (float)v1));
-    const float w3 = fmul(fsub(u, (float)u1), fsub((float)v2, v)), w4 = fmul(fsub(u, (float)u1), fsub(v, (float)v1));
-    const uint8_t* p1 = img + 3 * ((int64_t)v1 * cols + u1);
-    const uint8_t* p2 = img + 3 * ((int64_t)v2 * cols + u1);
-    const uint8_t* p3 = img + 3 * ((int64_t)v1 * cols + u2);
-    const uint8_t* p4 = img + 3 * ((int64_t)v2 * cols + u2);
-#pragma unroll
-    for (int ch = 0; ch < 3; ++ch)
-        out[ch] = fadd(fadd(fadd(fmul((float)p1[ch], w1), fmul((float)p2[ch], w2)), fmul((float)p3[ch], w3)),
-                       fmul((float)p4[ch], w4));
-}
-
 // Bilinear sample of a float map and of uint8 RGB (interpF, interp: stitcher.cu:56-116) in
 // fused multiply-adds, for the batched 16-bit path's merge
 __device__ __forceinline__ float interp_f_fast(const float* __restrict__ s, float u, float v, int cols)
@@ -1275,6 +1259,39 @@ __device__ __forceinline__ void texel_pair_words(const uint8_t* p, uint32_t& lo,
     const uint32_t w2 = s == 24 ? __ldg(w + 2) : 0u;
     lo = __funnelshift_r(w0, w1, s);
     hi = __funnelshift_r(w1, w2, s);
+}
+
+// interp (stitcher.cu:56-83) on uint8 RGB; words: the texel pairs are read with texel_pair_words (same
+// values, fewer loads)
+__device__ __forceinline__ void interp_rgb(const uint8_t* __restrict__ img, float u, float v, int cols, float out[3],
+                                           bool words)
+{
+    const int u1 = __float2int_rd(u), v1 = __float2int_rd(v), u2 = u1 + 1, v2 = v1 + 1;
+    const float w1 = fmul(fsub((float)u2, u), fsub((float)v2, v)), w2 = fmul(fsub((float)u2, u), fsub(v, (float)v1));
+    const float w3 = fmul(fsub(u, (float)u1), fsub((float)v2, v)), w4 = fmul(fsub(u, (float)u1), fsub(v, (float)v1));
+    const uint8_t* top = img + 3 * ((int64_t)v1 * cols + u1);
+    const uint8_t* bottom = img + 3 * ((int64_t)v2 * cols + u1);
+    uint32_t t1 = 0, t2 = 0, t3 = 0, t4 = 0;  // the texels' bytes
+    if (words) {
+        uint32_t hi;
+        texel_pair_words(top, t1, hi);
+        t3 = __byte_perm(t1, hi, 0x0543);
+        texel_pair_words(bottom, t2, hi);
+        t4 = __byte_perm(t2, hi, 0x0543);
+    } else {
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+            t1 |= (uint32_t)top[ch] << (8 * ch);
+            t2 |= (uint32_t)bottom[ch] << (8 * ch);
+            t3 |= (uint32_t)top[3 + ch] << (8 * ch);
+            t4 |= (uint32_t)bottom[3 + ch] << (8 * ch);
+        }
+    }
+    const auto byte = [](uint32_t t, int ch) { return (float)((t >> (8 * ch)) & 0xFFu); };
+#pragma unroll
+    for (int ch = 0; ch < 3; ++ch)
+        out[ch] = fadd(fadd(fadd(fmul(byte(t1, ch), w1), fmul(byte(t2, ch), w2)), fmul(byte(t3, ch), w3)),
+                       fmul(byte(t4, ch), w4));
 }
 
 // words: the texel pairs are read with texel_pair_words (same values, fewer loads)
@@ -1334,8 +1351,11 @@ __device__ __forceinline__ void project_fast(const float p[3], const Intr& k, fl
     uv[1] = fmaf(k.fy * p[1], den, k.cy);
 }
 
-// mergeRGBDPanoramaKernel, stitcher.cu:423-473
-__global__ void __launch_bounds__(kStitchBlock) merge_kernel(const __grid_constant__ MergeParams p,
+// mergeRGBDPanoramaKernel, stitcher.cu:423-473.  Bound by instruction issue: the camera model's IEEE
+// divisions and square roots, some 400 instructions a pixel and reference.  2048 x 1024, two
+// references: 65.6 us with byte loads, 63.7 with word loads, 61.9 with eight blocks per SM; 70 with
+// both references in flight.
+__global__ void __launch_bounds__(kStitchBlock, 8) merge_kernel(const __grid_constant__ MergeParams p,
                                                              const float2* __restrict__ lut,
                                                              const float* __restrict__ weights,
                                                              const float* __restrict__ reproj,
@@ -1356,6 +1376,7 @@ __global__ void __launch_bounds__(kStitchBlock) merge_kernel(const __grid_consta
     rgb_pano += frame * Q * 3;
     float inv = 0.0f, rgb[3] = {0.0f, 0.0f, 0.0f};
     const float colsm = fsub((float)p.image_cols, 1.1f), rowsm = fsub((float)p.image_rows, 1.1f);
+#pragma unroll 1
     for (int r = 0; r < p.nref; ++r) {
         const float w = weights[(int64_t)r * Q + i];
         float2 uv = lut[(int64_t)r * Q + i];
@@ -1381,7 +1402,7 @@ __global__ void __launch_bounds__(kStitchBlock) merge_kernel(const __grid_consta
         o[1] = fadd(o[1], (float)(r * p.image_rows));
         float c[3];
         interp_rgb(images + (int64_t)(p.image_slot[r] - r) * p.image_rows * p.image_cols * 3, o[0], o[1],
-                   p.image_cols, c);
+                   p.image_cols, c, p.word_rows);
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) rgb[ch] = fadd(rgb[ch], fmul(c[ch], w));
     }

@@ -284,13 +284,18 @@ __device__ __forceinline__ bool down_reader(const LevelGeom& g, int n, int X, in
     return !none && x < g.cols_in && y < g.rows_in;
 }
 
-constexpr int kTransposeBlock = 256, kTransposeRanges = kTransposeBlock / 32;
+// Threads of a transposed step's block: 8 warps share out the candidates, or 4, which repeat the set-up
+// half as often, where the level has enough groups of 32 cells.  48 candidates, 8 and 4 warps: 4096
+// groups (level 0 of two 512 x 512 references) up 81 and 72 us, down 69 and 53; 1024 groups up 26.2 and
+// 24.8, down 16.4 and 15.5; at 256 groups 4 warps lost 10 and 8 us.
+constexpr int kTransposeBlock = 256, kTransposeFull = 1024;
 
 // Up step transposed: g_f(coarse) = sum over the cell's readers.  (A fine pixel's own part, own weight *
 // g_f(fine), is formed by the down step's kernel, which reads g_f once more instead of adding to a
-// volume written here.)  A block takes 32 coarse cells; its 8 warps share out their weights and then
-// the candidates.  blockIdx.y: instance.
-__global__ void __launch_bounds__(kTransposeBlock) isb_up_transpose_table_kernel(
+// volume written here.)  A block takes 32 coarse cells; its warps share out their weights and then the
+// candidates.  blockIdx.y: instance.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) isb_up_transpose_table_kernel(
     const float* __restrict__ tables, int64_t table_stride, LevelGeom g, int ncand,
     const float* __restrict__ grad_f_fine, float* __restrict__ grad_f_coarse)
 {
@@ -301,10 +306,11 @@ __global__ void __launch_bounds__(kTransposeBlock) isb_up_transpose_table_kernel
     grad_f_fine += inst * ncand * pio;
     grad_f_coarse += inst * ncand * pin;
     const int px = threadIdx.x & 31, range = threadIdx.x >> 5;
+    constexpr int ranges = kThreads / 32;
     const int o = blockIdx.x * 32 + px, oc = min(o, pin - 1);
     const int Y = oc / g.cols_in, X = oc - Y * g.cols_in;
 #pragma unroll 1
-    for (int e = range; e < kEntries; e += kTransposeRanges) {
+    for (int e = range; e < kEntries; e += ranges) {
         const TransposeEntry t = transpose_entry(e);
         sk[e][px] = read_weight(t.f, tables, g, X + t.dx, Y + t.dy, X, Y);
     }
@@ -316,7 +322,7 @@ __global__ void __launch_bounds__(kTransposeBlock) isb_up_transpose_table_kernel
         k[e] = sk[e][px];
         full = full && k[e] != 0.0f;
     }
-    const int share = (ncand + kTransposeRanges - 1) / kTransposeRanges;
+    const int share = (ncand + ranges - 1) / ranges;
     const int z0 = range * share, z1 = min(z0 + share, ncand);
     const int corner = (2 * Y - 2) * g.cols_out + 2 * X - 2;  // of the 5 x 5 fine pixels
     const bool in = o < pin;
@@ -366,8 +372,8 @@ __host__ __device__ constexpr QuadEntry quad_entry(int e)
 }
 constexpr int kQuadEntries = 9;
 
-template <bool kPairs>
-__global__ void __launch_bounds__(kTransposeBlock) isb_down_transpose_table_kernel(
+template <bool kPairs, int kThreads>
+__global__ void __launch_bounds__(kThreads) isb_down_transpose_table_kernel(
     const float* __restrict__ tables, int64_t table_stride, LevelGeom g, int ncand, float weight_up,
     const float* __restrict__ grad_f_fine, const float* __restrict__ grad_c_coarse, float* __restrict__ grad_c_fine,
     uint32_t* __restrict__ absmax)
@@ -376,7 +382,8 @@ __global__ void __launch_bounds__(kTransposeBlock) isb_down_transpose_table_kern
     const int pin = g.rows_in * g.cols_in, pio = g.rows_out * g.cols_out;
     const int64_t inst = blockIdx.y;
     tables += inst * table_stride;
-    const int px = threadIdx.x & 31, range = threadIdx.x >> 5, ranges = blockDim.x >> 5;
+    const int px = threadIdx.x & 31, range = threadIdx.x >> 5;
+    constexpr int ranges = kThreads / 32;
     const int o = blockIdx.x * 32 + px, oc = min(o, pin - 1);
     const int y = oc / g.cols_in, x = oc - y * g.cols_in;
     const bool set1 = 2 * y + 1 < g.rows_out, set2 = 2 * x + 1 < g.cols_out;
@@ -645,7 +652,7 @@ __device__ __forceinline__ void project_jacobian_packed(const float p[3], const 
 // A block takes 32 x 8 pixels of one reference (blockIdx.z), a warp 8 x 4 of them: the samples of
 // neighbouring pixels land on neighbouring texels, and what two lanes have for one texel is added in
 // the warp.  Per pixel the candidates are taken in order (the float32 sums of the pose gradient).
-__global__ void __launch_bounds__(kBwdBlock, 3) sweep_backward_references_kernel(
+__global__ void __launch_bounds__(kBwdBlock, 4) sweep_backward_references_kernel(
     const __grid_constant__ SweepBwdReferences p, const float4* __restrict__ packed, const int8_t* __restrict__ selected,
     const float* __restrict__ grad_cost, const uint32_t* __restrict__ absmax, long long* __restrict__ image_acc,
     double* __restrict__ pose_partial)
@@ -1020,7 +1027,10 @@ extern "C" int ssg_isb_filter_transpose(uint8_t* const* d_guides, uint8_t* const
     const auto pair = [&](int s) { return LevelGeom{T.rows[s + 1], T.cols[s + 1], T.rows[s], T.cols[s]}; };
     for (int s = 0; s + 1 < level_count && s < first; ++s) {
         const LevelGeom g = pair(s);
-        isb_up_transpose_table_kernel<<<dim3(grid_1d((int64_t)g.rows_in * g.cols_in, 32), instances), kTransposeBlock, 0, st>>>(
+        const dim3 grid(grid_1d((int64_t)g.rows_in * g.cols_in, 32), instances);
+        const bool full = (int64_t)grid.x * instances >= kTransposeFull;
+        const auto kernel = full ? isb_up_transpose_table_kernel<kTransposeBlock / 2> : isb_up_transpose_table_kernel<kTransposeBlock>;
+        kernel<<<grid, full ? kTransposeBlock / 2 : kTransposeBlock, 0, st>>>(
             d_tables + T.offset[s], T.stride, g, candidate_count, d_grad_filtered[s], d_grad_filtered[s + 1]);
         if (int err = launch_status("isb_up_transpose_table_kernel")) return err;
     }
@@ -1044,8 +1054,12 @@ extern "C" int ssg_isb_filter_transpose(uint8_t* const* d_guides, uint8_t* const
         const float* coarse = s == level_count - 1 && first == level_count ? d_grad_filtered[s] : d_grad_costs[s];
         const dim3 grid(grid_1d((int64_t)g.rows_in * g.cols_in, 32), instances);
         const bool pairs = g.cols_out % 2 == 0 && (((uintptr_t)d_grad_filtered[s - 1] | (uintptr_t)d_grad_costs[s - 1]) & 7) == 0;
-        const auto kernel = pairs ? isb_down_transpose_table_kernel<true> : isb_down_transpose_table_kernel<false>;
-        kernel<<<grid, kTransposeBlock, 0, st>>>(d_tables + T.offset[s - 1], T.stride, g, candidate_count,
+        const bool full = (int64_t)grid.x * instances >= kTransposeFull;
+        constexpr int kHalf = kTransposeBlock / 2;
+        const auto kernel = full ? (pairs ? isb_down_transpose_table_kernel<true, kHalf> : isb_down_transpose_table_kernel<false, kHalf>)
+                                 : (pairs ? isb_down_transpose_table_kernel<true, kTransposeBlock>
+                                          : isb_down_transpose_table_kernel<false, kTransposeBlock>);
+        kernel<<<grid, full ? kHalf : kTransposeBlock, 0, st>>>(d_tables + T.offset[s - 1], T.stride, g, candidate_count,
                                                  c.weight_up[s - 1], d_grad_filtered[s - 1], coarse, d_grad_costs[s - 1],
                                                  s == 1 ? d_absmax : nullptr);
         if (int err = launch_status("isb_down_transpose_table_kernel")) return err;

@@ -59,7 +59,8 @@ def _per_step(N, isb, sweep, images, rel, grad_q):
 
 
 @pytest.mark.parametrize("cols,rows,n,refs", [(64, 64, 16, [2, 3]), (33, 40, 5, [1]), (97, 75, 17, [0, 1, 2, 3, 1]),
-                                              (130, 66, 9, [3, 0]), (40, 200, 8, [2])])
+                                              (130, 66, 9, [3, 0]), (40, 200, 8, [2]),
+                                              (264, 250, 3, [0, 1, 2, 3, 1]), (263, 251, 5, [0, 1, 2, 3, 1])])
 @pytest.mark.parametrize("finite", [True, False])
 def test_equals_the_per_step_entry_points(ss, native, synthetic, cols, rows, n, refs, finite):
     N = ss._native

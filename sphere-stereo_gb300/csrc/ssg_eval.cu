@@ -93,7 +93,7 @@ struct SquareSum {
 
 // Per-pixel sums: squared colour differences, inverse-distance errors and bad-pixel counts.
 // blockIdx.y: frame.  kVec: the frame's arrays are read 16 bytes at a time (all four 16-byte aligned
-// in every frame).  Bound by memory: 4 frames of 2048x1024 (117 MB) 450 -> 57 us.
+// in every frame).  Bound by instruction issue: 4 frames of 2048x1024 (117 MB) 450 -> 57 us.
 template <bool kVec>
 __global__ void __launch_bounds__(kEvalThreads) eval_pointwise_kernel(const __grid_constant__ EvalParams p,
                                                                       const uint8_t* __restrict__ rgb,

@@ -8,7 +8,7 @@ selection, candidates and stitcher tables come from it).  Per batch:
     ssg_stage_images[_u8]    one launch per job (inputs -> 8-bit footprint planes + guides)
     ssg_uneven_run           one persistent sweep launch over every instance, one launch per
                              cost-filter and post-filter step, the fused selection, then fill,
-                             reprojection, hole lists and merge over every job
+                             reprojection, hole filling and merge over every job
 
 The inputs are written into this object's buffers (``match_inputs`` / ``stitch_inputs``, or
 through ``run``), so the whole sequence is captured once in a CUDA graph and replayed.

@@ -198,6 +198,17 @@ __device__ __forceinline__ float2 load_fine(const float* __restrict__ c, int at,
     else return make_float2(c[at], second ? c[at + 1] : 0.0f);
 }
 
+// How many candidates ahead of its use a step asks for its lines to be brought into L2 (0: not).  Rows
+// read value by value (an odd width) gain by it, the selecting step with registers for 10 blocks of 64
+// threads: 4 x 637 x 479 x 43, level 1 58 -> 49.5 us, selecting level 204 -> 192 us, the frame 938 -> 925 us.
+// Rows read in pairs lose: 1024^2 x 32 filtered 311 -> 316 us, a frame of 2 x 1024^2 x 32 1097 -> 1107 us.
+template <bool kPairs>
+constexpr int kUpAhead = kPairs ? 0 : 4;
+
+// blocks per SM the up step's registers are bounded for
+template <int kRanges, bool kSelect, bool kPairs>
+constexpr int up_blocks = kRanges == 8 ? 2 : (kSelect && !kPairs ? 10 : 12) / kRanges;
+
 // Candidates [k0, k1) of the two fine pixels FA, FB of one fine row of coarse pixel (x, y) in column
 // `px` of sw, filtered; sink.take(k, at, a, b) gets each pair, `at` the pair's place in the level.
 template <int FA, int FB, bool kPairs, typename Sink>
@@ -249,6 +260,12 @@ __device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in,
             }
             va = fmul(va, inv_a);
             vb = fmul(vb, inv_b);
+            constexpr int kAhead = Sink::kAhead;
+            if (kAhead && k + j + kAhead < k1) {
+                if ((px & 15) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(f + (int64_t)kAhead * pio + f0));
+                if (px == 8)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(c + (int64_t)(kAhead - 1) * pin + rr[2] + cc[1]));
+            }
             if (k + j + kUpDepth < k1) own[j] = load_fine<kPairs>(f + (int64_t)kUpDepth * pio, f0, second);
             sink.take(k + j, f0, va, vb);
             f += pio;
@@ -262,6 +279,7 @@ __device__ __forceinline__ void planar_up_row(const float* __restrict__ cost_in,
 // writes the pairs to a level
 template <bool kPairs>
 struct StoreSink {
+    static constexpr int kAhead = kUpAhead<kPairs>;
     float* level;
     int pio;
     bool second;
@@ -278,7 +296,9 @@ struct StoreSink {
 };
 
 // selects among the candidates of a range that starts at k0
+template <bool kPairs>
 struct SelectSink {
+    static constexpr int kAhead = kUpAhead<kPairs>;
     int k0;
     Selector a, b;
     float first_a = 0.0f, first_b = 0.0f;
@@ -329,7 +349,7 @@ __device__ __forceinline__ void planar_setup(const uint8_t* __restrict__ guide_i
 // one of kRanges ranges of candidates.  The filtered fine guide goes to guide_out (guide_fine itself,
 // another pyramid's level, or none).  blockIdx.x: group of coarse pixels; blockIdx.y: instance.
 template <int kRanges, bool kSelect, bool kPairs, typename GL>
-__global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges) isb_up_planar_kernel(
+__global__ void __launch_bounds__(64 * kRanges, up_blocks<kRanges, kSelect, kPairs>) isb_up_planar_kernel(
     const uint8_t* __restrict__ guide_in, const float* __restrict__ cost_in, const uint8_t* guide_fine,
     uint8_t* guide_out, float* cost_io, LevelGeom g, int ncand, float weight_up, float weight_down, float var_inv_i,
     const float* __restrict__ table, SelectOut so)
@@ -355,11 +375,12 @@ __global__ void __launch_bounds__(64 * kRanges, kRanges == 8 ? 2 : 12 / kRanges)
     const bool upper = (warp & 1) == 0;  // the fine row of F = 0, 2, or of F = 1, 3
     if (in && k0 < k1 && (upper || 2 * y + 1 < g.rows_out)) {
         if constexpr (kSelect) {
-            SelectSink sink{k0};
+            using Sink = SelectSink<kPairs>;
+            Sink sink{k0};
             if (upper) planar_up_row<0, 2, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px, sink);
             else planar_up_row<1, 3, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px, sink);
-            part[range][(upper ? 0 : kPx) + px] = SelectSink::range(sink.a, sink.first_a);
-            part[range][(upper ? 2 * kPx : 3 * kPx) + px] = SelectSink::range(sink.b, sink.first_b);
+            part[range][(upper ? 0 : kPx) + px] = Sink::range(sink.a, sink.first_a);
+            part[range][(upper ? 2 * kPx : 3 * kPx) + px] = Sink::range(sink.b, sink.first_b);
         } else {
             StoreSink<kPairs> sink{cost_io, pio, 2 * x + 1 < g.cols_out};
             if (upper) planar_up_row<0, 2, kPairs>(cost_in, cost_io, g, x, y, k0, k1, weight_up, sw, px, sink);

@@ -28,6 +28,7 @@ namespace ssg {
 // a warp per fine row; a pixel's candidates are taken in order (the online softmax).
 // ---------------------------------------------------------------------------------------------
 struct SoftSink {
+    static constexpr int kAhead = 0;
     float inv_tau;
     const float* inv_cand;
     OnlineSoftmax a, b;
@@ -40,6 +41,7 @@ struct SoftSink {
 // the same, keeping the filtered costs in `level` for the second pass
 template <bool kPairs>
 struct SoftKeepSink {
+    static constexpr int kAhead = 0;
     SoftSink soft;
     StoreSink<kPairs> store;
     __device__ __forceinline__ void take(int k, int at, float va, float vb)

@@ -9,7 +9,8 @@
 //     coarse pixel), and the transposed steps read the 25 values that concern a cell;
 //   * the small levels of the transposed filter run in one launch, a block per candidate;
 //   * the 64-bit conversions of the image gradient and the pose sums ran on the FP64 pipe, which is 64
-//     times slower than the FP32 pipes: conversions are shifts, pose sums are reduced transposed;
+//     times slower than the FP32 pipes: conversions are sums with constants or shifts, pose sums are
+//     reduced transposed;
 //   * the image gradient took 12 atomic adds per sample: neighbouring pixels' samples that land on
 //     the same texel are added within the warp first (integers: the sum does not depend on it).
 #include <algorithm>
@@ -361,7 +362,8 @@ __global__ void __launch_bounds__(kThreads) isb_up_transpose_table_kernel(
 // cell.  A thread takes the 2 x 2 fine pixels of a coarse one, which are read by it and its right and
 // lower neighbours (9 weights); a block takes 32 of them, its warps share out the weights and then the
 // candidates.  kPairs: fine rows are read and written in pairs.  absmax (level 0, else nullptr): the
-// largest |g_c| of the instance, as float bits.
+// largest |g_c| of the instance, as float bits.  (A thread per fine pixel that added to the up step's
+// volume: 131 us at level 0 of two 512 x 512 references, 48 candidates, for its set-up; 53 now.)
 struct QuadEntry {
     int a, b, n;  // fine column and row, reader
 };
@@ -654,6 +656,9 @@ __device__ __forceinline__ void project_jacobian_packed(const float p[3], const 
 // A block takes 32 x 8 pixels of one reference (blockIdx.z), a warp 8 x 4 of them: the samples of
 // neighbouring pixels land on neighbouring texels, and what two lanes have for one texel is added in
 // the warp.  Per pixel the candidates are taken in order (the float32 sums of the pose gradient).
+// Bound by instruction issue, some 800 a sample with the warp's sums, and by how many warps hide their
+// latency: two references of 512 x 512, 48 candidates, 1016 us with two blocks per SM (117
+// registers), 888 with three, 825 with four (64 registers), 872 with five (spills).
 __global__ void __launch_bounds__(kBwdBlock, 4) sweep_backward_references_kernel(
     const __grid_constant__ SweepBwdReferences p, const float4* __restrict__ packed, const int8_t* __restrict__ selected,
     const float* __restrict__ grad_cost, const uint32_t* __restrict__ absmax, long long* __restrict__ image_acc,

@@ -368,9 +368,9 @@ SSG_API int ssg_stage_images_resized(const uint8_t* d_images, int src_cols, int 
                                      int cols, int rows, const int* reference_cameras, int references,
                                      float* d_staged, uint8_t* d_guides, int32_t* d_plane_flags, void* stream);
 
-/* float32 -> uint8 truncation of `count` values in [0, 255] (the float -> uint8 copy of the images
- * to stitch, python/depth_estimation.py:239-240); 16-byte loads and stores where both buffers are
- * 16-byte aligned. */
+/* float32 -> uint8 truncation of `count` values (the float -> uint8 copy of the images to stitch,
+ * python/depth_estimation.py:239-240); outside [0, 256) the low byte of the truncated 64-bit integer, as
+ * torch's copy gives it; 16-byte loads and stores where both buffers are 16-byte aligned. */
 SSG_API int ssg_convert_u8(const float* d_src, uint8_t* d_dst, int64_t count, void* stream);
 
 /* Sphere sweep + cost for every instance (python/depth_estimation.py:141-175), 16-bit output.

@@ -1134,6 +1134,15 @@ static int stage_images(const Tin* d_images, int frames, int cameras, int cols, 
     return launch_status("stage_images_kernel");
 }
 
+// The low byte of v's integer part taken in 64 bits (saturated, NaN 0), as torch converts float32 to uint8.
+// Below 2^31 in magnitude the 32-bit conversion has the same low byte; a float of at least 2^31 is a
+// multiple of 256; below -2^31 both saturated values end in 0, and from 2^63 on in 255.
+__device__ __forceinline__ uint32_t low_byte(float v)
+{
+    const uint32_t i = (uint32_t)__float2int_rz(v);
+    return v >= 0x1p31f && v < 0x1p63f ? 0u : i & 0xFFu;
+}
+
 // float32 -> uint8 truncation (the reference's float -> uint8 copy of the images to stitch,
 // python/depth_estimation.py:239-240): 16 values per thread, four 16-byte loads and one store
 template <bool kAligned>
@@ -1148,8 +1157,7 @@ __global__ void __launch_bounds__(kBatchBlock) convert_u8_kernel(const float* __
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const float4 v = __ldg(reinterpret_cast<const float4*>(src + i) + q);
-            w[q] = __float2uint_rz(v.x) | (__float2uint_rz(v.y) << 8) | (__float2uint_rz(v.z) << 16) |
-                   (__float2uint_rz(v.w) << 24);
+            w[q] = low_byte(v.x) | (low_byte(v.y) << 8) | (low_byte(v.z) << 16) | (low_byte(v.w) << 24);
         }
         reinterpret_cast<uint4*>(dst + i)[0] = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
@@ -1157,7 +1165,7 @@ __global__ void __launch_bounds__(kBatchBlock) convert_u8_kernel(const float* __
 #pragma unroll 4
         for (int q = 0; q < 16; ++q) {
             const int64_t k = base + q * kBatchBlock + threadIdx.x;
-            if (k < n) dst[k] = (uint8_t)__float2uint_rz(src[k]);
+            if (k < n) dst[k] = (uint8_t)low_byte(src[k]);
         }
     }
 }

@@ -58,7 +58,7 @@ __device__ __forceinline__ float unit_value(uint8_t v) { return __fdiv_rn((float
 // integers, distance errors and SSIM values in two floats.
 
 // s.hi + s.lo += v (and + low), the rounding error of the sum kept in lo (Knuth's TwoSum, "The Art of
-// Computer Programming" vol. 2, 4.2.2).  An infinite or NaN v leaves hi as a plain sum would.
+// Computer Programming" vol. 2, 4.2.2).  The sum has to stay in float32's range.
 struct TwoFloat {
     float hi = 0.0f, lo = 0.0f;
     __device__ __forceinline__ void add(float v, float low = 0.0f)
@@ -67,10 +67,7 @@ struct TwoFloat {
         lo += (__fsub_rn(hi, __fsub_rn(t, b)) + __fsub_rn(v, b)) + low;
         hi = t;
     }
-    __device__ __forceinline__ double value() const
-    {
-        return fabsf(hi) <= 3.402823466e38f ? (double)hi + (double)lo : (double)hi;
-    }
+    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
 
 // Sum of float32 squares d2 in [0, 1] that are multiples of 2^-40, exact: every d2 is split into a
@@ -135,6 +132,7 @@ __global__ void __launch_bounds__(kEvalThreads) eval_pointwise_kernel(const __gr
         sq += s.units();
     }
     TwoFloat err, err2;
+    float largest = 0.0f;
     int bad[SSG_EVAL_MAX_THRESHOLDS];
 #pragma unroll
     for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k) bad[k] = 0;
@@ -142,6 +140,7 @@ __global__ void __launch_bounds__(kEvalThreads) eval_pointwise_kernel(const __gr
         const float e = fabsf(__fsub_rn(a, b));
         err.add(e);
         err2.add(__fmul_rn(e, e));
+        largest = fmaxf(largest, e);
 #pragma unroll
         for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k) {
             if (k >= p.thresholds) break;
@@ -157,12 +156,26 @@ __global__ void __launch_bounds__(kEvalThreads) eval_pointwise_kernel(const __gr
         distance(a.w, b.w);
     }
     for (int64_t i = 4 * quads + first; i < n; i += stride) distance(__ldg(inv + i), __ldg(gt_inv + i));
+    double sum = err.value(), sum2 = err2.value();
+    if (largest >= 0x1p48f) {
+        // the two floats hold fewer than 2^31 squares below 2^96: larger errors (a NaN is never the largest, and
+        // stays one in the two floats) are summed once more in FP64
+        sum = sum2 = 0.0;
+        const auto again = [&](int64_t i) {
+            const float e = fabsf(__fsub_rn(__ldg(inv + i), __ldg(gt_inv + i)));
+            sum += (double)e;
+            sum2 += (double)__fmul_rn(e, e);
+        };
+        for (int64_t i = first; i < quads; i += stride)
+            for (int k = 0; k < 4; ++k) again(4 * i + k);
+        for (int64_t i = 4 * quads + first; i < n; i += stride) again(i);
+    }
     double* out = partials + ((int64_t)frame * gridDim.x + blockIdx.x) * eval_slots(p);
     double s = block_sum((double)sq * 0x1p-40, sh);
     if (threadIdx.x == 0) out[kSlotSq] = s;
-    s = block_sum(err.value(), sh);
+    s = block_sum(sum, sh);
     if (threadIdx.x == 0) out[kSlotErr] = s;
-    s = block_sum(err2.value(), sh);
+    s = block_sum(sum2, sh);
     if (threadIdx.x == 0) out[kSlotErr2] = s;
 #pragma unroll
     for (int k = 0; k < SSG_EVAL_MAX_THRESHOLDS; ++k) {

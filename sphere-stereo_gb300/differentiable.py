@@ -139,9 +139,30 @@ class DifferentiableSweep:
 
     def set_selection(self, selected):
         """Use another run's camera-selection maps ([references][rows, cols])."""
-        self._selected = torch.stack([torch.as_tensor(s).reshape(self.rows, self.cols).to(self.device, torch.int8)
-                                      for s in selected])
+        maps = [self._map(s, torch.int8) for s in selected]
+        self._selected = torch.stack(maps) if maps else torch.empty(0, self.rows, self.cols, dtype=torch.int8)
         self.selected = list(self._selected)
+
+    def _map(self, m, dtype: torch.dtype) -> torch.Tensor:
+        return torch.as_tensor(m).reshape(self.rows, self.cols).to(self.device, dtype)
+
+    def _selection(self, g0: int, count: int) -> torch.Tensor:
+        """The maps of ``self.selected`` of ``count`` references from slot g0 on, one after the other as the
+        kernels read them: ``self._selected``'s own, or a copy where entries were replaced."""
+        maps = [self.selected[g0 + i] for i in range(count)]  # IndexError: a reference without a map
+        own = self._selected[g0:g0 + count]
+        if len(own) == count and all(m.data_ptr() == own.data_ptr() + i * self.P for i, m in enumerate(maps)):
+            return own
+        return torch.stack([self._map(m, torch.int8) for m in maps])
+
+    def _gradient_maps(self, grad_q) -> torch.Tensor:
+        """The incoming gradient's maps, one after the other as the kernels read them."""
+        shape = (len(self.refs), self.rows, self.cols)
+        if (isinstance(grad_q, torch.Tensor) and tuple(grad_q.shape) == shape and grad_q.dtype == torch.float32
+                and grad_q.device == self.device and grad_q.is_contiguous()):
+            return grad_q
+        maps = [grad_q[slot] for slot in range(len(self.refs))]  # IndexError: a reference without a map
+        return torch.stack([self._map(m, torch.float32) for m in maps])
 
     # ------------------------------------------------------------------------------------
     def _poses(self, deltas: torch.Tensor) -> _Poses:
@@ -155,17 +176,17 @@ class DifferentiableSweep:
 
     def _pyramid(self, g0: int, refs: list[int], images: torch.Tensor, poses: _Poses, stream):
         """Sweep + filter of a group of references (levels 1..L-1 filtered; level 0 left raw).  Returns
-        what the sweep was called with: the references and their relative poses."""
+        what the sweep was called with: the references, their relative poses and their selection maps."""
         count = len(refs)
+        selection = self._selection(g0, count)
         refs_c, rel = N.ints(refs), N.floats(np.concatenate(poses.relative[g0:g0 + count]))
         N.call("ssg_pack_images", N.pointers([images[c].data_ptr() for c in range(self.C)]), self.C, self.P, refs_c,
                count, self.packed.data_ptr(), self.g_orig[0].data_ptr(), stream)
         N.call("ssg_sweep_cost_references", self.cols, self.rows, self.C, self._cams, count, refs_c, rel,
-               self.packed.data_ptr(), self._selected[g0].data_ptr(), self._cand, self.N, self.costs[0].data_ptr(),
-               stream)
+               self.packed.data_ptr(), selection.data_ptr(), self._cand, self.N, self.costs[0].data_ptr(), stream)
         N.call("ssg_isb_filter", self._levels["g_orig"], self._levels["g_filt"], self._levels["costs"], self.L,
                self.rows, self.cols, self.N, count, self.sigma_i, self.sigma_s, stream)
-        return refs_c, rel
+        return refs_c, rel, selection
 
     def _last_level(self, count: int):
         """The arguments of the soft-argmin's last filter level."""
@@ -187,11 +208,12 @@ class DifferentiableSweep:
     def backward(self, images: torch.Tensor, deltas: torch.Tensor, grad_q: torch.Tensor, poses: _Poses | None = None):
         stream = N.stream_of(images)
         poses = self._poses(deltas) if poses is None else poses
+        grad_q = self._gradient_maps(grad_q)
         grad_images = torch.zeros_like(images)
         grad_local = torch.zeros(self.C, 6, dtype=torch.float64, device=self.device)
         targets = N.pointers([grad_images[c].data_ptr() for c in range(self.C)])
         for g0, refs, count in self._groups():
-            refs_c, rel = self._pyramid(g0, refs, images, poses, stream)
+            refs_c, rel, selection = self._pyramid(g0, refs, images, poses, stream)
             # dL/dF of the filtered level 0, then the filter transposed, then the sweep
             N.call("ssg_soft_argmin_backward", *self._last_level(count), grad_q[g0].data_ptr(), self.gf[0].data_ptr(),
                    stream)
@@ -199,7 +221,7 @@ class DifferentiableSweep:
                    self.cols, self.N, count, self.sigma_i, self.sigma_s, self._levels["gf"], self._levels["gc"],
                    self._tables.data_ptr(), self._absmax.data_ptr(), stream)
             N.call("ssg_sweep_backward_references", self.cols, self.rows, self.C, self._cams, count, refs_c, rel,
-                   self.packed.data_ptr(), targets, self._selected[g0].data_ptr(), self._cand, self.N,
+                   self.packed.data_ptr(), targets, selection.data_ptr(), self._cand, self.N,
                    self.gc[0].data_ptr(), self._absmax.data_ptr(), grad_local.data_ptr(), self._bwd_scratch.data_ptr(),
                    stream)
         to_deltas = torch.from_numpy(poses.to_deltas()).to(self.device, non_blocking=True)

@@ -166,7 +166,11 @@ class DifferentiableSweep:
 
     # ------------------------------------------------------------------------------------
     def _poses(self, deltas: torch.Tensor) -> _Poses:
-        return _Poses(self.base_poses, self.refs, deltas.detach().to("cpu", torch.float64).numpy().copy())
+        """deltas: a row per camera (rows after the last camera's are not read)."""
+        d = deltas.detach().to("cpu", torch.float64).numpy()
+        if len(d) < self.C:
+            raise IndexError(f"pose_deltas has {len(d)} rows, one for each of the {self.C} cameras is required")
+        return _Poses(self.base_poses, self.refs, d[:self.C].copy())
 
     def _groups(self):
         """(first slot, references, how many) of each group of references."""

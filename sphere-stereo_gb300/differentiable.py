@@ -66,12 +66,12 @@ class _Poses:
         self.relative = [(inverse @ T[r])[:, :3].reshape(-1) for r in refs]  # camera_count x 12 each
 
     def to_deltas(self) -> np.ndarray:
-        """[cameras, 6, 6]: gradients of local right perturbations at T [Exp(omega), v] -> gradients with
-        respect to (omega, v)."""
-        out = np.zeros((len(self.deltas), 6, 6))
+        """[cameras, 2, 3, 3]: gradients of local right perturbations at T [Exp(omega), v] -> gradients with
+        respect to omega and to v."""
+        out = np.empty((len(self.deltas), 2, 3, 3))
         for c, d in enumerate(self.deltas):
-            out[c, :3, :3] = so3_right_jacobian(d[:3]).T
-            out[c, 3:, 3:] = so3_exp(d[:3])
+            out[c, 0] = so3_right_jacobian(d[:3]).T
+            out[c, 1] = so3_exp(d[:3])
         return out
 
 
@@ -229,7 +229,7 @@ class DifferentiableSweep:
                    self.gc[0].data_ptr(), self._absmax.data_ptr(), grad_local.data_ptr(), self._bwd_scratch.data_ptr(),
                    stream)
         to_deltas = torch.from_numpy(poses.to_deltas()).to(self.device, non_blocking=True)
-        out = (to_deltas * grad_local[:, None, :]).sum(-1)
+        out = (to_deltas * grad_local.view(self.C, 2, 1, 3)).sum(-1).view(self.C, 6)
         return grad_images, out.to(deltas.device)
 
     def __call__(self, images: torch.Tensor, pose_deltas: torch.Tensor | None = None) -> torch.Tensor:

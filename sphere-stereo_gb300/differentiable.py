@@ -31,24 +31,40 @@ from .isb_filter import level_shapes
 from .utils import _cpu32, camera_struct, relative_poses
 
 
-def skew(w) -> np.ndarray:
+def _skew(w) -> np.ndarray:
     return np.array([[0.0, -w[2], w[1]], [w[2], 0.0, -w[0]], [-w[1], w[0], 0.0]])
 
 
-def so3_exp(w) -> np.ndarray:
+def _so3_exp(w) -> np.ndarray:
     th = float(np.linalg.norm(w))
-    k = skew(w)
+    k = _skew(w)
     if th < 1e-8:
         return np.eye(3) + k + 0.5 * k @ k
     return np.eye(3) + math.sin(th) / th * k + (1 - math.cos(th)) / th ** 2 * k @ k
 
 
-def so3_right_jacobian(w) -> np.ndarray:
+def _so3_right_jacobian(w) -> np.ndarray:
     th = float(np.linalg.norm(w))
-    k = skew(w)
+    k = _skew(w)
     if th < 1e-6:
         return np.eye(3) - 0.5 * k + k @ k / 6
     return np.eye(3) - (1 - math.cos(th)) / th ** 2 * k + (th - math.sin(th)) / th ** 3 * k @ k
+
+
+def _vector(w) -> np.ndarray:
+    return torch.as_tensor(w).detach().to("cpu", torch.float64).numpy()
+
+
+def skew(w) -> torch.Tensor:
+    return torch.from_numpy(_skew(_vector(w)))
+
+
+def so3_exp(w) -> torch.Tensor:
+    return torch.from_numpy(_so3_exp(_vector(w)))
+
+
+def so3_right_jacobian(w) -> torch.Tensor:
+    return torch.from_numpy(_so3_right_jacobian(_vector(w)))
 
 
 class _Poses:
@@ -59,7 +75,7 @@ class _Poses:
         self.deltas = deltas
         E = np.tile(np.eye(4), (len(deltas), 1, 1))
         for c, d in enumerate(deltas):
-            E[c, :3, :3] = so3_exp(d[:3])
+            E[c, :3, :3] = _so3_exp(d[:3])
         E[:, :3, 3] = deltas[:, 3:]
         T = base @ E
         inverse = np.linalg.inv(T)
@@ -70,8 +86,8 @@ class _Poses:
         respect to omega and to v."""
         out = np.empty((len(self.deltas), 2, 3, 3))
         for c, d in enumerate(self.deltas):
-            out[c, 0] = so3_right_jacobian(d[:3]).T
-            out[c, 1] = so3_exp(d[:3])
+            out[c, 0] = _so3_right_jacobian(d[:3]).T
+            out[c, 1] = _so3_exp(d[:3])
         return out
 
 
@@ -103,7 +119,7 @@ class DifferentiableSweep:
         self.candidates = (1 / torch.linspace(1 / min_dist, 1 / max_dist, candidate_count)).tolist()
         self._cand = N.floats(self.candidates)
         self._cams = N.cameras_array([camera_struct(c) for c in calibrations])
-        self.base_poses = np.stack([_cpu32(c.rt).double().numpy() for c in calibrations])
+        self.base_poses = [_cpu32(c.rt).double() for c in calibrations]
         dev = device
         # camera selection of the unperturbed rig (a discrete choice: no gradient)
         mask_stack = torch.stack([torch.as_tensor(m, dtype=torch.float32).reshape(self.rows, self.cols)
@@ -151,7 +167,8 @@ class DifferentiableSweep:
         kernels read them: ``self._selected``'s own, or a copy where entries were replaced."""
         maps = [self.selected[g0 + i] for i in range(count)]  # IndexError: a reference without a map
         own = self._selected[g0:g0 + count]
-        if len(own) == count and all(m.data_ptr() == own.data_ptr() + i * self.P for i, m in enumerate(maps)):
+        first = own.data_ptr()
+        if len(own) == count and all(m.data_ptr() == first + i * self.P for i, m in enumerate(maps)):
             return own
         return torch.stack([self._map(m, torch.int8) for m in maps])
 
@@ -170,7 +187,8 @@ class DifferentiableSweep:
         d = deltas.detach().to("cpu", torch.float64).numpy()
         if len(d) < self.C:
             raise IndexError(f"pose_deltas has {len(d)} rows, one for each of the {self.C} cameras is required")
-        return _Poses(self.base_poses, self.refs, d[:self.C].copy())
+        base = torch.stack(self.base_poses[:self.C]).numpy()
+        return _Poses(base, self.refs, d[:self.C].copy())
 
     def _groups(self):
         """(first slot, references, how many) of each group of references."""
@@ -183,7 +201,7 @@ class DifferentiableSweep:
         what the sweep was called with: the references, their relative poses and their selection maps."""
         count = len(refs)
         selection = self._selection(g0, count)
-        refs_c, rel = N.ints(refs), N.floats(np.concatenate(poses.relative[g0:g0 + count]))
+        refs_c, rel = N.ints(refs), N.floats(np.concatenate(poses.relative[g0:g0 + count]).tolist())
         N.call("ssg_pack_images", N.pointers([images[c].data_ptr() for c in range(self.C)]), self.C, self.P, refs_c,
                count, self.packed.data_ptr(), self.g_orig[0].data_ptr(), stream)
         N.call("ssg_sweep_cost_references", self.cols, self.rows, self.C, self._cams, count, refs_c, rel,

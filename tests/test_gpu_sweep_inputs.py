@@ -20,6 +20,7 @@ def test_replaced_maps_and_expanded_gradients(ss, native, synthetic, refs):
                     for _ in range(2))
     images = torch.as_tensor((rng.random((4, rows, cols, 3)) * 255).astype(np.float32), device=DEV)
     deltas = torch.zeros(4, 6, dtype=torch.float64)
+    assert all(isinstance(p, torch.Tensor) and torch.equal(p, c.rt.double()) for p, c in zip(sweep.base_poses, cals))
     before = sweep.forward(images, deltas)
     maps = [t.clone() for t in plain.selected]
     maps[1] = (maps[1] + 1) % 4

@@ -137,17 +137,28 @@ class Stitcher:
         into ``self.reprojected_distances[reference]``."""
         self._reproject_and_inpaint(distance_map, reference, 1)
 
+    def _fill_tables(self, first: int, count: int) -> torch.Tensor:
+        """The entries of ``inpainting_weights_list`` of references first .. first + count - 1, one after the
+        other as the kernels read them: ``inpainting_tables``' own, or a copy where entries were replaced."""
+        tables = [self.inpainting_weights_list[first + i] for i in range(count)]
+        own = self.inpainting_tables[first:first + count]
+        address, size = own.data_ptr(), 2 * self.rows * self.cols
+        if all(t.data_ptr() == address + i * size for i, t in enumerate(tables)):
+            return own
+        for i, t in enumerate(tables):
+            N.require(t, f"inpainting_weights_list[{first + i}]", torch.uint8, (self.rows, self.cols, 2), self.device)
+        return torch.stack(tables)
+
     def _reproject_and_inpaint(self, maps: torch.Tensor, first: int, count: int) -> None:
         """reproject_and_inpaint of references first .. first + count - 1, whose maps are contiguous."""
         stream = N.stream_of(maps)
-        reprojected = self.reprojected_distances[first].data_ptr()
+        reprojected, tables = self.reprojected_distances[first].data_ptr(), self._fill_tables(first, count)
         intrinsics = N.intrinsics_array(self.intrinsics[first:first + count])
         translations = N.floats(self.translations_host[3 * first:3 * (first + count)].tolist())
         N.call("ssg_reproject_distance_batch", maps.data_ptr(), reprojected, self.cols, self.rows, count, count,
                intrinsics, translations, 1, stream)
-        N.call("ssg_inpaint_batch", reprojected, self.inpainting_tables[first].data_ptr(),
-               self.inpainting_scratch[first].data_ptr(), self.cols, self.rows, count, count, self.max_dist,
-               self.inpainting_iterations, stream)
+        N.call("ssg_inpaint_batch", reprojected, tables.data_ptr(), self.inpainting_scratch[first].data_ptr(),
+               self.cols, self.rows, count, count, self.max_dist, self.inpainting_iterations, stream)
 
     def merge(self) -> None:
         """Blend the stacked maps and images into the panorama (python/stitcher.py:205-218)."""

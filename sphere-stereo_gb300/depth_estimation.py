@@ -52,9 +52,19 @@ class _Fp32Buffers:
         self.costs = [torch.zeros(G, candidates, r, c, **f32) for r, c in shapes]
         self.df_guides = [torch.empty(G, r, c, 3, **u8) for r, c in shapes[1:]]
         self.df_costs = [torch.empty(G, r, c, **f32) for r, c in shapes[1:]]
-        self.guide_levels = N.pointers([g.data_ptr() for g in self.guides])
-        self.cost_levels = N.pointers([c.data_ptr() for c in self.costs])
-        self.df_guide_levels = N.pointers([g.data_ptr() for g in [self.guides[0], *self.df_guides]])
+        self._levels: dict[int, tuple] = {}
+
+    def levels(self, count: int) -> tuple:
+        """Of the last ``count`` references of a group: the first one's place, the level pointers of the
+        guides, the costs and the post-filter's guides, and the addresses of its coarse maps.  A shorter group
+        lies at the end, so that the last reference worked on always has the last place."""
+        if count not in self._levels:
+            at = self.group - count
+            self._levels[count] = (at, N.pointers([g[at].data_ptr() for g in self.guides]),
+                                   N.pointers([c[at].data_ptr() for c in self.costs]),
+                                   N.pointers([g[at].data_ptr() for g in [self.guides[0], *self.df_guides]]),
+                                   [c[at].data_ptr() for c in self.df_costs])
+        return self._levels[count]
 
 
 class RGBD_Estimator:
@@ -168,9 +178,8 @@ class RGBD_Estimator:
         reference worked on."""
         if self._cost_filter is None:
             b = self._fp32_buffers()
-            last = (len(self.references_indices) - 1) % b.group
             self._cost_filter = ISB_Filter.over(self.candidate_count, self.matching_resolution,
-                                                [g[last] for g in b.guides], [c[last] for c in b.costs])
+                                                [g[-1] for g in b.guides], [c[-1] for c in b.costs])
         return self._cost_filter
 
     @property
@@ -294,28 +303,29 @@ class RGBD_Estimator:
             refs = self.references_indices[first + g0:first + g0 + group]
             refs_c = N.ints(refs)
             poses = self._poses[refs[0]] if group == 1 else N.floats([v for r in refs for v in self._poses_list[r]])
+            at, guide_levels, cost_levels, df_guide_levels, df_costs = b.levels(group)
+            cost = b.costs[0][at:]
             # the images stay packed for the later groups; the guides are each group's own
             N.call("ssg_pack_images", pointers, C, rows * cols, refs_c, group if guides is None else 0,
-                   b.packed.data_ptr(), b.guides[0].data_ptr(), stream)
+                   b.packed.data_ptr(), b.guides[0][at].data_ptr(), stream)
             if guides is not None:
-                b.guides[0][:group].copy_(guides[g0:g0 + group])
+                b.guides[0][at:].copy_(guides[g0:g0 + group])
             N.call("ssg_sweep_cost_references", cols, rows, C, self._cams, group, refs_c, poses, b.packed.data_ptr(),
-                   self._selected_maps[first + g0].data_ptr(), self._candidates, n, b.costs[0].data_ptr(), stream)
+                   self._selected_maps[first + g0].data_ptr(), self._candidates, n, cost.data_ptr(), stream)
             raw, index = self.distance_raw_maps[first + g0], self.index_maps[first + g0]
             maps = out[g0:g0 + group]
             if L < 2:
                 for i in range(group):
-                    N.call("ssg_select_distance", b.costs[0][i].data_ptr(), n, rows * cols, self._candidates,
+                    N.call("ssg_select_distance", cost[i].data_ptr(), n, rows * cols, self._candidates,
                            self.distance_raw_maps[first + g0 + i].data_ptr(),
                            self.index_maps[first + g0 + i].data_ptr(), stream)
                 maps.copy_(self.distance_raw_maps[first + g0:first + g0 + group])
                 continue
             # the selection writes the raw distance and, for the post-filter to filter in place, a copy
-            N.call("ssg_isb_filter_select", b.guide_levels, b.cost_levels, L, rows, cols, n, group, float(self.sigma_i),
+            N.call("ssg_isb_filter_select", guide_levels, cost_levels, L, rows, cols, n, group, float(self.sigma_i),
                    float(self.sigma_s), self._candidates, raw.data_ptr(), index.data_ptr(), maps.data_ptr(), stream)
             # distance post-filter with higher edge preservation (python/depth_estimation.py:200-203)
-            N.call("ssg_isb_apply_maps", b.df_guide_levels,
-                   N.pointers([maps.data_ptr(), *(c.data_ptr() for c in b.df_costs)]), L, rows, cols, group,
+            N.call("ssg_isb_apply_maps", df_guide_levels, N.pointers([maps.data_ptr(), *df_costs]), L, rows, cols, group,
                    float(self.sigma_i) / 2, float(self.sigma_s) / 2, N.ISB_SKIP_FINE_GUIDE, stream)
 
     def estimate_fisheye_distance(self, reference_image, guide, reference_calibration, selected_camera, images):

@@ -267,6 +267,19 @@ def pointers(values) -> ctypes.Array:
     return (ctypes.c_void_p * len(values))(*[int(v) for v in values])
 
 
+def largest_group(group: int, allocate) -> int:
+    """How many references are worked on together: ``group``, halved as long as ``allocate(group)``, which
+    makes their buffers, runs out of GPU memory."""
+    while True:
+        try:
+            allocate(group)
+            return group
+        except torch.cuda.OutOfMemoryError:
+            if group == 1:
+                raise
+        group = (group + 1) // 2
+
+
 def fill_launches(iterations: int) -> int:
     """Kernels a tiled hole filling launches: one of up to 8 steps, then one per 24 (copies of whole
     maps not counted)."""

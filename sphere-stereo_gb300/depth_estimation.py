@@ -38,21 +38,24 @@ class _Fp32Buffers:
     pyramid (candidate_count float32 planes per level) and the post-filter's pyramid."""
 
     # References are worked on together as long as their pyramids fit these bytes (the launches of one
-    # reference do not fill the GPU at small sizes; at large ones nothing is gained)
+    # reference do not fill the GPU at small sizes; at large ones nothing is gained) and the GPU's memory
     GROUP_BYTES = 2 << 30
 
     def __init__(self, cameras: int, references: int, candidates: int, shapes, device):
+        per_reference = sum(4 * candidates * r * c for r, c in shapes)
+        self.group = N.largest_group(max(1, min(references, 4, self.GROUP_BYTES // per_reference)),
+                                     lambda G: self._allocate(G, cameras, candidates, shapes, device))
+        self._levels: dict[int, tuple] = {}
+
+    def _allocate(self, G: int, cameras: int, candidates: int, shapes, device) -> None:
         rows, cols = shapes[0]
         u8, f32 = dict(dtype=torch.uint8, device=device), dict(dtype=torch.float32, device=device)
-        per_reference = sum(4 * candidates * r * c for r, c in shapes)
-        self.group = max(1, min(references, 4, self.GROUP_BYTES // per_reference))
-        G = self.group
+        self.packed = self.guides = self.costs = self.df_guides = self.df_costs = None
         self.packed = torch.empty(cameras, rows, cols, 4, **f32)
         self.guides = [torch.zeros(G, r, c, 3, **u8) for r, c in shapes]
         self.costs = [torch.zeros(G, candidates, r, c, **f32) for r, c in shapes]
         self.df_guides = [torch.empty(G, r, c, 3, **u8) for r, c in shapes[1:]]
         self.df_costs = [torch.empty(G, r, c, **f32) for r, c in shapes[1:]]
-        self._levels: dict[int, tuple] = {}
 
     def levels(self, count: int) -> tuple:
         """Of the last ``count`` references of a group: the first one's place, the level pointers of the

@@ -131,27 +131,34 @@ class DifferentiableSweep:
                    float(max_dist), selected[slot].data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
         self._selected = selected
         self.selected = list(selected)
-        # References are worked on together as long as their volumes (costs, and the two gradients of
-        # the filter) fit GROUP_BYTES: the launches of one reference do not fill the GPU
-        f32 = dict(dtype=torch.float32, device=dev)
-        u8 = dict(dtype=torch.uint8, device=dev)
+        self._allocate()
+
+    # References are worked on together as long as their volumes (costs, and the two gradients of the
+    # filter) fit these bytes (the launches of one reference do not fill the GPU) and the GPU's memory
+    GROUP_BYTES = 4 << 30
+
+    def _allocate(self) -> None:
         pyramid = sum(r * c for r, c in self.shapes)
         per_reference = 12 * self.N * pyramid + 24 * self.C * self.P
-        self.group = G = max(1, min(len(self.refs), 4, self.GROUP_BYTES // per_reference))
+        self.group = N.largest_group(max(1, min(len(self.refs), 4, self.GROUP_BYTES // per_reference)), self._buffers)
+        self._levels = {name: N.pointers([t.data_ptr() for t in getattr(self, name)])
+                        for name in ("g_orig", "g_filt", "costs", "gf", "gc")}
+
+    def _buffers(self, G: int) -> None:
+        f32 = dict(dtype=torch.float32, device=self.device)
+        u8 = dict(dtype=torch.uint8, device=self.device)
+        lib = N.library()
+        self.packed = self.g_orig = self.g_filt = self.costs = self.gf = self.gc = None
+        self._tables = self._absmax = self._bwd_scratch = None
         self.packed = torch.empty(self.C, self.rows, self.cols, 4, **f32)
         self.g_orig = [torch.empty(G * r * c * 3, **u8) for r, c in self.shapes]
         self.g_filt = [self.g_orig[0]] + [torch.empty(G * r * c * 3, **u8) for r, c in self.shapes[1:]]
         self.costs, self.gf, self.gc = ([torch.empty(G * self.N * r * c, **f32) for r, c in self.shapes]
                                         for _ in range(3))
-        lib = N.library()
         self._tables = torch.empty(G * lib.ssg_isb_table_floats(self.rows, self.cols, self.L), **f32)
-        self._absmax = torch.empty(G, dtype=torch.int32, device=dev)
+        self._absmax = torch.empty(G, dtype=torch.int32, device=self.device)
         scratch = lib.ssg_sweep_backward_references_scratch_bytes(self.cols, self.rows, self.C, G)
         self._bwd_scratch = torch.empty((scratch + 255) // 256 * 256, **u8)
-        self._levels = {name: N.pointers([t.data_ptr() for t in getattr(self, name)])
-                        for name in ("g_orig", "g_filt", "costs", "gf", "gc")}
-
-    GROUP_BYTES = 4 << 30
 
     def set_selection(self, selected):
         """Use another run's camera-selection maps ([references][rows, cols])."""

@@ -354,6 +354,11 @@ __global__ void __launch_bounds__(kStitchBlock) reproject_frames_kernel(const __
 //     the first step that fills nothing.
 // A cell k pixels inside the region is exact through step k.
 //
+// A mean that is rounded up to a hole's value leaves its cell an open hole of that value, to be visited again
+// when another neighbour is filled.  Where the two bounds overlap (by one float32, if one lies between
+// max_dist + 0.1 and max_dist + 0.1f: 10.0 for 9.9) a hole can be a usable neighbour, and a block that
+// meets one, or such a mean, starts over with plain Jacobi steps.
+//
 // The steps are a chain of dependent accesses: a step takes a fraction of a microsecond in shared
 // memory, and 4 us and more over lists in global memory (ssg_inpaint_holes_batch).  What is left is
 // bound by instruction issue (73 % in the first launch), so the halo follows the work: on rendered
@@ -378,7 +383,7 @@ struct FillShared {
     uint16_t list[cells];   // cells in the order they were filled
     uint8_t stamp[cells];
     uint32_t claimed[cells / 32];
-    int filled[kHalo + 2];  // cells filled by each step
+    int filled[kHalo + 2];  // cells filled by each step; [0] (overlapping bounds): whether a usable value is a hole's
     static_assert(kHalo % 4 == 0 && cells % 32 == 0 && 4 * quads <= 32 && (kFillW * kFillH) % (4 * threads) == 0,
                   "rows of whole quads, a bit per cell of a thread");
 };
@@ -395,10 +400,11 @@ __device__ __forceinline__ int fill_offset(uint32_t b, int cols)
     return ((int)((b >> 2) & 3u) - 1) * cols + (int)(b & 3u) - 1;
 }
 
-// fills open hole `cell` (table entry t) at step `step` if a usable neighbour exists, and lists it
-template <int kHalo>
+// fills open hole `cell` (table entry t) at step `step` if a usable neighbour exists, and lists it; largest
+// (overlapping bounds): of the values filled in
+template <bool kOverlap, int kHalo>
 __device__ __forceinline__ void fill_cell(FillShared<kHalo>& sh, int cell, uint32_t t, int step, int list_begin,
-                                          float valid_at_most)
+                                          float hole_at_least, float valid_at_most, float& largest)
 {
     float val = 0.0f, ws = 0.0f;
 #pragma unroll
@@ -414,7 +420,14 @@ __device__ __forceinline__ void fill_cell(FillShared<kHalo>& sh, int cell, uint3
         }
     }
     if (!(ws > 0.0f)) return;
-    sh.value[cell] = fdiv(val, ws);
+    const float mean = fdiv(val, ws);
+    sh.value[cell] = mean;
+    if (kOverlap) {
+        largest = fmaxf(largest, mean);
+    } else if (mean >= hole_at_least) {  // still a hole, as any number of visits in this step find
+        atomicAnd(&sh.claimed[cell >> 5], ~(1u << (cell & 31)));
+        return;
+    }
     sh.stamp[cell] = (uint8_t)step;
     // one atomic for the lanes that got here together
     const unsigned mask = __activemask(), before = mask & ((1u << (threadIdx.x & 31)) - 1u);
@@ -443,7 +456,52 @@ struct UniformFill {  // instances of one size, tables per reference slot
     }
 };
 
-template <int kHalo, typename Maps>
+// Overlapping bounds: `steps` Jacobi steps on the block's region, read anew from the map: every fillable hole (sh.table) that has
+// a hole's value before a step takes the weighted mean of its usable neighbours' values before the step
+template <int kHalo>
+__device__ __noinline__ void jacobi_steps(FillShared<kHalo>& sh, const FillMap m, int x0, int y0, int steps,
+                                          float hole_at_least, float valid_at_most)
+{
+    using Shared = FillShared<kHalo>;
+    constexpr int W = Shared::width, kThreads = Shared::threads, kOwn = (Shared::cells + kThreads - 1) / kThreads;
+    __syncthreads();  // nothing of the first attempt is read any more
+    for (int cell = threadIdx.x; cell < Shared::cells; cell += kThreads) {
+        const int x = x0 - kHalo + cell % W, y = y0 - kHalo + cell / W;
+        const bool in = x >= 0 && x < m.cols && y >= 0 && y < m.rows;
+        sh.value[cell] = in ? __ldg(m.src + (int64_t)y * m.cols + x) : 0.0f;
+    }
+    __syncthreads();
+    for (int step = 0; step < steps; ++step) {
+        float next[kOwn];
+#pragma unroll
+        for (int r = 0; r < kOwn; ++r) {
+            const int cell = threadIdx.x + r * kThreads;
+            next[r] = cell < Shared::cells ? sh.value[cell] : 0.0f;
+            const uint32_t t = cell < Shared::cells ? sh.table[cell] : 0u;
+            if (t == 0u || !(next[r] >= hole_at_least)) continue;
+            float val = 0.0f, ws = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t b = i == 0 ? t & 255u : t >> 8;
+                if (!fill_weighted(b)) continue;
+                const float sd = sh.value[cell + fill_offset(b, W)], w = (float)(b & 240u);
+                if (sd <= valid_at_most) {
+                    val = fadd(val, fmul(w, sd));
+                    ws = fadd(ws, w);
+                }
+            }
+            if (ws > 0.0f) next[r] = fdiv(val, ws);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kOwn; ++r)
+            if (threadIdx.x + r * kThreads < Shared::cells) sh.value[threadIdx.x + r * kThreads] = next[r];
+        __syncthreads();
+    }
+}
+
+// kOverlap: hole_at_least <= valid_at_most
+template <int kHalo, bool kOverlap, typename Maps>
 __global__ void __launch_bounds__(FillShared<kHalo>::threads) fill_holes_kernel(const Maps maps, int steps,
                                                                                float hole_at_least,
                                                                                float valid_at_most)
@@ -524,6 +582,7 @@ __global__ void __launch_bounds__(FillShared<kHalo>::threads) fill_holes_kernel(
     for (int i = threadIdx.x; i < Shared::cells / 32; i += kThreads) sh.claimed[i] = 0;
     if (threadIdx.x < kHalo + 2) sh.filled[threadIdx.x] = 0;
     uint32_t open = 0;  // bit 4 r + i: cell i of the thread's r-th quad is a fillable hole
+    float largest = -INFINITY;  // overlapping bounds: of the usable holes and of the values filled in
     {
         float v[Shared::quads][4];
         uint2 t[Shared::quads];
@@ -547,7 +606,10 @@ __global__ void __launch_bounds__(FillShared<kHalo>::threads) fill_holes_kernel(
                     const bool inside = lx + i >= 1 && lx + i < W - 1 && ly >= 1 && ly < Shared::height - 1;
                     e[i] = inside ? hole_entry(x0 - kHalo + lx, y0 - kHalo + ly, i, v[r], t[r]) : 0u;
                     if (e[i]) open |= 1u << (4 * r + i);
-                    if (v[r][i] >= hole_at_least) stamps |= (uint32_t)kUnfilled << (8 * i);
+                    if (v[r][i] >= hole_at_least) {
+                        stamps |= (uint32_t)kUnfilled << (8 * i);
+                        if (kOverlap && v[r][i] <= valid_at_most) largest = v[r][i];
+                    }
                 }
                 entries = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
             }
@@ -564,8 +626,9 @@ __global__ void __launch_bounds__(FillShared<kHalo>::threads) fill_holes_kernel(
         // most holes lie among holes: their neighbours' stamps are all that is read
         if ((fill_weighted(b0) && sh.stamp[cell + fill_offset(b0, W)] == 0) ||
             (fill_weighted(b1) && sh.stamp[cell + fill_offset(b1, W)] == 0))
-            fill_cell(sh, cell, t, 1, 0, valid_at_most);
+            fill_cell<kOverlap>(sh, cell, t, 1, 0, hole_at_least, valid_at_most, largest);
     }
+    if (kOverlap && largest >= hole_at_least) sh.filled[0] = 1;
     __syncthreads();
     int begin = 0, count = sh.filled[1];
     for (int step = 2; step <= steps && count > 0; ++step) {
@@ -582,12 +645,14 @@ __global__ void __launch_bounds__(FillShared<kHalo>::threads) fill_holes_kernel(
                                (fill_weighted(b1) && q + fill_offset(b1, W) == p);
             // no other thread has taken q
             if (reads && !(atomicOr(&sh.claimed[q >> 5], 1u << (q & 31)) & (1u << (q & 31))))
-                fill_cell(sh, q, t, step, begin + count, valid_at_most);
+                fill_cell<kOverlap>(sh, q, t, step, begin + count, hole_at_least, valid_at_most, largest);
         }
+        if (kOverlap && largest >= hole_at_least) sh.filled[0] = 1;
         __syncthreads();
         begin += count;
         count = sh.filled[step];
     }
+    if (kOverlap && sh.filled[0]) jacobi_steps(sh, m, x0, y0, steps, hole_at_least, valid_at_most);
 #pragma unroll
     for (int r = 0; r < kOwn; ++r) {
         const float4 q = *reinterpret_cast<const float4*>(sh.value + (kHalo + ty + r * kOwnRows) * W + kHalo + tx);
@@ -596,31 +661,37 @@ __global__ void __launch_bounds__(FillShared<kHalo>::threads) fill_holes_kernel(
     }
 }
 
-// one launch: up to kHalo steps of every map
-template <int kHalo, typename Maps>
-static int fill_pass(const Maps& maps, int max_cols, int max_rows, int count, int steps, double max_dist,
-                     cudaStream_t st)
+template <int kHalo, bool kOverlap, typename Maps>
+static int launch_fill(const Maps& maps, const dim3& grid, int steps, float hole, float ok, cudaStream_t st)
 {
     // more than 48 KB of shared memory: opted in once per device
     static std::atomic<uint64_t> done{0};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return launch_status("cudaGetDevice");
     const uint64_t bit = 1ull << (dev & 63);
+    const auto kernel = fill_holes_kernel<kHalo, kOverlap, Maps>;
     if (!(done.load() & bit)) {
-        const cudaError_t e = cudaFuncSetAttribute(fill_holes_kernel<kHalo, Maps>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)sizeof(FillShared<kHalo>));
         if (e != cudaSuccess)
             return fail(SSG_ERR_CUDA, "cudaFuncSetAttribute(fill_holes_kernel): %s", cudaGetErrorString(e));
         done.fetch_or(bit);
     }
+    kernel<<<grid, FillShared<kHalo>::threads, sizeof(FillShared<kHalo>), st>>>(maps, steps, hole, ok);
+    return launch_status("fill_holes_kernel");
+}
+
+// one launch: up to kHalo steps of every map
+template <int kHalo, typename Maps>
+static int fill_pass(const Maps& maps, int max_cols, int max_rows, int count, int steps, double max_dist,
+                     cudaStream_t st)
+{
     // hole: distance >= MAX_DIST + 0.1 (double, stitcher.cu:287); usable neighbour:
     // distance <= MAX_DIST + 0.1f (stitcher.cu:311)
     const float hole = float_at_least(max_dist + 0.1), ok = float_at_most(max_dist + (double)0.1f);
     const dim3 grid((max_cols + kFillW - 1) / kFillW, (max_rows + kFillH - 1) / kFillH, count);
-    fill_holes_kernel<kHalo, Maps><<<grid, FillShared<kHalo>::threads, sizeof(FillShared<kHalo>), st>>>(maps, steps,
-                                                                                                      hole, ok);
-    return launch_status("fill_holes_kernel");
+    return hole <= ok ? launch_fill<kHalo, true>(maps, grid, steps, hole, ok, st)
+                      : launch_fill<kHalo, false>(maps, grid, steps, hole, ok, st);
 }
 
 // launches of `iterations` steps: the first of kFillFirst, the others of up to kFillRest

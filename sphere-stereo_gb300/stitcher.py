@@ -8,6 +8,8 @@ this object's buffers and are overwritten by the next call, as in the reference.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _native as N
@@ -137,13 +139,18 @@ class Stitcher:
         into ``self.reprojected_distances[reference]``."""
         self._reproject_and_inpaint(distance_map, reference, 1)
 
-    def _fill_tables(self, first: int, count: int) -> torch.Tensor:
+    def _fill_tables(self, first: int, count: int) -> torch.Tensor | int:
         """The entries of ``inpainting_weights_list`` of references first .. first + count - 1, one after the
-        other as the kernels read them: ``inpainting_tables``' own, or a copy where entries were replaced."""
+        other as the kernels read them: the address in ``inpainting_tables``, or a copy where entries were
+        replaced."""
         tables = [self.inpainting_weights_list[first + i] for i in range(count)]
-        own = self.inpainting_tables[first:first + count]
-        address, size = own.data_ptr(), 2 * self.rows * self.cols
-        if all(t.data_ptr() == address + i * size for i, t in enumerate(tables)):
+        size = 2 * self.rows * self.cols
+        own = address = self.inpainting_tables.data_ptr() + first * size
+        for t in tables:
+            if t.data_ptr() != address:
+                break
+            address += size
+        else:
             return own
         for i, t in enumerate(tables):
             N.require(t, f"inpainting_weights_list[{first + i}]", torch.uint8, (self.rows, self.cols, 2), self.device)
@@ -151,14 +158,18 @@ class Stitcher:
 
     def _reproject_and_inpaint(self, maps: torch.Tensor, first: int, count: int) -> None:
         """reproject_and_inpaint of references first .. first + count - 1, whose maps are contiguous."""
+        if not 0 <= first <= self.reference_count - count:
+            raise IndexError(f"reference {first} outside [0, {self.reference_count})")
         stream = N.stream_of(maps)
-        reprojected, tables = self.reprojected_distances[first].data_ptr(), self._fill_tables(first, count)
-        intrinsics = N.intrinsics_array(self.intrinsics[first:first + count])
-        translations = N.floats(self.translations_host[3 * first:3 * (first + count)].tolist())
+        tables = self._fill_tables(first, count)
+        bytes_before = 4 * self.rows * self.cols * first
+        reprojected = self.reprojected_distances.data_ptr() + bytes_before
         N.call("ssg_reproject_distance_batch", maps.data_ptr(), reprojected, self.cols, self.rows, count, count,
-               intrinsics, translations, 1, stream)
-        N.call("ssg_inpaint_batch", reprojected, tables.data_ptr(), self.inpainting_scratch[first].data_ptr(),
-               self.cols, self.rows, count, count, self.max_dist, self.inpainting_iterations, stream)
+               ctypes.byref(self._intr, first * ctypes.sizeof(N.ssg_intrinsics)),
+               ctypes.byref(self._trans, 3 * first * ctypes.sizeof(ctypes.c_float)), 1, stream)
+        N.call("ssg_inpaint_batch", reprojected, tables if isinstance(tables, int) else tables.data_ptr(),
+               self.inpainting_scratch.data_ptr() + bytes_before, self.cols, self.rows, count, count, self.max_dist,
+               self.inpainting_iterations, stream)
 
     def merge(self) -> None:
         """Blend the stacked maps and images into the panorama (python/stitcher.py:205-218)."""

@@ -1332,10 +1332,10 @@ __device__ __forceinline__ void texel_pair_words(const uint8_t* p, uint32_t& lo,
     hi = __funnelshift_r(w1, w2, s);
 }
 
-// interp (stitcher.cu:56-83) on uint8 RGB; words: the texel pairs are read with texel_pair_words (same
+// interp (stitcher.cu:56-83) on uint8 RGB; kWords: the texel pairs are read with texel_pair_words (same
 // values, fewer loads)
-__device__ __forceinline__ void interp_rgb(const uint8_t* __restrict__ img, float u, float v, int cols, float out[3],
-                                           bool words)
+template <bool kWords>
+__device__ __forceinline__ void interp_rgb(const uint8_t* __restrict__ img, float u, float v, int cols, float out[3])
 {
     const int u1 = __float2int_rd(u), v1 = __float2int_rd(v), u2 = u1 + 1, v2 = v1 + 1;
     const float w1 = fmul(fsub((float)u2, u), fsub((float)v2, v)), w2 = fmul(fsub((float)u2, u), fsub(v, (float)v1));
@@ -1343,7 +1343,7 @@ __device__ __forceinline__ void interp_rgb(const uint8_t* __restrict__ img, floa
     const uint8_t* top = img + 3 * ((int64_t)v1 * cols + u1);
     const uint8_t* bottom = img + 3 * ((int64_t)v2 * cols + u1);
     uint32_t t1 = 0, t2 = 0, t3 = 0, t4 = 0;  // the texels' bytes
-    if (words) {
+    if constexpr (kWords) {
         uint32_t hi;
         texel_pair_words(top, t1, hi);
         t3 = __byte_perm(t1, hi, 0x0543);
@@ -1423,10 +1423,11 @@ __device__ __forceinline__ void project_fast(const float p[3], const Intr& k, fl
 }
 
 // mergeRGBDPanoramaKernel, stitcher.cu:423-473.  Bound by instruction issue: the camera model's IEEE
-// divisions and square roots, some 400 instructions a pixel and reference.  2048 x 1024, two
-// references: 65.6 us with byte loads, 63.7 with word loads, 61.9 with eight blocks per SM; 70 with
-// both references in flight.
-__global__ void __launch_bounds__(kStitchBlock, 8) merge_kernel(const __grid_constant__ MergeParams p,
+// divisions and square roots, some 400 instructions a pixel and reference, and by the gathers of texels.
+// kWords: texel pairs as words (texel_pair_words), which take fewer loads and more instructions, and eight
+// blocks per SM; else bytes and six blocks (use_words says when).
+template <bool kWords>
+__global__ void __launch_bounds__(kStitchBlock, kWords ? 8 : 6) merge_kernel(const __grid_constant__ MergeParams p,
                                                              const float2* __restrict__ lut,
                                                              const float* __restrict__ weights,
                                                              const float* __restrict__ reproj,
@@ -1472,8 +1473,8 @@ __global__ void __launch_bounds__(kStitchBlock, 8) merge_kernel(const __grid_con
         o[1] = fminf(fmaxf(o[1], 0.1f), rowsm);
         o[1] = fadd(o[1], (float)(r * p.image_rows));
         float c[3];
-        interp_rgb(images + (int64_t)(p.image_slot[r] - r) * p.image_rows * p.image_cols * 3, o[0], o[1],
-                   p.image_cols, c, p.word_rows);
+        interp_rgb<kWords>(images + (int64_t)(p.image_slot[r] - r) * p.image_rows * p.image_cols * 3, o[0], o[1],
+                           p.image_cols, c);
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) rgb[ch] = fadd(rgb[ch], fmul(c[ch], w));
     }
@@ -1921,7 +1922,14 @@ static int merge_batch(const float* d_lut, const float* d_weights, const float* 
                 p, frames, lut, d_weights, d_reprojected, d_distances, d_images, d_distance_panorama, d_rgb_panorama);
         return launch_status("merge_frames_kernel");
     } else {
-        merge_kernel<<<grid, kStitchBlock, 0, as_stream(stream)>>>(
+        // Words where they are possible and an image holds 0.7 of the panorama's pixels or more: neighbouring
+        // panorama pixels then share fewer texels.  2048 x 1024, two references, in us by words and by bytes:
+        // images of 2048 x 2048 pixels 62 and 70, 1216 x 1216 60 and 60 (four references 113 and 117),
+        // 512 x 512 60 and 57; 1536 x 768 from 768 x 768 38 and 36, 1280 x 640 from 640 x 480, four
+        // references, 51 and 47.
+        const bool use_words = p.word_rows && (int64_t)image_rows * image_cols * 10 >= Q * 7;
+        const auto kernel = use_words ? merge_kernel<true> : merge_kernel<false>;
+        kernel<<<grid, kStitchBlock, 0, as_stream(stream)>>>(
             p, reinterpret_cast<const float2*>(d_lut), d_weights, d_reprojected, d_distances, d_images,
             d_distance_panorama, d_rgb_panorama);
         return launch_status("merge_kernel");

@@ -43,7 +43,7 @@ TUNE_STAGE_COLUMNS = 15
 STATUS_TMA_TIMEOUT = 1
 STATUS_BARRIER_TIMEOUT = 2
 HOLE_SCRATCH_HEADER = 8
-MAX_FILL_STEPS = 254  # of a batch's hole filling
+MAX_FILL_STEPS = 254  # of a batch's hole filling: what the batched calls have always taken
 ISB_SKIP_FINE_GUIDE = 1
 PIXEL_U8 = 0
 PIXEL_F32 = 1

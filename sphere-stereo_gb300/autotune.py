@@ -1,9 +1,10 @@
 """Autotuner of the batched kernels' launch shapes (no counterpart in the reference).
 
 The library exposes a few launch-shape knobs (include/sphere_stereo_gb300.h, SSG_TUNE_*): the
-sweep's block shape, the blocks per SM of the hole-filling steps, the frames one merge thread
-handles, the work-item span of the uneven sweep and the register bounds of the ISB upsampling
-(coarse levels and the fused selecting level).  For a workload (a key naming the device and
+sweep's block shape, the frames one merge thread handles, the work-item span of the uneven sweep,
+the register bounds of the ISB upsampling (coarse levels and the fused selecting level), and those
+of the hole filling over lists, which no workload of this package launches any more (results that
+name them are still read).  For a workload (a key naming the device and
 the shapes), ``Tuner.tune`` runs the caller's launch sequence eagerly, times the entry point each
 knob affects with CUDA events on the stream it is enqueued on, one knob at a time over its
 choices (coordinate descent: the knobs act on different kernels), and keeps the fastest.  Results

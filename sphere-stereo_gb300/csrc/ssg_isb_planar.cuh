@@ -13,7 +13,7 @@
 // 134 MB (up) to move at 1024^2 x 32 candidates, 25 and 45 us at the measured copy rate.  One block
 // of a tile staged per candidate between two barriers, as the steps ran before, took 74 and 132 us
 // there, and 26 us on every small level, whose time is one thread's chain over all candidates;
-// now 48 and 95 us, and 5 to 8 us.
+// now 45 and 115 us from cold caches (95 us when the caller has just written the volume), and 5 to 8 us.
 #pragma once
 
 #include "ssg_isb_common.cuh"
@@ -202,10 +202,12 @@ __device__ __forceinline__ float2 load_fine(const float* __restrict__ c, int at,
 // read value by value (an odd width) gain by it, the selecting step with registers for 10 blocks of 64
 // threads: 4 x 637 x 479 x 43, level 1 58 -> 49.5 us, selecting level 204 -> 192 us, the frame 938 -> 925 us.
 // Rows read in pairs lose: 1024^2 x 32 filtered 311 -> 316 us, a frame of 2 x 1024^2 x 32 1097 -> 1107 us.
+// (Measured at these sizes only, where a block has one range of candidates.)
 template <bool kPairs>
 constexpr int kUpAhead = kPairs ? 0 : 4;
 
-// blocks per SM the up step's registers are bounded for
+// blocks per SM the up step's registers are bounded for: 640 threads (odd widths, selecting) or 768 with one
+// range, as many as whole blocks hold with more (of 4 ranges 2 and 3 blocks of 256 threads), 1024 with 8
 template <int kRanges, bool kSelect, bool kPairs>
 constexpr int up_blocks = kRanges == 8 ? 2 : (kSelect && !kPairs ? 10 : 12) / kRanges;
 
@@ -602,7 +604,8 @@ static int planar_tail_first(const int* rows, const int* cols, int levels, int n
 // Into how many ranges a step's candidates are shared out: a power of two of at most `ncand`.  Every
 // range more repeats the set-up of the pixel's weights, which costs about as much as 10
 // candidates, and a level too small to fill the GPU needs the ranges to keep enough loads in
-// flight.  Measured at 32 candidates, in microseconds for 1, 2, 4 and 8 ranges: the down step to
+// flight.  Measured at 32 candidates alone (fewer than the ranges only cap them), in microseconds for 1, 2, 4
+// and 8 ranges: the down step to
 // 262144 pixels 54, 49, 48, 52, to 65536 27, 18, 16, 16, to 16384 24, 14, 9, 7; the up step from
 // 262144 pixels (selecting) 116, 128, 152, 192, from 65536 25, 31, 35, 42, from 16384 23, 15, 12, 15,
 // from 4096 22, 14, 10, 8.

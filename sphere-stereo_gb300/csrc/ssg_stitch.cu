@@ -6,8 +6,9 @@
 //    compare-and-store twice, stitcher.py:185-192) and targets outside the map are dropped (the
 //    reference's index is unchecked, stitcher.cu:198);
 //  * inpainting is a sequence of Jacobi steps (every pixel reads the map as it was before the
-//    step; the reference updates in place and its result depends on thread timing).  Up to 32
-//    steps run per launch on a shared-memory tile with a 32-pixel halo, from one map to another;
+//    step; the reference updates in place and its result depends on thread timing).  A first launch
+//    runs 8 steps and each later one 24, on shared-memory tiles with a halo of as many pixels, from one
+//    map to another;
 //  * a table entry whose two best weights stay 0 (outside the model's valid area) encodes the
 //    offsets (0, 0); the reference leaves them uninitialised (stitcher.cu:231).
 #include <algorithm>
@@ -366,8 +367,9 @@ __global__ void __launch_bounds__(kStitchBlock) reproject_frames_kernel(const __
 // ever filled is filled within 8 steps, and later steps fill something in 5 % of the tiles.  One
 // launch of 32 steps stages 6 cells per pixel; 8 steps stage 1.9 everywhere, and the other 24 stage
 // 4.4 only where a hole is still open.  Measured, 16 such maps: 465 us over lists, 560 us in one
-// launch, 158 + 104 us in two; two maps of noisy distances: 260 us (two launches of 16 steps over
-// every hole of a tile), 140 us in one, 38 + 48 us now.
+// launch, 164 + 104 us in two; two maps of noisy distances: 260 us (two launches of 16 steps over
+// every hole of a tile), 140 us in one, 45 + 49 us now.  Maps with next to no holes are slower than over
+// lists, which only scan them: 16 maps 76 and 31 us.
 // ---------------------------------------------------------------------------------------------
 constexpr uint8_t kUnfilled = 255;
 constexpr int kFillW = 64, kFillH = 32;
@@ -735,7 +737,8 @@ static int fill_uniform(float* map, float* scratch, const uint8_t* tables, int c
 
 // ---------------------------------------------------------------------------------------------
 // Hole filling over lists of holes in global memory (ssg_inpaint_holes_batch), in place and with the
-// result of the steps above.
+// result of the steps above, but at values on the two bounds: here a filled hole is never a hole again,
+// and a hole is never a usable neighbour.
 // Only holes change, a filled hole keeps its value from then on, and a hole whose two table
 // weights are 0 (outside the model's valid area) never changes.  Every pixel gets a one-byte
 // stamp: 0 for a pixel that is not a hole, kUnfilled for a hole, s for a hole filled at step s.
@@ -748,7 +751,7 @@ static int fill_uniform(float* map, float* scratch, const uint8_t* tables, int c
 //     holes that read a pixel filled at step s - 1: the work of a step is its frontier.  A claim
 //     word per pixel (the last step that queued it) keeps a hole from being visited twice.
 // ---------------------------------------------------------------------------------------------
-constexpr int kMaxListIterations = 254;
+constexpr int kMaxListIterations = 254;  // stamps are bytes; the uneven batch keeps the limit it had with lists
 
 struct HoleOffsets {
     int64_t n0, n1;

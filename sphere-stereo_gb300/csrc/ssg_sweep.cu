@@ -197,7 +197,8 @@ __global__ void __launch_bounds__(kBlock) rgb_to_guide_kernel(const float* __res
 //
 // ssg_pack_images writes the images as 16-byte texels (R, G, B, 0), so that a bilinear tap is one load
 // instead of three loads of a 12-byte stride, which touch three times the cache lines; the pass
-// costs 28 bytes per texel once per frame and forms the references' guides on the way.  The sweep
+// costs 28 bytes per texel, once per group of references that are worked on together, and forms their
+// guides on the way (one reference with few candidates is not worth it: ssg_sweep_cost).  The sweep
 // itself does what sweep_cost_kernel does, value by value (same bits), with its quotients taken
 // from a reciprocal (div_by_reciprocal).
 //
@@ -492,9 +493,9 @@ extern "C" int ssg_sweep_cost_references(int cols, int rows, int camera_count, c
             std::memcpy(p.rt[r], relative_poses + (int64_t)(r0 + r) * camera_count * 12,
                         sizeof(float) * 12 * camera_count);
         }
-        // below two threads per resident slot of the GPU the candidates are shared out over 2 or 4
-        // threads (a thread's unprojection costs about one candidate): two references of 256^2 x 32
-        // took 2 x 44 us in a launch each, 31 us in one
+        // below 600000 threads (four for each of the 1024 that an SM holds of this kernel) the candidates are
+        // shared out over 2 or 4 threads (a thread's unprojection costs about one candidate): two references
+        // of 256^2 x 32, the size the line was set at, took 2 x 44 us in a launch each, 31 us in one
         p.ranges = 1;
         while (p.ranges < 4 && P * count * p.ranges < 600000 && candidate_count >= 16 * p.ranges) p.ranges *= 2;
         sweep_references_kernel<<<dim3(((cols + kTileX - 1) / kTileX) * ((rows + kBlock / kTileX - 1) / (kBlock / kTileX)), count, p.ranges), kBlock, 0, as_stream(stream)>>>(

@@ -31,24 +31,28 @@ from .isb_filter import level_shapes
 from .utils import _cpu32, camera_struct, relative_poses
 
 
+_EYE3, _EYE4 = np.eye(3), np.eye(4)
+
+
 def _skew(w) -> np.ndarray:
-    return np.array([[0.0, -w[2], w[1]], [w[2], 0.0, -w[0]], [-w[1], w[0], 0.0]])
+    x, y, z = w.tolist()
+    return np.array([[0.0, -z, y], [z, 0.0, -x], [-y, x, 0.0]])
 
 
 def _so3_exp(w) -> np.ndarray:
-    th = float(np.linalg.norm(w))
+    th = math.sqrt(w.dot(w))
     k = _skew(w)
     if th < 1e-8:
-        return np.eye(3) + k + 0.5 * k @ k
-    return np.eye(3) + math.sin(th) / th * k + (1 - math.cos(th)) / th ** 2 * k @ k
+        return _EYE3 + k + 0.5 * k @ k
+    return _EYE3 + math.sin(th) / th * k + (1 - math.cos(th)) / th ** 2 * k @ k
 
 
 def _so3_right_jacobian(w) -> np.ndarray:
-    th = float(np.linalg.norm(w))
+    th = math.sqrt(w.dot(w))
     k = _skew(w)
     if th < 1e-6:
-        return np.eye(3) - 0.5 * k + k @ k / 6
-    return np.eye(3) - (1 - math.cos(th)) / th ** 2 * k + (th - math.sin(th)) / th ** 3 * k @ k
+        return _EYE3 - 0.5 * k + k @ k / 6
+    return _EYE3 - (1 - math.cos(th)) / th ** 2 * k + (th - math.sin(th)) / th ** 3 * k @ k
 
 
 def _vector(w) -> np.ndarray:
@@ -73,7 +77,8 @@ class _Poses:
 
     def __init__(self, base: np.ndarray, refs: list[int], deltas: np.ndarray):
         self.deltas = deltas
-        E = np.tile(np.eye(4), (len(deltas), 1, 1))
+        E = np.empty((len(deltas), 4, 4))
+        E[:] = _EYE4
         for c, d in enumerate(deltas):
             E[c, :3, :3] = _so3_exp(d[:3])
         E[:, :3, 3] = deltas[:, 3:]

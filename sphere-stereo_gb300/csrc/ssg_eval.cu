@@ -196,6 +196,7 @@ __global__ void __launch_bounds__(kEvalThreads) eval_pointwise_kernel(const __gr
 //     N (sum p^2 -+ sum m^2) - ((sum p)^2 -+ (sum m)^2)    are N^2 times 4 cov and 2 (var + var),
 // so the four factors of the SSIM ratio are, up to a common scale, those integers plus a constant
 // each: the variances suffer no cancellation.  The ratio is formed in two floats (error 2^-43).
+// Against 113-bit sums the mean of an image is within 2e-14 (FP64 window sums: 5e-15).
 //
 // Bound by instruction issue (about 130 per value).  FP64 sums per window took 7471 us for 4 frames
 // of 2048x1024, this form takes 167 us.
